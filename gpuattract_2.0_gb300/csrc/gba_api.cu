@@ -207,15 +207,27 @@ DevNL nl_from_desc(const gba_nl_desc& d) {
 	return g;
 }
 
-/* The sqrt-ratio table of src/model/NLGrid.tpp:45-50, bit-identical. */
-std::vector<float> nl_ratio_table(float dPlateau2) {
-	const int size = int(10000 * dPlateau2);
-	std::vector<float> r(size + 1);
-	for (int n = 0; n <= size; n++) {
-		double d2 = ((n + 0.5) / 10000);
-		r[n] = (float)std::sqrt(d2 / (double)dPlateau2);
-	}
-	return r;
+namespace {
+
+__global__ void ratio_table_kernel(float* __restrict__ out, size_t n, double dPlateau2) {
+	const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+	if (k >= n) return;
+	const double d2 = __ddiv_rn(__dadd_rn((double)k, 0.5), 10000.0);
+	out[k] = (float)__dsqrt_rn(__ddiv_rn(d2, dPlateau2));
+}
+
+}  // namespace
+
+/* The sqrt-ratio table of src/model/NLGrid.tpp:45-50, filled on the device:
+ * the same IEEE double operations, so bit-identical to the reference's (the
+ * host took 8 ms for its million square roots and the copy). */
+void nl_ratio_table(float dPlateau2, DevBuffer& out) {
+	if (!(10000 * dPlateau2 < 2147483520.0f))      /* the largest float below 2^31 */
+		throw ApiError(GBA_ERR_INVALID_ARGUMENT, "neighbour grid plateau too large for its ratio table");
+	const size_t n = (size_t)int(10000 * dPlateau2) + 1;
+	out.alloc(n * sizeof(float));
+	ratio_table_kernel<<<(unsigned)((n + 255) / 256), 256>>>((float*)out.ptr, n, (double)dPlateau2);
+	check_cuda(cudaGetLastError(), "ratio table");
 }
 
 }  // namespace gba
@@ -398,11 +410,12 @@ int gba_upload_grid(gba_ctx* ctx, const gba_intrpl_desc* inner, const float* inn
 	item->dev.outer = intrpl_from_desc(*outer);
 	item->dev.outer.data = (const float4*)item->outer.ptr;
 	item->dev.nl = nl_from_desc(*nl);
-	std::vector<float> ratio = nl_ratio_table(item->dev.nl.dPlateau2);
-	item->ratio.upload(ratio.data(), ratio.size() * sizeof(float));
+	nl_ratio_table(item->dev.nl.dPlateau2, item->ratio);
 	item->dev.nl.grid = (const uint2*)item->nlgrid.ptr;
 	item->dev.nl.list = (const uint32_t*)item->nllist.ptr;
 	item->dev.nl.ratio = (const float*)item->ratio.ptr;
+	/* calls on any stream may read the table */
+	check_cuda(cudaStreamSynchronize(0), "gba_upload_grid: ratio table");
 	/* every receptor index in the list is checked against the receptor at call time */
 	uint32_t max_idx = 0;
 	for (uint32_t k = 0; k < nl->numEl; ++k) max_idx = std::max(max_idx, nl_list[k]);

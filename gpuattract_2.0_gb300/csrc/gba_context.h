@@ -138,7 +138,7 @@ const uint32_t* pose_order_in(const void* dofs, size_t stride_floats, size_t n, 
 
 DevIntrpl intrpl_from_desc(const gba_intrpl_desc& d);
 DevNL nl_from_desc(const gba_nl_desc& d);
-std::vector<float> nl_ratio_table(float dPlateau2);
+void nl_ratio_table(float dPlateau2, DevBuffer& out);
 
 /* Launch shape chosen by the autotuner (or the defaults). */
 struct TuneParams {
