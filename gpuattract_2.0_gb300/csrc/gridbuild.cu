@@ -37,110 +37,355 @@ namespace gba {
 
 namespace {
 
-constexpr int kTile = 256;
-constexpr int kGroup = 4;   /* channels per thread */
+constexpr int kTile = 256;   /* receptor beads per FP32 partial sum; voxels per block of the list kernels */
 
 struct BuildArgs {
 	const float4* xyzq;      /* receptor beads */
 	const uint32_t* tm;      /* type | mapped << 16 */
 	uint32_t n;
 	DevParams par;
-	const uint32_t* alphabet;  /* device copy, n_alphabet entries */
 	uint32_t n_alphabet;
 	float plateau, plat2;
 	double cut2;
+	/* per receptor type (row 0: dummy beads, all zero) and type channel
+	 * (n_lj of them, the alphabet padded to whole warps): the pair parameters
+	 * as grid_potential_kernel reads them (pair_rows_kernel) */
+	const float4* rows;
+	uint32_t n_lj;
+	float one;               /* 1 */
 };
 
-__global__ void __launch_bounds__(kTile) grid_potential_kernel(BuildArgs a, gba_intrpl_desc d,
-		float4* __restrict__ out) {
-	__shared__ float4 sb[kTile];
-	__shared__ uint32_t stype[kTile];
+/* ---- potentials -------------------------------------------------------------
+ *
+ * Per voxel, channel and bead 12 FP32 operations that must each round on
+ * their own (the CPU builder's bits), so the FP32 pipe bounds the kernel:
+ * 1,500 beads, 1.15 M voxels and 32 channels are 6.6e11 operations, 17.5 ms at
+ * the 37.8e12 a second that the pipe does.  One thread per voxel and four
+ * channels repeated the geometry -- a division, near beads a square root and
+ * another division -- nine times per voxel and bead and took 77.7 ms.  Here a
+ * block holds a brick of 4 x 4 x 4 voxels and up to 32 channels: two warps
+ * compute the brick's geometry for 16 beads at a time into shared memory
+ * (one also sums the charge channel), eight warps of four channels each read it
+ * back, two voxels per lane in packed FP32 instructions, which halve the
+ * issue slots.  Double-buffered, one barrier per 16 beads (8: 6 % slower).
+ * Measured for the 1,500 beads: 36.8 ms with one geometry warp, which the
+ * others waited for; 27.5 ms with two. */
+
+constexpr int kChan = 4;                      /* type channels per warp */
+constexpr int kLjWarps = 8;                   /* most warps of type channels per block */
+constexpr int kCube = 4;                      /* voxels per axis of a block */
+constexpr int kChunk = 16;                    /* beads per barrier */
+constexpr int kRowAhead = 4;                  /* beads whose rows a warp loads together */
+static_assert(kTile % kChunk == 0, "a partial sum ends with a chunk");
+
+/* Two voxels of a lane (z and z + 2 of its column): packed FP32, each half
+ * rounded as the scalar operation. */
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float a, float b) {
+	f2 r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+	return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+	f2 r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+	f2 r;
+	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+	f2 r;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+	return r;
+}
+
+/* One bead's geometry for a lane's two voxels: 1/d^2, the direction over d^2
+ * and 1/d^6 at d = max(r, plateau), and d^2 itself. */
+struct VoxelGeo {
+	f2 rr2[32], ux[32], uy[32], uz[32], rr23[32], d2[32];
+};
+struct Chunk {
+	VoxelGeo geo[kChunk];
+	uint32_t row[kChunk];      /* receptor type, 0: no contribution */
+	float qf[kChunk];          /* charge times ffelec, 0: no contribution */
+};
+
+/* out[2 k] = {rc, rc, -ac, -ac}, out[2 k + 1] = {ipon, ipon, rmin2, emin} for
+ * k = receptor type * n_lj + channel */
+__global__ void pair_rows_kernel(DevParams par, const uint32_t* __restrict__ alphabet, uint32_t n_alphabet,
+		uint32_t n_lj, float4* __restrict__ out) {
+	const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+	if (k >= (size_t)(par.num_types + 1) * n_lj) return;
+	const uint32_t tr = (uint32_t)(k / n_lj), c = (uint32_t)(k % n_lj);
+	const uint32_t tl = c < n_alphabet ? alphabet[c] : 0u;
+	float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+	float iv = 0.f;
+	if (tr != 0 && tl != 0 && tl <= par.num_types) {
+		const size_t t = (size_t)par.num_types * (tr - 1) + (tl - 1);
+		p = par.lj[t];
+		iv = par.ivor[t];
+	}
+	out[2 * k] = make_float4(p.x, p.x, -p.y, -p.y);
+	out[2 * k + 1] = make_float4(iv, iv, p.z, p.w);
+}
+
+/* A geometry warp's share of the beads of a chunk, in pairs: the warp that
+ * also sums the charge channel takes fewer. */
+constexpr int kPairs = kChunk / 2, kChargePairs = 3;
+
+/* Bead j of the receptor as one lane holds it for its chunk: nothing for a
+ * dummy bead (type 0) or past the end. */
+struct Bead {
+	float4 r;
+	uint32_t type;
+};
+__device__ __forceinline__ Bead load_bead(const BuildArgs& a, uint32_t j) {
+	Bead b{make_float4(0.f, 0.f, 0.f, 0.f), 0u};
+	if (j < a.n) {
+		b.type = __ldg(&a.tm[j]) & 0xffffu;
+		if (b.type != 0) b.r = __ldg(&a.xyzq[j]);
+	}
+	return b;
+}
+
+/* The geometry of the bead pairs [i0, i1) of a chunk for the brick, by one
+ * warp: lane = column (x, y) of the brick and half = bead of the pair; lane b
+ * (< kChunk) brings bead b of the chunk. */
+__device__ __forceinline__ void fill_chunk(const BuildArgs& a, const Bead& mine, int i0, int i1, float px, float py,
+		const float pz[kCube], int lane, Chunk& C) {
+	const int col = lane & 15, half = lane >> 4;
+	for (int i = i0; i < i1; ++i) {
+		const int b = 2 * i + half;
+		const uint32_t tr = __shfl_sync(0xffffffffu, mine.type, b);
+		const float rx = __shfl_sync(0xffffffffu, mine.r.x, b), ry = __shfl_sync(0xffffffffu, mine.r.y, b),
+				rz = __shfl_sync(0xffffffffu, mine.r.z, b), rq = __shfl_sync(0xffffffffu, mine.r.w, b);
+		if (col == 0) {
+			const float qf = fmul(rq, a.par.ffelec);
+			C.row[b] = tr;
+			C.qf[b] = fabsf(qf) > 0.001f ? qf : 0.f;
+		}
+		const float ex0 = fsub(px, rx), ey0 = fsub(py, ry);
+		const float exy = fadd(fmul(ex0, ex0), fmul(ey0, ey0));
+		float ex[kCube], ey[kCube], ez[kCube], e2[kCube];
+		bool near = false;
+#pragma unroll
+		for (int z = 0; z < kCube; ++z) {
+			ex[z] = ex0;
+			ey[z] = ey0;
+			ez[z] = fsub(pz[z], rz);
+			e2[z] = fadd(exy, fmul(ez[z], ez[z]));
+			near |= e2[z] < a.plat2;
+		}
+		if (near) {
+#pragma unroll
+			for (int z = 0; z < kCube; ++z)
+				if (e2[z] < a.plat2) {
+					/* a bead at the voxel's centre has no direction */
+					const float sc = e2[z] > 0.f ? __fdiv_rn(a.plateau, __fsqrt_rn(e2[z])) : 0.f;
+					ex[z] = fmul(ex[z], sc); ey[z] = fmul(ey[z], sc); ez[z] = fmul(ez[z], sc);
+					e2[z] = a.plat2;
+				}
+		}
+		float rr2[kCube];
+#pragma unroll
+		for (int z = 0; z < kCube; ++z) rr2[z] = __frcp_rn(e2[z]);
+		VoxelGeo& g = C.geo[b];
+#pragma unroll
+		for (int h = 0; h < 2; ++h) {
+			const int l = col + 16 * h;
+			const f2 i2 = pack2(rr2[h], rr2[h + 2]);
+			g.rr2[l] = i2;
+			g.ux[l] = mul2(pack2(ex[h], ex[h + 2]), i2);
+			g.uy[l] = mul2(pack2(ey[h], ey[h + 2]), i2);
+			g.uz[l] = mul2(pack2(ez[h], ez[h + 2]), i2);
+			g.rr23[l] = mul2(mul2(i2, i2), i2);
+			g.d2[l] = pack2(e2[h], e2[h + 2]);
+		}
+	}
+}
+
+/* Adds a partial sum's packed pair to the two voxels' double sums. */
+__device__ __forceinline__ void fold2(f2& part, double acc[2]) {
+	float lo, hi;
+	unpack2(part, lo, hi);
+	acc[0] = __dadd_rn(acc[0], (double)lo);
+	acc[1] = __dadd_rn(acc[1], (double)hi);
+	part = 0;
+}
+
+/* PLAIN: every pair's ipon is 1, its minimum lies inside the plateau (no
+ * branch on d^2 < rmin2) and 2 (rep rr23) = rep (2 rr23) without underflow;
+ * the host checks all three (plain_pairs).  8-6 shape only. */
+template <bool PLAIN>
+__global__ void __launch_bounds__(32 * (kLjWarps + 2), 2) grid_potential_kernel(const BuildArgs a,
+		const gba_intrpl_desc d, float4* __restrict__ out) {
+	__shared__ Chunk buf[2];
 	const uint32_t Nx = d.dimN[0], Ny = d.dimN[1], Nz = d.dimN[2];
-	const uint32_t N = Nx * Ny * Nz;
-	const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-	const bool valid = v < N;
-	const uint32_t x = valid ? v % Nx : 0, y = valid ? (v / Nx) % Ny : 0, z = valid ? v / (Nx * Ny) : 0;
-	const double sp = (double)d.gridSpacing;
-	const float px = (float)__dadd_rn((double)d.posMin[0], __dmul_rn((double)x, sp));
-	const float py = (float)__dadd_rn((double)d.posMin[1], __dmul_rn((double)y, sp));
-	const float pz = (float)__dadd_rn((double)d.posMin[2], __dmul_rn((double)z, sp));
-	const uint32_t c0 = blockIdx.y * kGroup;
-	const uint32_t C = a.n_alphabet + 1;
-	const bool shape86 = a.par.potshape == GBA_POTSHAPE_8_6;
-	const bool cdiel = a.par.dielec == GBA_DIELEC_CONSTANT;
-	double acc[kGroup][4];
+	const size_t N = (size_t)Nx * Ny * Nz;
+	const int lane = threadIdx.x & 31;
+	const int warp = threadIdx.x >> 5, lj_warps = (blockDim.x >> 5) - 2;
+	const uint32_t bx = (Nx + kCube - 1) / kCube, by = (Ny + kCube - 1) / kCube;
+	const uint32_t x0 = blockIdx.x % bx * kCube, y0 = blockIdx.x / bx % by * kCube,
+			z0 = blockIdx.x / (bx * by) * kCube;
+	const uint32_t chunks = (a.n + kChunk - 1) / kChunk;
+	/* the lane's voxels when it holds sums: (x, y, z) and (x, y, z + 2) */
+	const uint32_t vx = x0 + (lane & 3), vy = y0 + ((lane >> 2) & 3), vz = z0 + (lane >> 4);
+	const size_t v0 = (size_t)Nx * ((size_t)vz * Ny + vy) + vx, v1 = v0 + 2 * (size_t)Nx * Ny;
+	const bool in0 = vx < Nx && vy < Ny && vz < Nz, in1 = vx < Nx && vy < Ny && vz + 2 < Nz;
+	if (warp >= lj_warps) {
+		/* the geometry warps, one chunk ahead (the beads' records two), the
+		 * first of them with the charge channel */
+		const double sp = (double)d.gridSpacing;
+		const float px = (float)__dadd_rn((double)d.posMin[0], __dmul_rn((double)vx, sp));
+		const float py = (float)__dadd_rn((double)d.posMin[1], __dmul_rn((double)vy, sp));
+		float pz[kCube];
 #pragma unroll
-	for (int g = 0; g < kGroup; ++g) acc[g][0] = acc[g][1] = acc[g][2] = acc[g][3] = 0.0;
-	uint32_t tl[kGroup];
-#pragma unroll
-	for (int g = 0; g < kGroup; ++g) {
-		const uint32_t c = c0 + g;
-		tl[g] = (c >= 1 && c < C) ? __ldg(&a.alphabet[c - 1]) : 0u;
-	}
-	for (uint32_t t0 = 0; t0 < a.n; t0 += kTile) {
-		const uint32_t j = t0 + threadIdx.x;
-		if (j < a.n) {
-			sb[threadIdx.x] = __ldg(&a.xyzq[j]);
-			stype[threadIdx.x] = __ldg(&a.tm[j]) & 0xffffu;
-		}
+		for (int z = 0; z < kCube; ++z)
+			pz[z] = (float)__dadd_rn((double)d.posMin[2], __dmul_rn((double)(z0 + z), sp));
+		const bool charge = warp == lj_warps && blockIdx.y == 0, cdiel = a.par.dielec == GBA_DIELEC_CONSTANT;
+		const int i0 = warp == lj_warps ? 0 : kChargePairs, i1 = warp == lj_warps ? kChargePairs : kPairs;
+		double acc[4][2] = {};
+		f2 part[4] = {0, 0, 0, 0};
+		/* lanes past the chunk load its beads again: inside the receptor or nothing */
+		Bead mine = load_bead(a, lane & (kChunk - 1));
+		fill_chunk(a, mine, i0, i1, px, py, pz, lane, buf[0]);
+		mine = load_bead(a, kChunk + (lane & (kChunk - 1)));
 		__syncthreads();
-		const uint32_t tn = min((uint32_t)kTile, a.n - t0);
-		float tacc[kGroup][4];
-#pragma unroll
-		for (int g = 0; g < kGroup; ++g) tacc[g][0] = tacc[g][1] = tacc[g][2] = tacc[g][3] = 0.f;
-		for (uint32_t b = 0; b < tn; ++b) {
-			const uint32_t tr = stype[b];
-			if (tr == 0) continue;
-			const float4 r = sb[b];
-			float ex = fsub(px, r.x), ey = fsub(py, r.y), ez = fsub(pz, r.z);
-			float e2 = fadd(fadd(fmul(ex, ex), fmul(ey, ey)), fmul(ez, ez));
-			bool dirless = false;
-			if (e2 < a.plat2) {
-				if (e2 > 0.f) {
-					const float sc = __fdiv_rn(a.plateau, __fsqrt_rn(e2));
-					ex = fmul(ex, sc); ey = fmul(ey, sc); ez = fmul(ez, sc);
-				} else {
-					dirless = true;
-				}
-				e2 = a.plat2;
+		for (uint32_t k = 0; k < chunks; ++k) {
+			if (k + 1 < chunks) {
+				const Bead now = mine;
+				mine = load_bead(a, (k + 2) * kChunk + (lane & (kChunk - 1)));
+				fill_chunk(a, now, i0, i1, px, py, pz, lane, buf[(k + 1) & 1]);
 			}
-			const float rr2 = __fdiv_rn(1.0f, e2);
-			const float ux = dirless ? 0.f : fmul(ex, rr2), uy = dirless ? 0.f : fmul(ey, rr2),
-					uz = dirless ? 0.f : fmul(ez, rr2);
+			if (charge) {
+				const Chunk& C = buf[k & 1];
+				for (int b = 0; b < kChunk; ++b) {
+					const float qf = C.qf[b];
+					if (qf == 0.f) continue;
+					const VoxelGeo& g = C.geo[b];
+					float i[2], ux[2], uy[2], uz[2], fx[2], fy[2], fz[2], e[2];
+					unpack2(g.rr2[lane], i[0], i[1]);
+					unpack2(g.ux[lane], ux[0], ux[1]);
+					unpack2(g.uy[lane], uy[0], uy[1]);
+					unpack2(g.uz[lane], uz[0], uz[1]);
 #pragma unroll
-			for (int g = 0; g < kGroup; ++g) {
-				const uint32_t c = c0 + g;
-				float fx, fy, fz, e;
-				if (c == 0) {
-					const float qf = fmul(r.w, a.par.ffelec);
-					if (!(fabsf(qf) > 0.001f)) continue;
-					charge_pot_force(rr2, ux, uy, uz, qf, cdiel, fx, fy, fz, e);
-				} else {
-					if (tl[g] == 0 || tl[g] > a.par.num_types || tr > a.par.num_types) continue;
-					const size_t k = (size_t)a.par.num_types * (tr - 1) + (tl[g] - 1);
-					lj_pot_force(e2, rr2, ux, uy, uz, __ldg(&a.par.lj[k]), __ldg(&a.par.ivor[k]),
-							shape86, fx, fy, fz, e);
+					for (int h = 0; h < 2; ++h)
+						charge_pot_force(i[h], ux[h], uy[h], uz[h], qf, cdiel, fx[h], fy[h], fz[h], e[h]);
+					part[0] = add2(part[0], pack2(fx[0], fx[1]));
+					part[1] = add2(part[1], pack2(fy[0], fy[1]));
+					part[2] = add2(part[2], pack2(fz[0], fz[1]));
+					part[3] = add2(part[3], pack2(e[0], e[1]));
 				}
-				tacc[g][0] = fadd(tacc[g][0], fx);
-				tacc[g][1] = fadd(tacc[g][1], fy);
-				tacc[g][2] = fadd(tacc[g][2], fz);
-				tacc[g][3] = fadd(tacc[g][3], e);
+				if ((k + 1) % (kTile / kChunk) == 0 || k + 1 == chunks)
+#pragma unroll
+					for (int c = 0; c < 4; ++c) fold2(part[c], acc[c]);
+			}
+			__syncthreads();
+		}
+		if (charge) {
+			if (in0) out[v0] = make_float4((float)acc[0][0], (float)acc[1][0], (float)acc[2][0], (float)acc[3][0]);
+			if (in1) out[v1] = make_float4((float)acc[0][1], (float)acc[1][1], (float)acc[2][1], (float)acc[3][1]);
+		}
+		return;
+	}
+	const bool shape86 = PLAIN || a.par.potshape == GBA_POTSHAPE_8_6;
+	const uint32_t c0 = blockIdx.y * (kLjWarps * kChan) + warp * kChan;   /* first type channel */
+	const float4* rows = a.rows + 2 * (size_t)c0;
+	/* The assembler fuses a packed product into a packed sum that follows it,
+	 * although both round; a factor of one that it cannot see keeps them apart. */
+	const f2 six = pack2(6.f, 6.f), one = pack2(a.one, a.one);
+	double acc[kChan][4][2] = {};
+	f2 part[kChan][4] = {};
+	__syncthreads();
+	for (uint32_t k = 0; k < chunks; ++k) {
+		const Chunk& C = buf[k & 1];
+#pragma unroll kRowAhead
+		for (int b = 0; b < kChunk; ++b) {
+			const float4* row = rows + 2 * (size_t)(C.row[b] * a.n_lj);
+			const VoxelGeo& g = C.geo[b];
+			const f2 rr2 = g.rr2[lane], ux = g.ux[lane], uy = g.uy[lane], uz = g.uz[lane], rr23 = g.rr23[lane];
+			if (PLAIN) {
+				const f2 dbl = add2(rr23, rr23);
+#pragma unroll
+				for (int i = 0; i < kChan; ++i) {
+					const float4 p = __ldg(row + 2 * i);
+					const f2 rep = mul2(pack2(p.x, p.y), rr2);
+					const f2 vlj = mul2(add2(rep, pack2(p.z, p.w)), rr23);
+					const f2 fb = fma2(six, vlj, mul2(rep, dbl));
+					part[i][0] = fma2(mul2(fb, ux), one, part[i][0]);
+					part[i][1] = fma2(mul2(fb, uy), one, part[i][1]);
+					part[i][2] = fma2(mul2(fb, uz), one, part[i][2]);
+					part[i][3] = add2(part[i][3], vlj);
+				}
+			} else {
+				const f2 sd = shape86 ? pack2(2.f, 2.f) : six;
+				const f2 rrd = shape86 ? rr2 : rr23;
+				float da, db;
+				unpack2(g.d2[lane], da, db);
+#pragma unroll
+				for (int i = 0; i < kChan; ++i) {
+					const float4 p = __ldg(row + 2 * i), m = __ldg(row + 2 * i + 1);   /* m: ipon, ipon, rmin2, emin */
+					const f2 rep = mul2(pack2(p.x, p.y), rrd);
+					const f2 vlj = mul2(add2(rep, pack2(p.z, p.w)), rr23);
+					const f2 fb = fma2(six, vlj, mul2(sd, mul2(rep, rr23)));
+					const f2 iv = pack2(m.x, m.y), off = pack2(fsub(m.x, 1.0f), fsub(m.x, 1.0f));
+					float e_in[2], e_out[2], f_in[2], f_out[2];
+					unpack2(fma2(off, pack2(m.w, m.w), vlj), e_in[0], e_in[1]);
+					unpack2(mul2(iv, vlj), e_out[0], e_out[1]);
+					unpack2(fb, f_in[0], f_in[1]);
+					unpack2(mul2(iv, fb), f_out[0], f_out[1]);
+					const f2 e = pack2(da < m.z ? e_in[0] : e_out[0], db < m.z ? e_in[1] : e_out[1]);
+					const f2 f = pack2(da < m.z ? f_in[0] : f_out[0], db < m.z ? f_in[1] : f_out[1]);
+					part[i][0] = fma2(mul2(f, ux), one, part[i][0]);
+					part[i][1] = fma2(mul2(f, uy), one, part[i][1]);
+					part[i][2] = fma2(mul2(f, uz), one, part[i][2]);
+					part[i][3] = add2(part[i][3], e);
+				}
 			}
 		}
+		if ((k + 1) % (kTile / kChunk) == 0 || k + 1 == chunks)
 #pragma unroll
-		for (int g = 0; g < kGroup; ++g)
+			for (int i = 0; i < kChan; ++i)
 #pragma unroll
-			for (int k = 0; k < 4; ++k) acc[g][k] = __dadd_rn(acc[g][k], (double)tacc[g][k]);
+				for (int c = 0; c < 4; ++c) fold2(part[i][c], acc[i][c]);
 		__syncthreads();
 	}
-	if (!valid) return;
 #pragma unroll
-	for (int g = 0; g < kGroup; ++g) {
-		const uint32_t c = c0 + g;
-		if (c < C)
-			out[(size_t)c * N + v] = make_float4((float)acc[g][0], (float)acc[g][1],
-					(float)acc[g][2], (float)acc[g][3]);
+	for (int i = 0; i < kChan; ++i)
+		if (c0 + i < a.n_alphabet) {
+			float4* o = out + (size_t)(1 + c0 + i) * N;
+			if (in0) o[v0] = make_float4((float)acc[i][0][0], (float)acc[i][1][0], (float)acc[i][2][0], (float)acc[i][3][0]);
+			if (in1) o[v1] = make_float4((float)acc[i][0][1], (float)acc[i][1][1], (float)acc[i][2][1], (float)acc[i][3][1]);
+		}
+}
+
+/* The three conditions of grid_potential_kernel's plain form, over the whole
+ * table; reach2: a bound of the squared distance between a voxel and a bead. */
+bool plain_pairs(const std::vector<gba_ffparam>& table, int potshape, float plat2, double reach2) {
+	if (potshape != GBA_POTSHAPE_8_6 || !(plat2 >= 1e-6f)) return false;
+	for (const gba_ffparam& p : table) {
+		if (p.ipon != 1 || p.rmin2 > plat2 || !std::isfinite(p.rc)) return false;
+		/* rep rr23 >= rc / reach2^4 has to stay a normal number */
+		if (p.rc != 0.f && std::fabs((double)p.rc) / (reach2 * reach2 * reach2 * reach2) < 1e-36) return false;
 	}
+	return true;
+}
+
+void launch_potentials(const BuildArgs& a, bool plain, const gba_intrpl_desc& d, float4* out, cudaStream_t s) {
+	uint64_t bricks = 1;
+	for (int k = 0; k < 3; ++k) bricks *= (d.dimN[k] + kCube - 1) / kCube;
+	const uint32_t warps = (a.n_alphabet + kChan - 1) / kChan;      /* type channels, in warps */
+	const unsigned groups = std::max<uint32_t>(1, (warps + kLjWarps - 1) / kLjWarps);
+	const unsigned threads = 32 * (std::min<uint32_t>(warps, kLjWarps) + 2);
+	if (plain)
+		grid_potential_kernel<true><<<dim3((unsigned)bricks, groups), threads, 0, s>>>(a, d, out);
+	else
+		grid_potential_kernel<false><<<dim3((unsigned)bricks, groups), threads, 0, s>>>(a, d, out);
+	check_cuda(cudaGetLastError(), "grid build: potentials");
 }
 
 /* Neighbour membership, unfused double arithmetic (bit-identical to the CPU builder). */
@@ -399,20 +644,32 @@ extern "C" int gba_build_grid(gba_ctx* ctx, gba_id rec, gba_id params,
 		a.xyzq = R->dev.xyzq;
 		a.tm = R->dev.tm;
 		a.n = R->dev.n;
+		a.one = 1.0f;
 		a.par = P->dev;
-		a.alphabet = (const uint32_t*)alpha.ptr;
 		a.n_alphabet = opt->n_alphabet;
 		a.plateau = opt->plateau;
 		a.plat2 = opt->plateau * opt->plateau;
 		a.cut2 = (double)opt->nl_cutoff * opt->nl_cutoff;
 		cudaStream_t s = 0;
-		const unsigned groups = (C + kGroup - 1) / kGroup;
-		grid_potential_kernel<<<dim3((unsigned)((Ni + kTile - 1) / kTile), groups), kTile, 0, s>>>(
-				a, item->inner_desc, (float4*)item->inner.ptr);
-		check_cuda(cudaGetLastError(), "grid build: inner launch");
-		grid_potential_kernel<<<dim3((unsigned)((No + kTile - 1) / kTile), groups), kTile, 0, s>>>(
-				a, item->outer_desc, (float4*)item->outer.ptr);
-		check_cuda(cudaGetLastError(), "grid build: outer launch");
+		/* whole blocks of channel warps, so that every warp's row loads stay inside */
+		a.n_lj = (opt->n_alphabet + kLjWarps * kChan - 1) / (kLjWarps * kChan) * (kLjWarps * kChan);
+		const size_t nrow = (size_t)(a.par.num_types + 1) * a.n_lj;
+		DevBuffer rows;
+		rows.alloc(std::max<size_t>(1, nrow) * 2 * sizeof(float4));
+		a.rows = (const float4*)rows.ptr;
+		if (nrow > 0) {
+			pair_rows_kernel<<<(unsigned)((nrow + 255) / 256), 256, 0, s>>>(a.par, (const uint32_t*)alpha.ptr, a.n_alphabet,
+					a.n_lj, (float4*)rows.ptr);
+			check_cuda(cudaGetLastError(), "grid build: pair rows");
+		}
+		double reach2 = 0.0;      /* beads lie inside the outer grid's box */
+		for (int k = 0; k < 3; ++k) {
+			const double e = (item->outer_desc.dimN[k] + kCube) * (double)item->outer_desc.gridSpacing;
+			reach2 += e * e;
+		}
+		const bool plain = plain_pairs(P->host_table, a.par.potshape, a.plat2, reach2);
+		launch_potentials(a, plain, item->inner_desc, (float4*)item->inner.ptr, s);
+		launch_potentials(a, plain, item->outer_desc, (float4*)item->outer.ptr, s);
 		DevBuffer counts, sums;
 		counts.alloc(Ni * sizeof(uint32_t));
 		const gba_nl_desc& nd = item->nl_desc;

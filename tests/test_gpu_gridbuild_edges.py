@@ -38,3 +38,31 @@ def test_lists_at_tile_edges(pkg, oracle, n, spacing, cutoff, offset):
     assert tuple(got.nl.dimN) == tuple(nl.dimN) and got.nl.numEl == nl.numEl
     assert np.array_equal(got.nl_grid, ng)
     assert np.array_equal(got.nl_list, lst)
+
+
+@pytest.mark.parametrize("n,n_types,shape,ipon,dielec,plateau,spacing", [
+    (1, 3, 1, 1, 1, 10.0, 2.0),          # one bead: partial chunk and tile
+    (16, 4, 1, 1, 0, 10.0, 1.9),         # exactly a chunk, a full channel warp, constant dielectric
+    (17, 5, 1, 1, 1, 10.0, 2.1),         # one channel past a warp
+    (256, 32, 1, 1, 1, 10.0, 3.1),       # exactly a tile and a block of channels
+    (257, 33, 1, 1, 1, 10.0, 3.3),       # one past both
+    (300, 32, 1, -1, 1, 10.0, 3.0),      # repulsive pairs: the general form
+    (300, 7, 1, 1, 1, 3.0, 2.6),         # minima beyond the plateau
+    (300, 9, 0, 1, 1, 10.0, 2.9),        # 12-6
+    (40, 0, 1, 1, 1, 10.0, 2.0),         # the charge channel alone
+])
+def test_potentials_at_tile_edges(pkg, oracle, n, n_types, shape, ipon, dielec, plateau, spacing):
+    rec, _ = _receptor(pkg, n, (0.0, 0.0, 0.0), 90 + n)
+    rng = np.random.default_rng(7)
+    T = max(n_types, 33)
+    table = pkg.model.attract_params(rng.uniform(3, 5, (T, T)), rng.uniform(0.1, 10, (T, T)),
+                                     ipon=np.where(rng.random((T, T)) < 0.3, ipon, 1).astype(np.int32), potshape=shape)
+    params = pkg.model.ParamTable(table=table, potshape=shape, dielec=dielec)
+    opts = pkg.GridOptions(spacing=spacing, plateau=plateau, outer_ext=9, alphabet=list(range(1, n_types + 1)))
+    from gbattract.context import GbaContext
+    with GbaContext(0) as ctx:
+        got = ctx.download_grid(ctx.build_grid(ctx.upload_protein(rec), ctx.upload_params(params), opts))
+    want = oracle.build_grid(rec, params, opts)
+    assert np.array_equal(got.inner_data.view(np.uint32), want.inner_data.view(np.uint32))
+    assert np.array_equal(got.outer_data.view(np.uint32), want.outer_data.view(np.uint32))
+    assert np.array_equal(got.nl_grid, want.nl_grid) and np.array_equal(got.nl_list, want.nl_list)
