@@ -55,7 +55,7 @@ struct PairwiseLaunch {
 	const float4* tab;     /* 3*T*T: per type pair the constants of lj86 (lj_table_kernel) */
 	const float4* rq;      /* rec.n: receptor x, y, z and this call's charge (pack_receptor_kernel) */
 	const uint32_t* tlist; /* the neighbour list with receptor types in bits 24..31, or nullptr */
-	unsigned long long* next;   /* pose counter, zero at launch (PoseFeed) */
+	unsigned long long* next;   /* pose counter, zero at launch (next_pose) */
 	const uint32_t* order;      /* visiting order (nearest ligands first), or nullptr */
 };
 
@@ -177,7 +177,7 @@ constexpr size_t kNearFirstMinPoses = 2048;
  * lane-per-bead staging (transform, neighbour-list voxel), then the round's
  * flattened (bead, neighbour) pairs in windows of 64, two per lane, so that
  * uneven list lengths do not idle lanes.  A warp takes its next pose from a
- * global counter when it finishes one (PoseFeed). */
+ * global counter when it finishes one (next_pose). */
 template <bool BACKWARD>
 __global__ void __launch_bounds__(kPairwiseThreads) pairwise_kernel(const PairwiseLaunch L) {
 	extern __shared__ double sm[];
@@ -195,8 +195,7 @@ __global__ void __launch_bounds__(kPairwiseThreads) pairwise_kernel(const Pairwi
 	const int lane = threadIdx.x & 31;
 	PairStage& W = stage[threadIdx.x >> 5];
 	const bool cdiel = L.dielec == GBA_DIELEC_CONSTANT;
-	PoseFeed feed(L.next);
-	for (size_t slot = feed.take(lane); slot < L.n; slot = feed.take(lane)) {
+	for (size_t slot = next_pose(L.next, lane); slot < L.n; slot = next_pose(L.next, lane)) {
 		const size_t p = L.order ? (size_t)__ldg(&L.order[slot]) : slot;
 		const float* dofp = reinterpret_cast<const float*>(L.dofs + p);
 		const float dv = lane < 6 ? __ldg(dofp + lane) : 0.f;

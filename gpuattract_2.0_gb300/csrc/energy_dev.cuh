@@ -46,33 +46,26 @@ struct PoseRot {
 	float cphi, sphi, cssi, sssi, crot, srot;
 };
 
-/* Lanes 0..2 each take one Euler angle (phi, ssi, rot) through double sincos
- * -- or, for angles the host table T covers, the host C library's sinf/cosf
- * read from it; the 6 values are broadcast and combined as euler2rotmat does
- * (src/model/matrixFunctions.h:40-77), unfused. */
-__device__ __forceinline__ PoseRot pose_rotation(float phi, float ssi, float rot, int lane, const DevTrig& T) {
-	float a = lane == 0 ? phi : (lane == 1 ? ssi : rot);
-	float s = 0.f, c = 1.f;
-	if (lane < 3) {
-		const uint32_t b = __float_as_uint(a), mag = b & 0x7fffffffu;
-		if (T.sc && mag >= T.lo && mag < T.hi) {
-			const float2 v = __ldg(&T.sc[(size_t)(b >> 31) * (T.hi - T.lo) + (mag - T.lo)]);
-			s = v.x;
-			c = v.y;
-		} else {
-			double sd, cd;
-			sincos((double)a, &sd, &cd);
-			s = (float)sd;
-			c = (float)cd;
-		}
+/* sin and cos of one Euler angle: double sincos rounded to float -- or, for
+ * angles the host table T covers, the host C library's sinf/cosf read from
+ * it. */
+__device__ __forceinline__ void angle_sincos(float a, const DevTrig& T, float& s, float& c) {
+	const uint32_t b = __float_as_uint(a), mag = b & 0x7fffffffu;
+	if (T.sc && mag >= T.lo && mag < T.hi) {
+		const float2 v = __ldg(&T.sc[(size_t)(b >> 31) * (T.hi - T.lo) + (mag - T.lo)]);
+		s = v.x;
+		c = v.y;
+	} else {
+		double sd, cd;
+		sincos((double)a, &sd, &cd);
+		s = (float)sd;
+		c = (float)cd;
 	}
-	PoseRot R;
-	R.cphi = __shfl_sync(GBA_FULL_MASK, c, 0);
-	R.sphi = __shfl_sync(GBA_FULL_MASK, s, 0);
-	R.cssi = __shfl_sync(GBA_FULL_MASK, c, 1);
-	R.sssi = __shfl_sync(GBA_FULL_MASK, s, 1);
-	R.crot = __shfl_sync(GBA_FULL_MASK, c, 2);
-	R.srot = __shfl_sync(GBA_FULL_MASK, s, 2);
+}
+
+/* The matrix of R's sin/cos as euler2rotmat combines them
+ * (src/model/matrixFunctions.h:40-77), unfused. */
+__device__ __forceinline__ void rot_matrix(PoseRot& R) {
 	const float cSSI_cPHI = fmul(R.cssi, R.cphi);
 	const float cSSI_sPHI = fmul(R.cssi, R.sphi);
 	const float sSSI_cPHI = fmul(R.sssi, R.cphi);
@@ -86,6 +79,22 @@ __device__ __forceinline__ PoseRot pose_rotation(float phi, float ssi, float rot
 	R.m[6] = fmul(-R.crot, R.sssi);
 	R.m[7] = fmul(-R.srot, R.sssi);
 	R.m[8] = R.cssi;
+}
+
+/* Lanes 0..2 each take one Euler angle (phi, ssi, rot); the 6 values go to
+ * every lane. */
+__device__ __forceinline__ PoseRot pose_rotation(float phi, float ssi, float rot, int lane, const DevTrig& T) {
+	const float a = lane == 0 ? phi : (lane == 1 ? ssi : rot);
+	float s = 0.f, c = 1.f;
+	if (lane < 3) angle_sincos(a, T, s, c);
+	PoseRot R;
+	R.cphi = __shfl_sync(GBA_FULL_MASK, c, 0);
+	R.sphi = __shfl_sync(GBA_FULL_MASK, s, 0);
+	R.cssi = __shfl_sync(GBA_FULL_MASK, c, 1);
+	R.sssi = __shfl_sync(GBA_FULL_MASK, s, 1);
+	R.crot = __shfl_sync(GBA_FULL_MASK, c, 2);
+	R.srot = __shfl_sync(GBA_FULL_MASK, s, 2);
+	rot_matrix(R);
 	return R;
 }
 
@@ -200,30 +209,16 @@ __device__ __forceinline__ void charge_pot_force(float dr2_inv, float dx, float 
 	}
 }
 
-/* Pose indices of one warp, identical on all lanes.  With a counter (zero
- * at launch) the warp takes the next unclaimed index whenever it finishes a
- * pose: per-pose cost varies by orders of magnitude (contact poses walk
- * thousands of neighbour pairs, distant ones none), and a fixed stride left
- * warps idle while others finished their share.  Without one, the fixed
- * stride warp, warp + nwarps, ... */
-struct PoseFeed {
-	unsigned long long* next;
-	size_t k, stride;
-	__device__ __forceinline__ PoseFeed(unsigned long long* counter)
-		: next(counter),
-		  k(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5),
-		  stride(((size_t)gridDim.x * blockDim.x) >> 5) {}
-	__device__ __forceinline__ size_t take(int lane) {
-		if (next) {
-			unsigned long long t = 0;
-			if (lane == 0) t = atomicAdd(next, 1ull);
-			return (size_t)__shfl_sync(GBA_FULL_MASK, t, 0);
-		}
-		const size_t r = k;
-		k += stride;
-		return r;
-	}
-};
+/* The warp's next pose (or round), identical on all lanes: the next
+ * unclaimed index of a counter that is zero at launch.  Per-pose cost varies
+ * by orders of magnitude (contact poses walk thousands of neighbour pairs,
+ * distant ones none), and a fixed stride left warps idle while others
+ * finished their share. */
+__device__ __forceinline__ size_t next_pose(unsigned long long* counter, int lane) {
+	unsigned long long t = 0;
+	if (lane == 0) t = atomicAdd(counter, 1ull);
+	return (size_t)__shfl_sync(GBA_FULL_MASK, t, 0);
+}
 
 /* Butterfly sum across the warp. */
 __device__ __forceinline__ float warp_sum(float v) {

@@ -736,8 +736,7 @@ __global__ void __launch_bounds__(kModesRecThreads, kModesRecBlocks) modes_rec_k
 	const int lane = threadIdx.x & 31;
 	const int wib = threadIdx.x >> 5;
 	const uint32_t Mr = L.rec.n_modes;
-	PoseFeed feed(L.next);
-	for (size_t p = feed.take(lane); p < L.n; p = feed.take(lane)) {
+	for (size_t p = next_pose(L.next, lane); p < L.n; p = next_pose(L.next, lane)) {
 		const float* d = reinterpret_cast<const float*>(L.dofs + p);
 		const float dv = lane < 26 ? __ldg(d + lane) : 0.f;
 		float ampR[MM], ampL[MM];
@@ -761,8 +760,7 @@ __global__ void __launch_bounds__(kModesThreads, 2) modes_lig_kernel(const Modes
 	const int lane = threadIdx.x & 31;
 	const int wib = threadIdx.x >> 5;
 	const uint32_t Mr = L.rec.n_modes;
-	PoseFeed feed(L.next2);
-	for (size_t p = feed.take(lane); p < L.n; p = feed.take(lane)) {
+	for (size_t p = next_pose(L.next2, lane); p < L.n; p = next_pose(L.next2, lane)) {
 		const float* d = reinterpret_cast<const float*>(L.dofs + p);
 		const float dv = lane < 26 ? __ldg(d + lane) : 0.f;
 		float ampR[MM], ampL[MM];
@@ -793,8 +791,7 @@ __global__ void __launch_bounds__(kModesRefThreads) modes_ref_kernel(const Modes
 	const int lane = threadIdx.x & 31;
 	const int wib = threadIdx.x >> 5;
 	float4* rf = L.ref_rf + (((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * L.rec.n;
-	PoseFeed feed(L.next);
-	for (size_t p = feed.take(lane); p < L.n; p = feed.take(lane)) {
+	for (size_t p = next_pose(L.next, lane); p < L.n; p = next_pose(L.next, lane)) {
 		const float* d = reinterpret_cast<const float*>(L.dofs + p);
 		const float dv = lane < 26 ? __ldg(d + lane) : 0.f;
 		const float v = eval_pose_modes_ref<MM>(L, dv, lane, stage[wib], extra[wib], rf);

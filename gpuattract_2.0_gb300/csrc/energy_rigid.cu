@@ -9,8 +9,10 @@
  *   d_NLPotForce     src/model/neighborlist.cu:21-171    NL pair term
  *   blockReduce      src/model/reduction.cu:50-391       13 sums per pose
  *   h_finalReduce    src/model/reduction.h:160-205       ForceLim + TorqueMat
- * by one kernel in which a warp owns a pose (grid-stride over poses) and
- * nothing per bead leaves the SM; lanes 0..6 store the 28-byte Result_6D.
+ * by one kernel in which a warp owns a pose and nothing per bead leaves the
+ * SM; lanes 0..6 store the 28-byte Result_6D.  Batches too small to keep every
+ * warp slot busy for several poses split each pose into its 64-bead rounds
+ * (rigid_rounds_kernel).
  */
 #include <atomic>
 
@@ -19,14 +21,12 @@
 namespace gba {
 
 /* BOUND4: registers capped for four resident 256-thread blocks per SM
- * (GBA_KOPT_FOUR_BLOCKS).  ROUNDWISE: the minimizers' round-wise summation
- * order (the plain per-step minimization form's launches). */
-template <bool CENSUS, bool BOUND4, bool ROUNDWISE = false>
+ * (GBA_KOPT_FOUR_BLOCKS). */
+template <bool CENSUS, bool BOUND4>
 __global__ void __launch_bounds__(256, BOUND4 ? 4 : 1) rigid_energy_kernel(const RigidLaunch L) {
 	__shared__ WarpStage stage[8];   /* one per warp of a <=256-thread block */
 	const int lane = threadIdx.x & 31;
-	PoseFeed feed(L.next);
-	for (size_t k = feed.take(lane); k < L.n; k = feed.take(lane)) {
+	for (size_t k = next_pose(L.next, lane); k < L.n; k = next_pose(L.next, lane)) {
 		const size_t p = L.order ? (size_t)__ldg(&L.order[k]) : k;
 		const float* dofp = reinterpret_cast<const float*>(L.dofs + p);
 		const float dv = lane < 6 ? __ldg(dofp + lane) : 0.f;
@@ -37,9 +37,87 @@ __global__ void __launch_bounds__(256, BOUND4 ? 4 : 1) rigid_energy_kernel(const
 		const float a1 = __shfl_sync(GBA_FULL_MASK, dv, 4);
 		const float a2 = __shfl_sync(GBA_FULL_MASK, dv, 5);
 		float res[7];
-		eval_pose_rigid<CENSUS, ROUNDWISE>(L.m, tx, ty, tz, a0, a1, a2, lane, stage[threadIdx.x >> 5], res,
-				CENSUS ? L.census + p : nullptr);
+		WarpStage& W = stage[threadIdx.x >> 5];
+		if (lane == 0) W.slot = p;
+		eval_pose_rigid<CENSUS>(L.m, tx, ty, tz, a0, a1, a2, lane, W, res, CENSUS ? L.census + p : nullptr);
+		store_result7(reinterpret_cast<float*>(L.out + *(volatile unsigned long long*)&W.slot), res, lane);
+		__syncwarp();
+	}
+}
+
+/* Before rigid_rounds_kernel: each pose's rotation and translation as the
+ * staging area holds them (a warp per round would repeat the double sincos,
+ * whose pipe issues one warp instruction per 16 cycles and SM, once a round),
+ * and its count of finished rounds and the launch's counter cleared.  Four
+ * lanes per pose, one Euler angle each. */
+__global__ void __launch_bounds__(128) rigid_setup_kernel(const RigidLaunch L) {
+	const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+	const size_t p = t >> 2;
+	const int lane = threadIdx.x & 31, j = lane & 3, base = lane & ~3;
+	const bool in = p < L.n;
+	const float* d = reinterpret_cast<const float*>(L.dofs + (in ? p : 0));
+	float s = 0.f, c = 1.f;
+	if (j < 3) angle_sincos(__ldg(d + 3 + j), L.m.trig, s, c);
+	PoseRot R;
+	R.cphi = __shfl_sync(GBA_FULL_MASK, c, base);
+	R.sphi = __shfl_sync(GBA_FULL_MASK, s, base);
+	R.cssi = __shfl_sync(GBA_FULL_MASK, c, base + 1);
+	R.sssi = __shfl_sync(GBA_FULL_MASK, s, base + 1);
+	R.crot = __shfl_sync(GBA_FULL_MASK, c, base + 2);
+	R.srot = __shfl_sync(GBA_FULL_MASK, s, base + 2);
+	rot_matrix(R);
+	if (t == 0) *L.next = 0;
+	if (!in) return;
+	float4* o = reinterpret_cast<float4*>(L.split.pose + kPoseRecord * p);
+	if (j == 0) {
+		o[0] = make_float4(R.m[0], R.m[1], R.m[2], R.m[3]);
+		L.split.done[p] = 0;
+	} else if (j == 1) {
+		o[1] = make_float4(R.m[4], R.m[5], R.m[6], R.m[7]);
+	} else if (j == 2) {
+		o[2] = make_float4(R.m[8], R.cphi, R.sphi, R.cssi);
+	} else {
+		o[3] = make_float4(R.sssi, R.crot, R.srot, __ldg(d));
+		o[4] = make_float4(__ldg(d + 1), __ldg(d + 2), 0.f, 0.f);
+	}
+}
+
+/* A warp takes one 64-bead round of a pose at a time; the warp that finishes
+ * a pose's last round adds the totals of all of them in round order, so the
+ * result is eval_pose_rigid's bit for bit.  Bound by the latency of one
+ * round, where a warp walking whole poses is bound by the sum of them. */
+__global__ void __launch_bounds__(256, 4) rigid_rounds_kernel(const RigidLaunch L) {
+	__shared__ WarpStage stage[8];
+	const int lane = threadIdx.x & 31;
+	WarpStage& W = stage[threadIdx.x >> 5];
+	const uint32_t rounds = L.split.rounds;
+	const size_t units = L.n * rounds;
+	for (size_t u = next_pose(L.next, lane); u < units; u = next_pose(L.next, lane)) {
+		const size_t k = u / rounds;
+		const uint32_t r = (uint32_t)(u - k * rounds);
+		const size_t p = L.order ? (size_t)__ldg(&L.order[k]) : k;
+		if (lane < 18) W.pose[lane] = __ldg(L.split.pose + kPoseRecord * p + lane);
+		__syncwarp();
+		RoundCensus cen;
+		PoseSums S = held_sums();
+		eval_round<false>(L.m, r * kBeadsPerRound, lane, W, cen, S);
+		const float v = round_total(S, W, lane);
+		float* tot = L.split.totals + (size_t)p * rounds * 16 + (lane >> 1);
+		if ((lane & 1) == 0) __stcg(tot + 16 * r, v);
+		/* the pose's last round: release this total, then acquire the others */
+		__threadfence();
+		__syncwarp();
+		uint32_t before = 0;
+		if (lane == 0) before = atomicAdd(&L.split.done[p], 1u);
+		before = __shfl_sync(GBA_FULL_MASK, before, 0);
+		if (before + 1 != rounds) continue;
+		__threadfence();
+		clear_totals(W, lane);
+		for (uint32_t q = 0; q < rounds; ++q) add_round(W, __ldcg(tot + 16 * q), lane);
+		float res[7];
+		finish_pose(W, res);
 		store_result7(reinterpret_cast<float*>(L.out + p), res, lane);
+		__syncwarp();
 	}
 }
 
@@ -52,8 +130,7 @@ __global__ void __launch_bounds__(256, BOUND4 ? 4 : 1) rigid_energy_kernel(const
 __global__ void __launch_bounds__(256, 4) rigid_energy_ref_kernel(const RigidLaunch L) {
 	__shared__ WarpStage stage[8];
 	const int lane = threadIdx.x & 31;
-	PoseFeed feed(L.next);
-	for (size_t k = feed.take(lane); k < L.n; k = feed.take(lane)) {
+	for (size_t k = next_pose(L.next, lane); k < L.n; k = next_pose(L.next, lane)) {
 		const size_t p = L.order ? (size_t)__ldg(&L.order[k]) : k;
 		const float* dofp = reinterpret_cast<const float*>(L.dofs + p);
 		const float dv = lane < 6 ? __ldg(dofp + lane) : 0.f;
@@ -71,8 +148,7 @@ template <bool REF>
 __global__ void __launch_bounds__(256) batch_energy_kernel(const BatchEnergyLaunch L) {
 	__shared__ WarpStage stage[8];   /* one per warp of a <=256-thread block */
 	const int lane = threadIdx.x & 31;
-	PoseFeed feed(L.next);
-	for (size_t p = feed.take(lane); p < L.n; p = feed.take(lane)) {
+	for (size_t p = next_pose(L.next, lane); p < L.n; p = next_pose(L.next, lane)) {
 		const RigidModel& M = L.models[__ldg(&L.pair_of[p])];
 		const float* dofp = reinterpret_cast<const float*>(L.dofs + p);
 		const float dv = lane < 6 ? __ldg(dofp + lane) : 0.f;
@@ -102,10 +178,6 @@ cudaError_t launch_rigid_energy(const RigidLaunch& L, int blocks, int threads, c
 		rigid_energy_kernel<true, false><<<blocks, threads, 0, s>>>(L);
 	else if (L.ref_order)
 		rigid_energy_ref_kernel<<<blocks, threads, 0, s>>>(L);
-	else if (L.roundwise && L.bound4)
-		rigid_energy_kernel<false, true, true><<<blocks, threads, 0, s>>>(L);
-	else if (L.roundwise)
-		rigid_energy_kernel<false, false, true><<<blocks, threads, 0, s>>>(L);
 	else if (L.bound4)
 		rigid_energy_kernel<false, true><<<blocks, threads, 0, s>>>(L);
 	else
@@ -113,27 +185,31 @@ cudaError_t launch_rigid_energy(const RigidLaunch& L, int blocks, int threads, c
 	return cudaGetLastError();
 }
 
+cudaError_t launch_rigid_rounds(const RigidLaunch& L, int blocks, int threads, cudaStream_t s) {
+	rigid_setup_kernel<<<(unsigned)((4 * L.n + 127) / 128), 128, 0, s>>>(L);
+	rigid_rounds_kernel<<<blocks, threads, 0, s>>>(L);
+	return cudaGetLastError();
+}
+
 /* resident blocks per SM, queried once per device, instantiation and block
  * size (the query costs host time on every launch otherwise) */
-int rigid_blocks_per_sm(int threads, bool census, bool bound4, bool roundwise, bool ref_order) {
-	static std::atomic<int> cache[64][6][33];
+int rigid_blocks_per_sm(int threads, bool census, bool bound4, bool ref_order, bool rounds) {
+	static std::atomic<int> cache[64][5][33];
 	int dev = 0;
 	cudaGetDevice(&dev);
-	const int v = census ? 0 : ref_order ? 5 : (roundwise ? (bound4 ? 3 : 4) : (bound4 ? 1 : 2)), t = threads / 32;
+	const int v = rounds ? 4 : census ? 0 : ref_order ? 1 : bound4 ? 2 : 3, t = threads / 32;
 	const bool cacheable = dev >= 0 && dev < 64 && threads % 32 == 0 && t >= 1 && t <= 32;
 	if (cacheable) {
 		const int c = cache[dev][v][t].load(std::memory_order_relaxed);
 		if (c > 0) return c;
 	}
 	int nb = 0;
-	if (census)
+	if (rounds)
+		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rigid_rounds_kernel, threads, 0);
+	else if (census)
 		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rigid_energy_kernel<true, false>, threads, 0);
 	else if (ref_order)
 		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rigid_energy_ref_kernel, threads, 0);
-	else if (roundwise && bound4)
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rigid_energy_kernel<false, true, true>, threads, 0);
-	else if (roundwise)
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rigid_energy_kernel<false, false, true>, threads, 0);
 	else if (bound4)
 		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rigid_energy_kernel<false, true>, threads, 0);
 	else

@@ -780,21 +780,56 @@ void Context::run_modes(ModesLaunch& L, cudaStream_t s) {
 	check_cuda(launch_modes_energy(L, num_sms, s), "modes energy launch");
 }
 
+namespace {
+
+/* A scoring launch is split into 64-bead rounds (rigid_rounds_kernel) while it
+ * brings at most this many poses per resident warp: there the slowest warp's
+ * whole poses set the time, beyond it the rounds' extra records and totals
+ * cost more than the shorter tail saves.  Measured, whole poses against rounds
+ * (4,864 warps): 2000/700 beads 100 poses 302 -> 48 us, 2,000 318 -> 137,
+ * 10,000 (2.1 a warp) 692 -> 572, 30,000 (6.2) 1572 -> 1567, 100,000 4658 ->
+ * 5057; 500/200 beads 10,000 248 -> 237, 30,000 523 -> 547. */
+constexpr size_t kSplitPosesPerWarp = 4;
+/* and its totals stay below this (ligands of thousands of beads) */
+constexpr size_t kSplitBytes = (size_t)64 << 20;
+
+}  // namespace
+
 void Context::run_rigid(RigidLaunch& L, cudaStream_t s, const TuneParams* shape) {
 	StreamScratch scratch(scratch_pool);
 	L.order = pose_order(L.dofs, 6, L.n, L.m.grid.outer, s, scratch);
-	L.next = (unsigned long long*)scratch.get(sizeof(unsigned long long), s);
-	check_cuda(cudaMemsetAsync(L.next, 0, sizeof(unsigned long long), s), "rigid energy: pose counter");
 	const TuneParams tp = shape ? *shape : tuned("energy", L.n);
-	const int threads = tp.threads;
-	const int warps_per_block = threads / 32;
-	const int bps = std::min(tp.blocks_per_sm, rigid_blocks_per_sm(threads, L.census != nullptr, L.bound4 && !L.census,
-			L.roundwise && !L.census, L.ref_order && !L.census));
-	size_t want = (L.n + warps_per_block - 1) / warps_per_block;
-	size_t blocks = std::min<size_t>(want, (size_t)num_sms * bps);
-	if (blocks == 0) blocks = 1;
+	const size_t rounds = (L.m.lig.n + 63) / 64;
+	const bool split = !L.census && !L.ref_order && rounds > 1 &&
+			L.n <= kSplitPosesPerWarp * num_sms * 8 * rigid_blocks_per_sm(256, false, false, false, true) &&
+			L.n * rounds * 16 * sizeof(float) <= kSplitBytes;
+	/* a tuned shape was timed on the launch of whole poses */
+	const int threads = split ? 256 : tp.threads;
+	const size_t warps_per_block = threads / 32;
+	const int bps = split ? rigid_blocks_per_sm(256, false, false, false, true)
+			: std::min(tp.blocks_per_sm, rigid_blocks_per_sm(threads, L.census != nullptr, L.bound4 && !L.census,
+					L.ref_order && !L.census));
+	if (split) {
+		/* one block: the records, the totals, the counts, the counter */
+		const size_t rec = L.n * kPoseRecord * sizeof(float), tot = L.n * rounds * 16 * sizeof(float);
+		char* b = (char*)scratch.get(rec + tot + L.n * sizeof(uint32_t) + 16, s);
+		L.split.pose = (float*)b;
+		L.split.totals = (float*)(b + rec);
+		L.next = (unsigned long long*)(b + rec + tot);
+		L.split.done = (uint32_t*)(b + rec + tot + 16);
+		L.split.rounds = (uint32_t)rounds;
+	} else {
+		L.next = (unsigned long long*)scratch.get(sizeof(unsigned long long), s);
+		check_cuda(cudaMemsetAsync(L.next, 0, sizeof(unsigned long long), s), "rigid energy: pose counter");
+	}
+	const size_t want = (L.n * (split ? rounds : 1) + warps_per_block - 1) / warps_per_block;
+	const int blocks = (int)std::max<size_t>(1, std::min<size_t>(want, (size_t)num_sms * bps));
+	auto launch = [&] {
+		check_cuda(split ? launch_rigid_rounds(L, blocks, threads, s) : launch_rigid_energy(L, blocks, threads, s),
+				"rigid energy launch");
+	};
 	if (!timing) {
-		check_cuda(launch_rigid_energy(L, (int)blocks, threads, s), "rigid energy launch");
+		launch();
 		return;
 	}
 	if (timing_used == kTimingPool) timing_fold();
@@ -806,7 +841,7 @@ void Context::run_rigid(RigidLaunch& L, cudaStream_t s, const TuneParams* shape)
 	}
 	auto& e = timing_events[timing_used];
 	check_cuda(cudaEventRecord(e.first, s), "kernel timing: record");
-	check_cuda(launch_rigid_energy(L, (int)blocks, threads, s), "rigid energy launch");
+	launch();
 	check_cuda(cudaEventRecord(e.second, s), "kernel timing: record");
 	++timing_used;
 }

@@ -117,6 +117,17 @@ struct RigidModel {
 	DevTrig trig;
 };
 
+/* Scratch of a launch split into rounds: per pose its rotation, sin/cos and
+ * translation (kPoseRecord floats: WarpStage::pose, padded), the rounds
+ * finished so far, and the totals of each round (16 floats). */
+constexpr int kPoseRecord = 20;
+struct RoundSplit {
+	float* pose;
+	uint32_t* done;
+	float* totals;
+	uint32_t rounds;          /* of the ligand */
+};
+
 struct RigidLaunch {
 	RigidModel m;
 	const gba_dof6d* dofs;
@@ -125,13 +136,16 @@ struct RigidLaunch {
 	const uint32_t* order;    /* visiting order (nullptr: submission order) */
 	size_t n;
 	int bound4;               /* launch the four-blocks-per-SM instantiation */
-	int roundwise;            /* the minimizers' round-wise summation order (plain form) */
 	int ref_order;            /* the reference CPU path's summation order (GBA_KOPT_REFERENCE_ORDER;
-	                             takes precedence over roundwise and bound4, not over census) */
-	unsigned long long* next; /* pose counter, zero at launch (PoseFeed); nullptr: fixed stride */
+	                             takes precedence over bound4, not over census) */
+	unsigned long long* next; /* pose counter, zero at launch (next_pose) */
+	RoundSplit split;         /* launch_rigid_rounds only */
 };
 
 cudaError_t launch_rigid_energy(const RigidLaunch& L, int blocks, int threads, cudaStream_t s);
+/* the default order with a warp per 64-bead round: L.split and L.next set,
+ * neither cleared */
+cudaError_t launch_rigid_rounds(const RigidLaunch& L, int blocks, int threads, cudaStream_t s);
 
 /* ---- persistent minimizer (minimize.cu) ---------------------------------- */
 
@@ -179,7 +193,7 @@ struct BatchEnergyLaunch {
 	const gba_dof6d* dofs;
 	gba_result6d* out;
 	size_t n;
-	unsigned long long* next; /* pose counter, zero at launch (PoseFeed); nullptr: fixed stride */
+	unsigned long long* next; /* pose counter, zero at launch (next_pose) */
 	int ref_order;            /* GBA_KOPT_REFERENCE_ORDER */
 };
 
@@ -200,8 +214,8 @@ struct ModesLaunch {
 	const gba_dof6d_modes* dofs;
 	gba_result6d_modes* out;
 	size_t n;
-	unsigned long long* next; /* pose counters, zero at launch (PoseFeed): receptor pass, */
-	unsigned long long* next2;/* ligand pass; nullptr: fixed stride */
+	unsigned long long* next; /* pose counters, zero at launch (next_pose): receptor pass, */
+	unsigned long long* next2;/* ligand pass */
 	int ref_order;            /* GBA_KOPT_REFERENCE_ORDER: the reference CPU path's order */
 	float4* ref_rf;           /* with ref_order: rec.n float4 per launched warp (modes_ref_warps) */
 };
@@ -229,8 +243,7 @@ cudaError_t launch_minimize_modes(const ModesMinLaunch& M, int blocks, int threa
 int minimize_modes_blocks_per_sm(int threads, const ModesLaunch& L);
 
 /* Number of resident blocks per SM of the rigid kernel for `threads`. */
-int rigid_blocks_per_sm(int threads, bool census, bool bound4 = false, bool roundwise = false,
-		bool ref_order = false);
+int rigid_blocks_per_sm(int threads, bool census, bool bound4 = false, bool ref_order = false, bool rounds = false);
 
 }  // namespace gba
 

@@ -15,8 +15,8 @@
  * per pose the last evaluated DOF and Result and the evaluation count are
  * written -- what RequestHandler::getResultStates / getResultEnGrads report.
  *
- * Both kernels sum each pose round-wise (rigid_pose.cuh), as the plain
- * per-step form's scoring launches do, so all three give the same bits.
+ * Both kernels sum each pose as the scoring launches do (rigid_pose.cuh), so
+ * the device and plain per-step forms give the same bits.
  * With GBA_KOPT_REFERENCE_ORDER both sum in the reference CPU path's order
  * instead (eval_pose_rigid_ref, eval_pose_rigid_team_ref: the same bits).
  *
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256, REF ? 2 : 4) minimize_rigid_kernel(const 
 					eval_pose_rigid_ref(M, cur[0], cur[1], cur[2], cur[3], cur[4], cur[5], lane, stage[threadIdx.x >> 5],
 							res);
 				else
-					eval_pose_rigid<false, true>(M, cur[0], cur[1], cur[2], cur[3], cur[4], cur[5], lane,
+					eval_pose_rigid<false>(M, cur[0], cur[1], cur[2], cur[3], cur[4], cur[5], lane,
 							stage[threadIdx.x >> 5], res, nullptr);
 				++nev;
 				/* objective E, gradient -(ang, pos), src/apps/em/meta.h:114-121;

@@ -591,7 +591,6 @@ int gba_minimize_6d_plain(gba_ctx* ctx, gba_id rec, gba_id lig, gba_id grid, gba
 			L.out = dout + b;
 			L.n = m;
 			L.census = nullptr;
-			L.roundwise = 1;      /* the device minimizer's summation order */
 			ctx->run_rigid(L, s, &shape);
 			check_cuda(cudaMemcpyAsync(hout + b, dout + b, m * sizeof(gba_result6d), cudaMemcpyDeviceToHost, s),
 					"plain: D2H");

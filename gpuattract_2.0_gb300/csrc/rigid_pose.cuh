@@ -24,19 +24,12 @@
  * Every lookup and pair contributes straight to the pose sums: energy,
  * force and the torque matrix sum_i x_i (x) f_i are linear in the bead
  * forces, so no per-bead force is kept (reducePotForce / reduceTorque,
- * src/model/reduction.h:40-103).  Two summation orders exist:
- *   per pose   (scoring kernels) each lane accumulates over all rounds and
- *              the warp reduces once per pose;
- *   round-wise (minimizer kernels and the plain per-step form's launches)
- *              each 64-bead round is reduced on its own by a fixed 16-value
- *              reduce-scatter (round_reduce) and the round totals are added
- *              in round order, so a pose's result does not depend on which
- *              warp evaluates which round: a team of warps splitting one
- *              pose (eval_pose_rigid_team) gives the same bits as one warp.
- * Both are deterministic; they differ from each other in the last bits.  The
- * per-pose order stays in the scoring kernels because the round-wise
- * reduction costs them registers at their 64-register bound (it spills and
- * measured 13 % slower on config 1).
+ * src/model/reduction.h:40-103).  Each 64-bead round is reduced over the warp
+ * on its own in a fixed butterfly (round_total) and the round totals are
+ * added in round order.  A pose's result therefore does not depend on which
+ * warp evaluates which round: one warp walking a whole pose, warps taking
+ * single rounds (rigid_rounds_kernel) and a team splitting a pose in the
+ * minimizer (eval_pose_rigid_team) all give the same bits.
  */
 #ifndef GBA_RIGID_POSE_CUH_
 #define GBA_RIGID_POSE_CUH_
@@ -64,9 +57,11 @@ struct WarpStage {
 	/* the pose: rotation matrix [0, 9), sin/cos of phi, ssi, rot [9, 15),
 	 * translation [15, 18); kept here rather than in registers */
 	float pose[18];
-	/* round-wise order: running total of the rounds, component c in tot[c]
-	 * (written by lane 2c) */
+	/* the sum of the round totals so far, component c in tot[c] (written by
+	 * lane 2c); in a register it cost the scoring kernel 7 %: that register
+	 * comes from the loads in flight */
 	float tot[16];
+	unsigned long long slot;           /* the pose's index, for the same reason */
 };
 
 /* Stores the pose rotation and translation in the warp's staging area. */
@@ -285,6 +280,18 @@ struct PoseSums {
 		T[6] = ffma(ux, fz, T[6]); T[7] = ffma(uy, fz, T[7]); T[8] = ffma(uz, fz, T[8]);
 	}
 };
+
+/* Zero sums that the compiler has to keep in registers from here on.  Left
+ * to itself it materialises the zeros after the round's staging, fills the
+ * freed registers with the staging's loads and spills (120 bytes in the
+ * scoring kernel's 64 registers). */
+__device__ __forceinline__ PoseSums held_sums() {
+	PoseSums S;
+	asm volatile("" : "+f"(S.E), "+f"(S.Fx), "+f"(S.Fy), "+f"(S.Fz));
+#pragma unroll
+	for (int k = 0; k < 9; ++k) asm volatile("" : "+f"(S.T[k]));
+	return S;
+}
 
 /* Cooperative accumulators of one lane: the lane always ends a butterfly
  * holding the same component (x, y, z of the force or E) of one of the two
@@ -608,30 +615,38 @@ __device__ __forceinline__ void eval_round(const RigidModel& M, uint32_t i0, int
 	__syncwarp();
 }
 
-/* Reduce-scatter of a round's lane sums over the warp in a fixed butterfly:
- * lane l returns component l >> 1 of (E, Fx, Fy, Fz, T[0..8], 0, 0, 0)
- * summed over all 32 lanes (lanes 2c and 2c + 1 hold the same value). */
-__device__ __forceinline__ float round_reduce(const PoseSums& S, int lane) {
-	const float v[16] = {S.E, S.Fx, S.Fy, S.Fz, S.T[0], S.T[1], S.T[2], S.T[3], S.T[4], S.T[5], S.T[6],
-			S.T[7], S.T[8], 0.f, 0.f, 0.f};
-	const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
-	float m8[8];
+/* A round's lane sums added over the warp in a fixed butterfly (lane
+ * distances 16, 8, 4, 2, 1): lanes 2c and 2c + 1 return component c of
+ * (E, Fx, Fy, Fz, T[0..8]); lanes 26..31 nothing of use.  The 13 components go
+ * through the round's corner weights, which nothing reads any more: even
+ * lanes' values of a component and odd lanes' lie in 16 floats each, which
+ * one lane loads in four words and adds up, so the reduction costs 34
+ * instructions a round against 95 for 31 shuffles with their selects (which
+ * also spilled in the scoring kernel's 64 registers: config 1 ran 13 %
+ * slower).  Rows of 36 floats: neither stores nor loads meet a bank twice. */
+constexpr int kTotalRow = 36;
+static_assert(13 * kTotalRow <= kBeadsPerRound * kCornerStride, "round_total overlays the corner weights");
+static_assert(offsetof(WarpStage, cw) % 16 == 0, "round_total loads float4");
+__device__ __forceinline__ float round_total(const PoseSums& S, WarpStage& W, int lane) {
+	float* to = W.cw + (lane & 1) * 16 + (lane >> 1);
+	to[0] = S.E;
+	to[kTotalRow] = S.Fx; to[2 * kTotalRow] = S.Fy; to[3 * kTotalRow] = S.Fz;
 #pragma unroll
-	for (int j = 0; j < 8; ++j)
-		m8[j] = fadd(b4 ? v[8 + j] : v[j], __shfl_xor_sync(GBA_FULL_MASK, b4 ? v[j] : v[8 + j], 16));
-	float m4[4];
-#pragma unroll
-	for (int j = 0; j < 4; ++j)
-		m4[j] = fadd(b3 ? m8[4 + j] : m8[j], __shfl_xor_sync(GBA_FULL_MASK, b3 ? m8[j] : m8[4 + j], 8));
-	float m2[2];
-#pragma unroll
-	for (int j = 0; j < 2; ++j)
-		m2[j] = fadd(b2 ? m4[2 + j] : m4[j], __shfl_xor_sync(GBA_FULL_MASK, b2 ? m4[j] : m4[2 + j], 4));
-	const float m1 = fadd(b1 ? m2[1] : m2[0], __shfl_xor_sync(GBA_FULL_MASK, b1 ? m2[0] : m2[1], 2));
-	return fadd(m1, __shfl_xor_sync(GBA_FULL_MASK, m1, 1));
+	for (int k = 0; k < 9; ++k) to[(4 + k) * kTotalRow] = S.T[k];
+	__syncwarp();
+	const int c = min(lane >> 1, 12);
+	const float4* from = reinterpret_cast<const float4*>(W.cw + c * kTotalRow + (lane & 1) * 16);
+	const float4 a = from[0], b = from[1], x = from[2], y = from[3];
+	/* lanes l and l + 16 lie 8 floats apart, l and l + 8 four, ... */
+	const float4 m = make_float4(fadd(fadd(a.x, x.x), fadd(b.x, y.x)), fadd(fadd(a.y, x.y), fadd(b.y, y.y)),
+			fadd(fadd(a.z, x.z), fadd(b.z, y.z)), fadd(fadd(a.w, x.w), fadd(b.w, y.w)));
+	const float h = fadd(fadd(m.x, m.z), fadd(m.y, m.w));
+	const float t = fadd(h, __shfl_xor_sync(GBA_FULL_MASK, h, 1));
+	__syncwarp();   /* read before the next round's weights */
+	return t;
 }
 
-/* Clears the warp's round totals. */
+/* Clears the warp's running totals. */
 __device__ __forceinline__ void clear_totals(WarpStage& W, int lane) {
 	if (lane < 16) W.tot[lane] = 0.f;
 	__syncwarp();
@@ -660,35 +675,19 @@ __device__ __forceinline__ void finish_pose(const WarpStage& W, float res[7]) {
 }
 
 /* res: E, force xyz, Euler gradient xyz (Result_6D order); identical on all
- * lanes.  W is this warp's shared staging area.  ROUNDWISE selects the
- * round-wise summation order (see the file comment). */
-template <bool CENSUS, bool ROUNDWISE = false>
+ * lanes.  W is this warp's shared staging area. */
+template <bool CENSUS>
 __device__ __forceinline__ void eval_pose_rigid(const RigidModel& M, float tx, float ty, float tz,
 		float a0, float a1, float a2, int lane, WarpStage& W, float res[7], PoseCensus* census) {
 	put_pose(W, pose_rotation(a0, a1, a2, lane, M.trig), tx, ty, tz, lane);
 	RoundCensus cen;
-	if (ROUNDWISE) {
-		clear_totals(W, lane);
-		for (uint32_t i0 = 0; i0 < M.lig.n; i0 += kBeadsPerRound) {
-			PoseSums S;
-			eval_round<CENSUS>(M, i0, lane, W, cen, S);
-			add_round(W, round_reduce(S, lane), lane);
-		}
-		finish_pose(W, res);
-	} else {
-		PoseSums S;
-		for (uint32_t i0 = 0; i0 < M.lig.n; i0 += kBeadsPerRound) eval_round<CENSUS>(M, i0, lane, W, cen, S);
-		float sE = warp_sum(S.E), sFx = warp_sum(S.Fx), sFy = warp_sum(S.Fy), sFz = warp_sum(S.Fz);
-		float T[9];
-#pragma unroll
-		for (int k = 0; k < 9; ++k) T[k] = warp_sum(S.T[k]);
-		force_lim(sFx, sFy, sFz);
-		float ang[3];
-		float ttx, tty, ttz;
-		torque_reduce(get_pose(W, ttx, tty, ttz), T, ang);
-		res[0] = sE; res[1] = sFx; res[2] = sFy; res[3] = sFz;
-		res[4] = ang[0]; res[5] = ang[1]; res[6] = ang[2];
+	clear_totals(W, lane);
+	for (uint32_t i0 = 0; i0 < M.lig.n; i0 += kBeadsPerRound) {
+		PoseSums S = held_sums();
+		eval_round<CENSUS>(M, i0, lane, W, cen, S);
+		add_round(W, round_total(S, W, lane), lane);
 	}
+	finish_pose(W, res);
 	if (CENSUS) {
 #pragma unroll
 		for (int o = 16; o > 0; o >>= 1) {
@@ -1070,7 +1069,7 @@ __device__ __forceinline__ void group_sync(int id, int nthreads) {
  * with named barrier bar_id: warp t takes rounds t, t + G, t + 2G, ...;
  * after each group of G rounds the warps park their round components in
  * slots[16 t + c] and warp 0 adds them in round order -- the arithmetic of
- * eval_pose_rigid<_, true>, so the result is the same bit for bit.  Warp 0
+ * eval_pose_rigid, so the result is the same bit for bit.  Warp 0
  * computes the rotation (double sincos: GB300's FP64 pipe is narrow) and the
  * others copy it.  Every warp of the team must call it; res is valid in
  * warp 0.  stages: the G warps' staging areas. */
@@ -1085,15 +1084,15 @@ __device__ __forceinline__ void eval_pose_rigid_team(const RigidModel& M, float 
 		if (lane < 18) W.pose[lane] = stages[0].pose[lane];
 		__syncwarp();
 	}
-	clear_totals(W, lane);
 	const uint32_t rounds = (M.lig.n + kBeadsPerRound - 1) / kBeadsPerRound;
 	RoundCensus cen;
+	clear_totals(W, lane);
 	for (uint32_t r0 = 0; r0 < rounds; r0 += G) {
 		const uint32_t r = r0 + t;
 		if (r < rounds) {
-			PoseSums S;
+			PoseSums S = held_sums();
 			eval_round<false>(M, r * kBeadsPerRound, lane, W, cen, S);
-			const float v = round_reduce(S, lane);
+			const float v = round_total(S, W, lane);
 			if ((lane & 1) == 0) slots[16 * t + (lane >> 1)] = v;
 		}
 		group_sync(bar_id, nthreads);
