@@ -465,7 +465,16 @@ int gba_upload_params(gba_ctx* ctx, uint32_t num_types, const gba_ffparam* table
  * lj_pot_force (unfused FP32, one fused multiply-add), so folding them in
  * changes no bit of the result.  Stored transposed against the host table
  * (which is indexed receptor type major): the pairs of one ligand bead then
- * read one contiguous row. */
+ * read one contiguous row.
+ *
+ * A pair term gathers one 16-byte entry, {rc, ac, fb, e}: the scoring kernel
+ * is bound by L1 wavefronts, most of them from the gathers of a pair, and a
+ * second entry per pair ({ipon, rmin2, emin}) was a third of those.  With
+ * ipon 1, LJPotForce's result does not depend on the other three (the same
+ * operations, times one or plus zero); pairs with another ipon -- and those
+ * whose rc has its sign bit set or whose emin is not finite -- are marked by
+ * the sign of the entry's rc and read {rmin2, emin, ipon, rc} from the second
+ * half of the table. */
 const float4* ParamsItem::pair_table(float dPlateau2, bool may_allocate) {
 	uint32_t key;
 	std::memcpy(&key, &dPlateau2, 4);
@@ -495,8 +504,9 @@ const float4* ParamsItem::pair_table(float dPlateau2, bool may_allocate) {
 		}
 		const size_t nt = (size_t)dev.num_types;
 		const size_t kt = (k % nt) * nt + k / nt;
-		t[2 * kt] = make_float4(p.rc, p.ac, p.rmin2, p.emin);
-		t[2 * kt + 1] = make_float4(ivor, fb, e, 0.0f);
+		const bool rest = p.ipon != 1 || std::signbit(p.rc) || !std::isfinite(p.emin);
+		t[kt] = make_float4(rest ? -1.0f : p.rc, p.ac, fb, e);
+		t[T2 + kt] = make_float4(p.rmin2, p.emin, ivor, p.rc);
 	}
 	auto buf = std::make_unique<DevBuffer>();
 	buf->upload(t.data(), t.size() * sizeof(float4));

@@ -85,11 +85,12 @@ struct DevParams {
 	float ffelec;
 	const float4* lj;         /* T*T {rc, ac, rmin2, emin} */
 	const float* ivor;        /* T*T ipon as float */
-	/* T*T pairs of float4 {rc, ac, rmin2, emin}, {ipon, fb_p, e_p, 0}: fb_p and
-	 * e_p are LJPotForce's force factor and energy at the plateau distance of
-	 * the grid in use, per type pair (set per launch); entry
-	 * (ligand type - 1) * T + (receptor type - 1), so the entries one ligand
-	 * bead meets lie in one row */
+	/* T*T float4 {rc, ac, fb_p, e_p}, then T*T float4 {rmin2, emin, ipon, rc}
+	 * for the pairs whose first entry has a negative rc (see
+	 * ParamsItem::pair_table): fb_p and e_p are LJPotForce's force factor and
+	 * energy at the plateau distance of the grid in use, per type pair (set
+	 * per launch); entry (ligand type - 1) * T + (receptor type - 1), so the
+	 * entries one ligand bead meets lie in one row */
 	const float4* pair;
 };
 

@@ -464,18 +464,24 @@ __device__ __forceinline__ bool nl_pair(const DevNL& nl, const DevParams& P, uin
 	const float dr2_inv = nl.approx_inv ? frcp_approx(dr2) : __frcp_rn(dr2);
 	const bool shape86 = P.potshape == GBA_POTSHAPE_8_6;
 	const size_t k = (size_t)P.num_types * (lig_type - 1) + (trec - 1);
-	const float4 p = __ldg(&P.pair[2 * k]);
-	const float4 pl = __ldg(&P.pair[2 * k + 1]);   /* ipon, plateau force factor, plateau energy */
+	const float4 p = __ldg(&P.pair[k]);   /* rc, ac, plateau force factor, plateau energy */
+	/* the sign of rc marks the pairs that need more (ParamsItem::pair_table) */
+	const bool rest = __float_as_uint(p.x) >> 31;
+	float4 q = make_float4(0.f, 0.f, 1.f, p.x);
+	if (rest) q = __ldg(&P.pair[(size_t)P.num_types * P.num_types + k]);   /* rmin2, emin, ipon, rc */
 	/* LJPotForce: energy and the radial factor fb (force = fb * d / r^2) */
 	const float rr23 = fmul(fmul(dr2_inv, dr2_inv), dr2_inv);
-	const float rep = fmul(p.x, shape86 ? dr2_inv : rr23);
+	const float rep = fmul(q.w, shape86 ? dr2_inv : rr23);
 	const float vlj = fmul(fsub(rep, p.y), rr23);
 	float fb = ffma(6.0f, vlj, fmul(shape86 ? 2.0f : 6.0f, fmul(rep, rr23)));
-	if (dr2 < p.z) {
-		e = ffma(fsub(pl.x, 1.0f), p.w, vlj);
-	} else {
-		e = fmul(pl.x, vlj);
-		fb = fmul(pl.x, fb);
+	e = vlj;
+	if (rest) {
+		if (dr2 < q.x) {
+			e = ffma(fsub(q.z, 1.0f), q.y, vlj);
+		} else {
+			e = fmul(q.z, vlj);
+			fb = fmul(q.z, fb);
+		}
 	}
 	/* getRatio's table bin, src/model/NLGrid.h:141-143 */
 	const int bin = (int)fmul(dr2, 10000.0f);
@@ -483,8 +489,8 @@ __device__ __forceinline__ bool nl_pair(const DevNL& nl, const DevParams& P, uin
 			? fsqrt_approx(fmul(fadd((float)bin, 0.5f), nl.ratio_scale))
 			: __ldg(&nl.ratio[bin]);
 	/* minus LJPotForce at the plateau (per type pair, precomputed) */
-	float s = ffma(-pl.y, ratio, fb);
-	e = fsub(e, pl.z);
+	float s = ffma(-p.z, ratio, fb);
+	e = fsub(e, p.w);
 	const float qq = fmul(fmul(qlig, rq), P.ffelec);
 	if (fabsf(qq) > 0.001f) {
 		/* ChargePotForce at r minus at the plateau: energy qq * dd when
