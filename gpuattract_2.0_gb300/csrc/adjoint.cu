@@ -21,8 +21,9 @@
  *             reference's gradient convention (src/apps/em/meta.h:114-121)
  *   dE/dq     per ligand and per receptor bead
  *   dE/dr0, dE/deps per type pair [rec type - 1][lig type - 1]
- * Parameter gradients accumulate in FP64 shared-memory partials per block and
- * are flushed with FP64 global atomics.
+ * Parameter gradients accumulate in the block's shared memory as unevaluated
+ * sums of two floats (TwoFloat), are written out per block in double and added
+ * up by a last kernel.
  */
 #include <cub/cub.cuh>
 
@@ -52,42 +53,198 @@ struct PairwiseLaunch {
 	double* g_qrec;        /* rec.n */
 	double* g_r0;          /* T*T */
 	double* g_eps;         /* T*T */
-	const float4* tab;     /* 3*T*T: per type pair the constants of lj86 (lj_table_kernel) */
-	const float4* rq;      /* rec.n: receptor x, y, z and this call's charge (pack_receptor_kernel) */
+	float4* tab;           /* 2*T*T: per type pair the constants of the 8-6 term (pairwise_setup_kernel) */
+	float4* rq;            /* rec.n: receptor x, y, z and this call's charge */
 	const uint32_t* tlist; /* the neighbour list with receptor types in bits 24..31, or nullptr */
-	unsigned long long* next;   /* pose counter, zero at launch (next_pose) */
-	const uint32_t* order;      /* visiting order (nearest ligands first), or nullptr */
+	unsigned long long* next;   /* pose (or round) counter, zero at launch (next_pose) */
+	uint32_t* order;            /* visiting order (nearest ligands first), or nullptr */
+	RoundSplit split;           /* pose records; totals and done only when split */
+	int by_round;               /* units are 64-bead rounds, else poses */
+	double* part;               /* backward: per block, then once for what no TwoFloat holds, the sums of
+	                               every cell (PairCells) */
+};
+
+/* The cells of the parameter gradients: per type pair the sums of
+ * w d(energy)/d(rc) and w d(energy)/d(ac), side by side, then the ligand and receptor charges'.
+ * Type pairs are stored ligand type major: neighbouring lanes hold pairs of
+ * one ligand bead, whose cells then lie in one row, in banks of their own.
+ * Receptor type major, as the caller's arrays are, put the 32 types of a row
+ * into one bank, and the adds to these cells took 730 us of a 1,190 us
+ * backward pass (10,000 poses, 2000/700 beads). */
+struct PairCells {
+	uint32_t T2, lig, rec;
+	__host__ __device__ uint32_t qlig() const { return 2 * T2; }
+	__host__ __device__ uint32_t qrec() const { return 2 * T2 + lig; }
+	__host__ __device__ uint32_t count() const { return 2 * T2 + lig + rec; }
 };
 
 namespace {
 
-/* Per type pair (r0, eps, ipon), the constants of the 8-6 term and of its
- * derivatives, computed once per call: {rc, ac, emin, rmin2},
- * {-3 emin / rc, 4 emin / ac, 8 r0^7, 6 r0^5}, {r0^8, r0^6, eps, ipon}, with
- * rc = eps r0^8, ac = eps r0^6, emin = -27 ac^4 / (256 rc^3),
- * rmin2 = 4 rc / (3 ac) as readParamTableFromFile derives them
- * (src/fileIO/readFile.cpp:484-497).  The pair loop then divides nothing but
- * 1/r^2. */
-__global__ void lj_table_kernel(uint32_t T2, const float* __restrict__ r0v, const float* __restrict__ epsv,
-		const int32_t* __restrict__ ipon, float4* __restrict__ tab) {
-	const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-	if (k >= T2) return;
-	const float r0 = r0v[k], eps = epsv[k];
-	const float r0_2 = r0 * r0, r0_6 = r0_2 * r0_2 * r0_2, r0_8 = r0_6 * r0_2;
-	const float rc = eps * r0_8, ac = eps * r0_6;
-	const bool ok = ac > 0.f && rc > 0.f;
-	const float emin = ok ? -27.f * (ac * ac) * (ac * ac) / (256.f * rc * rc * rc) : 0.f;
-	const float rmin2 = ok ? 4.f * rc / (3.f * ac) : 0.f;
-	tab[3 * k] = make_float4(rc, ac, emin, rmin2);
-	tab[3 * k + 1] = make_float4(ok ? -3.f * emin / rc : 0.f, ok ? 4.f * emin / ac : 0.f, 8.f * (r0_6 * r0),
-			6.f * (r0_2 * r0_2 * r0));
-	tab[3 * k + 2] = make_float4(r0_8, r0_6, eps, (float)ipon[k]);
+/* An unevaluated sum hi + lo, |lo| <= ulp(hi)/2: about 48 bits.  The additions
+ * are Knuth's two-sum (no ordering of the operands needed) and a
+ * renormalisation, ten FP32 operations, where a double costs a conversion and
+ * an addition on the FP64 pipe, 16 cycles each for a warp and SM. */
+struct TwoFloat {
+	float hi, lo;
+};
+__device__ __forceinline__ TwoFloat two_add(TwoFloat a, float v) {
+	const float s = __fadd_rn(a.hi, v);
+	const float b = __fsub_rn(s, a.hi);
+	const float err = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, b)), __fsub_rn(v, b));
+	const float l = __fadd_rn(a.lo, err);
+	const float hi = __fadd_rn(s, l);
+	return TwoFloat{hi, __fsub_rn(l, __fsub_rn(hi, s))};
 }
 
-/* Sort keys of the visiting order: the bits of |t|^2 for the pose's
- * translation t (non-negative floats order like their bit patterns; NaN
- * sorts last).  Ligands near the receptor's centre meet the most neighbour
- * pairs, so taking them first leaves cheap poses for the end of the launch. */
+/* Adds v to a shared cell; what would overflow a TwoFloat (or is no number)
+ * goes to the launch's double cell instead.  There is no shared FP64
+ * reduction: atomicAdd loops over a compare-and-swap too.  26 M adds to each
+ * of two random cells of 1,024: 0.28 ms as doubles, 0.14 ms as TwoFloats;
+ * global FP64 reductions 0.34-1.3 ms.  In the kernel lanes meet in cells
+ * (a ligand bead's 32 type pairs), and the loops repeat: cell_add2 halves
+ * them (10,000 poses, 2000/700 beads, forward and backward: 1,193 -> 966 us). */
+__device__ __forceinline__ void cell_add(unsigned long long* cell, float v, double* beyond) {
+	constexpr float kBig = 1e37f;
+	if (v == 0.f) return;
+	if (!(fabsf(v) < kBig)) {
+		atomicAdd(beyond, (double)v);
+		return;
+	}
+	unsigned long long old = *(volatile unsigned long long*)cell, was;
+	do {
+		was = old;
+		const TwoFloat a{__uint_as_float((uint32_t)was), __uint_as_float((uint32_t)(was >> 32))};
+		if (!(fabsf(a.hi) < kBig)) {
+			atomicAdd(beyond, (double)v);
+			return;
+		}
+		const TwoFloat t = two_add(a, v);
+		old = atomicCAS(cell, was, (unsigned long long)__float_as_uint(t.lo) << 32 | __float_as_uint(t.hi));
+	} while (old != was);
+}
+
+/* The same for a type pair's two sums, neighbours in shared memory, in one
+ * 128-bit compare-and-swap. */
+struct __align__(16) TwoFloat2 {
+	TwoFloat a, b;
+};
+__device__ __forceinline__ void cell_add2(TwoFloat2* cell, float va, float vb, double* beyond_a, double* beyond_b) {
+	constexpr float kBig = 1e37f;
+	if (va == 0.f && vb == 0.f) return;
+	if (!(fabsf(va) < kBig && fabsf(vb) < kBig)) {
+		atomicAdd(beyond_a, (double)va);
+		atomicAdd(beyond_b, (double)vb);
+		return;
+	}
+	TwoFloat2 old = *cell, was;
+	bool again;
+	do {
+		was = old;
+		if (!(fabsf(was.a.hi) < kBig && fabsf(was.b.hi) < kBig)) {
+			atomicAdd(beyond_a, (double)va);
+			atomicAdd(beyond_b, (double)vb);
+			return;
+		}
+		old = atomicCAS(cell, was, TwoFloat2{two_add(was.a, va), two_add(was.b, vb)});
+		again = __float_as_uint(old.a.hi) != __float_as_uint(was.a.hi) || __float_as_uint(old.a.lo) != __float_as_uint(was.a.lo) ||
+				__float_as_uint(old.b.hi) != __float_as_uint(was.b.hi) || __float_as_uint(old.b.lo) != __float_as_uint(was.b.lo);
+	} while (again);
+}
+
+/* ---- before the pair kernel ------------------------------------------------- */
+
+/* Poses nearest the receptor's centre first: their ligands meet the most
+ * pairs, so the launch ends with cheap poses.  A counting sort on the top bits
+ * of |t|^2 (non-negative floats order like their bit patterns, NaN last; 3 %
+ * bins), one block. */
+constexpr int kSetupThreads = 512;
+constexpr int kNearBins = 8192, kNearShift = 18;
+constexpr size_t kNearFirstMinPoses = 2048;
+constexpr size_t kNearOneBlock = 65536;    /* beyond: radix sort (near_first_order) */
+
+__device__ __forceinline__ uint32_t near_key(const gba_dof6d* __restrict__ dofs, size_t p) {
+	const float* d = reinterpret_cast<const float*>(dofs + p);
+	const float x = __ldg(d), y = __ldg(d + 1), z = __ldg(d + 2);
+	return __float_as_uint(x * x + y * y + z * z) & 0x7fffffffu;
+}
+
+__device__ void near_first_block(const PairwiseLaunch& L, uint32_t* bin) {
+	__shared__ uint32_t warp_tot[kSetupThreads / 32];
+	constexpr int per = kNearBins / kSetupThreads;
+	const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+	for (int k = t; k < kNearBins; k += kSetupThreads) bin[k] = 0;
+	__syncthreads();
+	for (size_t p = t; p < L.n; p += kSetupThreads) atomicAdd(&bin[near_key(L.dofs, p) >> kNearShift], 1u);
+	__syncthreads();
+	uint32_t v[per], sum = 0;
+#pragma unroll
+	for (int k = 0; k < per; ++k) {
+		v[k] = bin[t * per + k];
+		sum += v[k];
+	}
+	const uint32_t incl = warp_incl_scan(sum, lane);
+	if (lane == 31) warp_tot[w] = incl;
+	__syncthreads();
+	uint32_t run = incl - sum;
+	for (int k = 0; k < w; ++k) run += warp_tot[k];
+#pragma unroll
+	for (int k = 0; k < per; ++k) {
+		bin[t * per + k] = run;
+		run += v[k];
+	}
+	__syncthreads();
+	for (size_t p = t; p < L.n; p += kSetupThreads)
+		L.order[atomicAdd(&bin[near_key(L.dofs, p) >> kNearShift], 1u)] = (uint32_t)p;
+}
+
+/* One launch for everything the pair kernel reads, by block: block 0 the
+ * visiting order and the counter; then the pose records (and the counts of
+ * finished rounds); then per type pair the constants of the 8-6 term,
+ *   {rc, ac, ipon, 0}, {emin, rmin2, -3 emin / rc, 4 emin / ac}
+ * with rc = eps r0^8, ac = eps r0^6, emin = -27 ac^4 / (256 rc^3),
+ * rmin2 = 4 rc / (3 ac) as readParamTableFromFile derives them
+ * (src/fileIO/readFile.cpp:484-497), ligand type major, the receptor's positions with this
+ * call's charges, and zeros for the double cells.  Six launches before (two of
+ * them a 30 us radix sort). */
+__global__ void __launch_bounds__(kSetupThreads) pairwise_setup_kernel(const PairwiseLaunch L, const uint32_t pose_blocks,
+		const int sort, const uint32_t cells) {
+	__shared__ uint32_t bin[kNearBins];
+	if (blockIdx.x == 0) {
+		if (threadIdx.x == 0) *L.next = 0;
+		if (sort) near_first_block(L, bin);
+		return;
+	}
+	if (blockIdx.x <= pose_blocks) {
+		const size_t t = (size_t)(blockIdx.x - 1) * kSetupThreads + threadIdx.x;
+		const size_t p = t >> 2;
+		const bool in = p < L.n;
+		if (L.by_round && in && (t & 3) == 0) L.split.done[p] = 0;
+		write_pose_record(reinterpret_cast<const float*>(L.dofs + (in ? p : 0)), DevTrig{nullptr, 0u, 0u}, in,
+				threadIdx.x & 31, L.split.pose + kPoseRecord * p);
+		return;
+	}
+	const uint32_t stride = (gridDim.x - 1 - pose_blocks) * kSetupThreads;
+	const uint32_t first = (blockIdx.x - 1 - pose_blocks) * kSetupThreads + threadIdx.x;
+	for (uint32_t k = first; k < L.T * L.T; k += stride) {
+		const uint32_t from = L.T * (k % L.T) + k / L.T;      /* the caller's: receptor type major */
+		const float r0 = L.r0[from], eps = L.eps[from];
+		const float r0_2 = r0 * r0, r0_6 = r0_2 * r0_2 * r0_2, r0_8 = r0_6 * r0_2;
+		const float rc = eps * r0_8, ac = eps * r0_6;
+		const bool ok = ac > 0.f && rc > 0.f;
+		const float emin = ok ? -27.f * (ac * ac) * (ac * ac) / (256.f * rc * rc * rc) : 0.f;
+		L.tab[k] = make_float4(rc, ac, (float)L.ipon[from], 0.f);
+		L.tab[L.T * L.T + k] = make_float4(emin, ok ? 4.f * rc / (3.f * ac) : 0.f, ok ? -3.f * emin / rc : 0.f,
+				ok ? 4.f * emin / ac : 0.f);
+	}
+	for (uint32_t j = first; j < L.rec.n; j += stride) {
+		const float4 r = L.rec.xyzq[j];
+		L.rq[j] = make_float4(r.x, r.y, r.z, L.q_rec[j]);
+	}
+	for (uint32_t k = first; k < cells; k += stride) L.part[k] = 0.0;
+}
+
+/* The same for more poses than one block sorts quickly: a radix sort of the
+ * bits of |t|^2. */
 __global__ void near_first_keys_kernel(const gba_dof6d* __restrict__ dofs, uint32_t n, uint32_t* __restrict__ keys,
 		uint32_t* __restrict__ idx) {
 	const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -100,7 +257,7 @@ __global__ void near_first_keys_kernel(const gba_dof6d* __restrict__ dofs, uint3
 
 /* Poses ordered nearest first (sorted on the top 16 bits of the key: the
  * exponent and 7 mantissa bits of |t|^2, about 0.4 % bins), scratch from S. */
-const uint32_t* near_first_order(const gba_dof6d* dofs, size_t n, StreamScratch& S, cudaStream_t s) {
+uint32_t* near_first_order(const gba_dof6d* dofs, size_t n, StreamScratch& S, cudaStream_t s) {
 	cub::DoubleBuffer<uint32_t> kb(nullptr, nullptr), ib(nullptr, nullptr);
 	size_t tmp = 0;
 	check_cuda(cub::DeviceRadixSort::SortPairs(nullptr, tmp, kb, ib, (int)n, 16, 32, s), "pairwise order: size");
@@ -119,49 +276,6 @@ const uint32_t* near_first_order(const gba_dof6d* dofs, size_t n, StreamScratch&
 	return ib.Current();
 }
 
-/* rq[j] = (x, y, z, q_rec[j]): a neighbour's position and charge in one
- * 16-byte gather (the receptor records are read in random order, so every
- * separate load is its own L1 wavefront). */
-__global__ void pack_receptor_kernel(uint32_t n, const float4* __restrict__ xyzq, const float* __restrict__ q,
-		float4* __restrict__ rq) {
-	for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-		const float4 r = xyzq[j];
-		rq[j] = make_float4(r.x, r.y, r.z, q[j]);
-	}
-}
-
-/* LJ energy, radial force factor and d/d(r0, eps) of one 8-6 pair from the
- * type pair's table entry t. */
-template <bool DERIV>
-__device__ __forceinline__ void lj86(float r2, float ir2, const float4* __restrict__ t, float& e, float& fb,
-		float& de_dr0, float& de_deps) {
-	const float4 c = __ldg(t);
-	const float4 k = DERIV ? __ldg(t + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
-	const float4 m = __ldg(t + 2);
-	const float rc = c.x, ac = c.y, emin = c.z, rmin2 = c.w, iv = m.w;
-	const float ir6 = ir2 * ir2 * ir2, ir8 = ir6 * ir2;
-	const float vlj = rc * ir8 - ac * ir6;
-	float de_drc = 0.f, de_dac = 0.f;
-	fb = 6.f * vlj + 2.f * rc * ir8;     /* force factor: f = fb * d / r^2 */
-	if (r2 < rmin2) {
-		e = vlj + (iv - 1.f) * emin;
-		if (DERIV) {
-			de_drc = ir8 + (iv - 1.f) * k.x;
-			de_dac = -ir6 + (iv - 1.f) * k.y;
-		}
-	} else {
-		e = iv * vlj;
-		fb *= iv;
-		if (DERIV) {
-			de_drc = iv * ir8;
-			de_dac = -iv * ir6;
-		}
-	}
-	/* rc = eps r0^8, ac = eps r0^6 */
-	de_dr0 = DERIV ? m.z * (k.z * de_drc + k.w * de_dac) : 0.f;
-	de_deps = DERIV ? m.x * de_drc + m.y * de_dac : 0.f;
-}
-
 /* Per-warp staging of the pairwise kernels: one round of 64 ligand beads. */
 struct PairStage {
 	float4 pq[kBeadsPerRound];       /* transformed x, y, z; charge */
@@ -169,92 +283,118 @@ struct PairStage {
 	uint32_t lbase[kBeadsPerRound];  /* list start - first flattened pair of the slot */
 	float gq[kBeadsPerRound];        /* backward: dE/dq of the slot's bead over this round */
 	uint8_t own[64];                 /* PairWindow: slot of the bead starting at window position b */
+	float pose[kPoseRecord];         /* as WarpStage::pose */
+	float tot[16];                   /* the sum of the round totals so far */
+	unsigned long long slot;         /* the pose's index */
+	unsigned long long pad;
 };
-constexpr int kPairwiseThreads = 256;
-constexpr size_t kNearFirstMinPoses = 2048;
+static_assert(13 * kTotalRow * sizeof(float) <= 2 * kBeadsPerRound * sizeof(float4), "sums_total overlays the bead records");
+static_assert(sizeof(PairStage) % 16 == 0 && offsetof(PairStage, pose) % 16 == 0, "records are read as words");
 
-/* One warp per pose, the ligand in rounds of 64 beads like the rigid kernel:
- * lane-per-bead staging (transform, neighbour-list voxel), then the round's
- * flattened (bead, neighbour) pairs in windows of 64, two per lane, so that
- * uneven list lengths do not idle lanes.  A warp takes its next pose from a
- * global counter when it finishes one (next_pose). */
-template <bool BACKWARD>
-__global__ void __launch_bounds__(kPairwiseThreads) pairwise_kernel(const PairwiseLaunch L) {
-	extern __shared__ double sm[];
-	__shared__ PairStage stage[kPairwiseThreads / 32];
-	const uint32_t T2 = L.T * L.T;
-	double* s_r0 = sm;
-	double* s_eps = sm + T2;
-	double* s_ql = sm + 2 * T2;
-	double* s_qr = sm + 2 * T2 + L.lig.n;
-	if (BACKWARD) {
-		const uint32_t tot = 2 * T2 + L.lig.n + L.rec.n;
-		for (uint32_t k = threadIdx.x; k < tot; k += blockDim.x) sm[k] = 0.0;
-		__syncthreads();
+/* Sum of v over the run of lanes with the same owner, on the run's first
+ * lane; last: the run's last lane.  Every lane of the warp calls it. */
+__device__ __forceinline__ float run_sum(float v, int lane, int last) {
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const float t = __shfl_down_sync(GBA_FULL_MASK, v, o);
+		if (lane + o <= last) v += t;
 	}
-	const int lane = threadIdx.x & 31;
-	PairStage& W = stage[threadIdx.x >> 5];
+	return v;
+}
+
+/* A round of a pose: 64 ligand beads from i0, the flattened (bead, neighbour)
+ * pairs two per lane.  Forward: energies into S.E.  Backward: forces and
+ * torques into S, the parameters' sums into the cells. */
+template <bool BACKWARD>
+__device__ __forceinline__ void pairwise_round(const PairwiseLaunch& L, const PairCells& cells, uint32_t i0, int lane,
+		float w, PairStage& W, unsigned long long* cell, PoseSums& S) {
 	const bool cdiel = L.dielec == GBA_DIELEC_CONSTANT;
-	for (size_t slot = next_pose(L.next, lane); slot < L.n; slot = next_pose(L.next, lane)) {
-		const size_t p = L.order ? (size_t)__ldg(&L.order[slot]) : slot;
-		const float* dofp = reinterpret_cast<const float*>(L.dofs + p);
-		const float dv = lane < 6 ? __ldg(dofp + lane) : 0.f;
-		float c[6];
+	uint32_t nln[2];
+	{
+		float tx, ty, tz;
+		const PoseRot R = get_pose(W, tx, ty, tz);
 #pragma unroll
-		for (int k = 0; k < 6; ++k) c[k] = __shfl_sync(GBA_FULL_MASK, dv, k);
-		const PoseRot R = pose_rotation(c[3], c[4], c[5], lane, DevTrig{nullptr, 0u, 0u});
-		const float w = BACKWARD ? __ldg(&L.gE[p]) : 0.f;
-		float sE = 0.f, sFx = 0.f, sFy = 0.f, sFz = 0.f;
-		float Tq[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-		for (uint32_t i0 = 0; i0 < L.lig.n; i0 += kBeadsPerRound) {
-			uint32_t nln[2];
-#pragma unroll
-			for (int h = 0; h < 2; ++h) {
-				const int s = lane + 32 * h;
-				const uint32_t i = i0 + s;
-				nln[h] = 0;
-				if (i < L.lig.n) {
-					const float4 b = __ldg(&L.lig.xyzq[i]);
-					const uint32_t tl = __ldg(&L.lig.tm[i]) & 0xffffu;
-					if (tl != 0) {
-						float px, py, pz;
-						rot_apply(R.m, b.x, b.y, b.z, px, py, pz);
-						px = fadd(px, c[0]); py = fadd(py, c[1]); pz = fadd(pz, c[2]);
-						W.pq[s] = make_float4(px, py, pz, __ldg(&L.q_lig[i]));
-						W.ut[s] = make_float4(b.x, b.y, b.z, __uint_as_float(tl));
-						if (BACKWARD) W.gq[s] = 0.f;
-						bool in_nl;
-						nln[h] = stage_nl(L.nl, px, py, pz, s, W, in_nl);
-					}
+		for (int h = 0; h < 2; ++h) {
+			const int s = lane + 32 * h;
+			const uint32_t i = i0 + s;
+			nln[h] = 0;
+			if (i < L.lig.n) {
+				const float4 b = __ldg(&L.lig.xyzq[i]);
+				const uint32_t tl = __ldg(&L.lig.tm[i]) & 0xffffu;
+				if (tl != 0) {
+					float px, py, pz;
+					rot_apply(R.m, b.x, b.y, b.z, px, py, pz);
+					px = fadd(px, tx); py = fadd(py, ty); pz = fadd(pz, tz);
+					W.pq[s] = make_float4(px, py, pz, __ldg(&L.q_lig[i]));
+					W.ut[s] = make_float4(b.x, b.y, b.z, __uint_as_float(tl));
+					if (BACKWARD) W.gq[s] = 0.f;
+					bool in_nl;
+					nln[h] = stage_nl(L.nl, px, py, pz, s, W, in_nl);
 				}
 			}
-			uint32_t start[2];
-			const uint32_t n_pair = queue_pairs(W, nln, lane, start);
-			__syncwarp();
-			PairWindow win;
-			for (uint32_t w0 = 0; w0 < n_pair; w0 += 64) {
-				uint32_t so[2];
-				win.owners(W, w0, start, nln, lane, so[0], so[1]);
+		}
+	}
+	uint32_t start[2];
+	const uint32_t n_pair = queue_pairs(W, nln, lane, start);
+	__syncwarp();
+	/* the next window's list entries are on their way while this one is computed */
+	const uint32_t* lst = L.tlist ? L.tlist : L.nl.list;
+	PairWindow win;
+	uint32_t so[2] = {0, 0}, en[2] = {0, 0};
+	if (n_pair > 0) {
+		win.owners(W, 0, start, nln, lane, so[0], so[1]);
 #pragma unroll
-				for (int h = 0; h < 2; ++h) {
-					const uint32_t q = w0 + 32 * h + lane;
-					if (q >= n_pair) continue;
-					const uint32_t s = so[h];
-					const uint32_t ent = __ldg(&(L.tlist ? L.tlist : L.nl.list)[W.lbase[s] + q]);
-					const uint32_t j = L.tlist ? ent & 0xffffffu : ent;
-					const uint32_t tr = L.tlist ? ent >> 24 : __ldg(&L.rec.tm[j]) & 0xffffu;
-					if (tr == 0) continue;
-					const float4 r = __ldg(&L.rq[j]);
-					const float4 b = W.pq[s];
-					const float dx = b.x - r.x, dy = b.y - r.y, dz = b.z - r.z;
-					const float r2 = dx * dx + dy * dy + dz * dz;
-					if (!(r2 < L.cut2)) continue;
-					const float4 u = W.ut[s];
-					const uint32_t tl = __float_as_uint(u.w);
-					const float ir2 = __frcp_rn(r2);      /* = 1.0f / r2, correctly rounded */
-					const uint32_t tp = L.T * (tr - 1) + (tl - 1);
-					float el, fb, dr0, deps;
-					lj86<BACKWARD>(r2, ir2, L.tab + 3 * (size_t)tp, el, fb, dr0, deps);
+		for (int h = 0; h < 2; ++h)
+			if ((uint32_t)lane + 32 * h < n_pair) en[h] = __ldg(&lst[W.lbase[so[h]] + lane + 32 * h]);
+	}
+	for (uint32_t w0 = 0; w0 < n_pair; w0 += 64) {
+		const uint32_t sc[2] = {so[0], so[1]}, ec[2] = {en[0], en[1]};
+		if (w0 + 64 < n_pair) {
+			win.owners(W, w0 + 64, start, nln, lane, so[0], so[1]);
+#pragma unroll
+			for (int h = 0; h < 2; ++h)
+				if (w0 + 64 + 32 * h + lane < n_pair) en[h] = __ldg(&lst[W.lbase[so[h]] + w0 + 64 + 32 * h + lane]);
+		}
+#pragma unroll
+		for (int h = 0; h < 2; ++h) {
+			const uint32_t q0 = w0 + 32 * h;
+			if (q0 >= n_pair) break;
+			const uint32_t s = sc[h];
+			float gqv = 0.f;      /* this pair's part of dE/dq of the ligand bead */
+			bool in = q0 + lane < n_pair;
+			uint32_t j = 0, tr = 0;
+			if (in) {
+				j = L.tlist ? ec[h] & 0xffffffu : ec[h];
+				tr = L.tlist ? ec[h] >> 24 : __ldg(&L.rec.tm[j]) & 0xffffu;
+				in = tr != 0;
+			}
+			if (in) {
+				const float4 r = __ldg(&L.rq[j]);
+				const float4 b = W.pq[s];
+				const float4 u = W.ut[s];
+				const float dx = b.x - r.x, dy = b.y - r.y, dz = b.z - r.z;
+				const float r2 = dx * dx + dy * dy + dz * dz;
+				if (r2 < L.cut2) {
+					const uint32_t tp = L.T * (__float_as_uint(u.w) - 1) + (tr - 1);
+					const float4 c = __ldg(&L.tab[tp]);           /* rc, ac, ipon */
+					const float ir2 = __frcp_rn(r2);              /* = 1.0f / r2, correctly rounded */
+					const float ir6 = ir2 * ir2 * ir2, ir8 = ir6 * ir2;
+					const float vlj = c.x * ir8 - c.y * ir6;
+					float e = vlj, fb = 6.f * vlj + 2.f * c.x * ir8;      /* force factor: f = fb d / r^2 */
+					float drc = ir8, dac = -ir6;
+					if (c.z != 1.f) {
+						const float4 m = __ldg(&L.tab[L.T * L.T + tp]);   /* emin, rmin2, -3 emin / rc, 4 emin / ac */
+						if (r2 < m.y) {
+							e = vlj + (c.z - 1.f) * m.x;
+							drc = ir8 + (c.z - 1.f) * m.z;
+							dac = -ir6 + (c.z - 1.f) * m.w;
+						} else {
+							e = c.z * vlj;
+							fb *= c.z;
+							drc *= c.z;
+							dac *= c.z;
+						}
+					}
 					/* Coulomb, no |q q| switch: smooth in the charges */
 					const float qi = b.w, qj = r.w;
 					float dd, fcf;
@@ -268,59 +408,220 @@ __global__ void __launch_bounds__(kPairwiseThreads) pairwise_kernel(const Pairwi
 					}
 					dd = fmaxf(dd, 0.f);
 					const float qq = L.ffelec * qi * qj;
-					sE += el + qq * dd;
-					if (BACKWARD) {
+					if (!BACKWARD) {
+						S.E += e + qq * dd;
+					} else {
 						const float ff = (fb + qq * fcf) * ir2;
 						const float fx = ff * dx, fy = ff * dy, fz = ff * dz;
-						sFx += fx; sFy += fy; sFz += fz;
-						Tq[0] += u.x * fx; Tq[1] += u.y * fx; Tq[2] += u.z * fx;
-						Tq[3] += u.x * fy; Tq[4] += u.y * fy; Tq[5] += u.z * fy;
-						Tq[6] += u.x * fz; Tq[7] += u.y * fz; Tq[8] += u.z * fz;
-						atomicAdd(&W.gq[s], L.ffelec * qj * dd);
-						atomicAdd(&s_qr[j], (double)(w * (L.ffelec * qi * dd)));
-						atomicAdd(&s_r0[tp], (double)(w * dr0));
-						atomicAdd(&s_eps[tp], (double)(w * deps));
+						S.Fx += fx; S.Fy += fy; S.Fz += fz;
+						S.T[0] += u.x * fx; S.T[1] += u.y * fx; S.T[2] += u.z * fx;
+						S.T[3] += u.x * fy; S.T[4] += u.y * fy; S.T[5] += u.z * fy;
+						S.T[6] += u.x * fz; S.T[7] += u.y * fz; S.T[8] += u.z * fz;
+						gqv = L.ffelec * qj * dd;
+						cell_add(cell + cells.qrec() + j, w * (L.ffelec * qi * dd), L.part + cells.qrec() + j);
+						cell_add2(reinterpret_cast<TwoFloat2*>(cell) + tp, w * drc, w * dac, L.part + 2 * tp, L.part + 2 * tp + 1);
 					}
 				}
 			}
 			if (BACKWARD) {
+				/* the pairs of a bead are neighbouring lanes: their sum goes to the
+				 * slot at once (an atomic per pair had up to 32 lanes retrying on
+				 * one address).  Lanes past the end are their own runs. */
+				const uint32_t key = q0 + lane < n_pair ? s : 64u + lane;
+				const uint32_t prev = __shfl_up_sync(GBA_FULL_MASK, key, 1);
+				const uint32_t heads = __ballot_sync(GBA_FULL_MASK, lane == 0 || key != prev);
+				const uint32_t after = lane == 31 ? 0u : heads >> (lane + 1);
+				const int last = after ? lane + __ffs(after) - 1 : 31;
+				const float g = run_sum(gqv, lane, last);
+				if ((heads >> lane & 1u) && key < 64u) W.gq[s] += g;
 				__syncwarp();
-#pragma unroll
-				for (int h = 0; h < 2; ++h) {
-					const int s = lane + 32 * h;
-					if (nln[h] && W.gq[s] != 0.f) atomicAdd(&s_ql[i0 + s], (double)(w * W.gq[s]));
-				}
 			}
-			__syncwarp();
-		}
-		if (!BACKWARD) {
-			sE = warp_sum(sE);
-			if (lane == 0) L.E[p] = sE;
-		} else {
-			sFx = warp_sum(sFx); sFy = warp_sum(sFy); sFz = warp_sum(sFz);
-#pragma unroll
-			for (int k = 0; k < 9; ++k) Tq[k] = warp_sum(Tq[k]);
-			float ang[3];
-			torque_reduce(R, Tq, ang);
-			/* dE/dDOF = -(force, Euler torque), DOF_6D order (pos, ang) */
-			const float g[6] = {-w * sFx, -w * sFy, -w * sFz, -w * ang[0], -w * ang[1], -w * ang[2]};
-			float v = 0.f;
-#pragma unroll
-			for (int k = 0; k < 6; ++k) v = lane == k ? g[k] : v;
-			if (lane < 6) L.g_dofs[6 * p + lane] = v;
 		}
 	}
 	if (BACKWARD) {
-		__syncthreads();
-		for (uint32_t k = threadIdx.x; k < T2; k += blockDim.x) {
-			if (s_r0[k] != 0.0) atomicAdd(&L.g_r0[k], s_r0[k]);
-			if (s_eps[k] != 0.0) atomicAdd(&L.g_eps[k], s_eps[k]);
-		}
-		for (uint32_t k = threadIdx.x; k < L.lig.n; k += blockDim.x)
-			if (s_ql[k] != 0.0) atomicAdd(&L.g_qlig[k], s_ql[k]);
-		for (uint32_t k = threadIdx.x; k < L.rec.n; k += blockDim.x)
-			if (s_qr[k] != 0.0) atomicAdd(&L.g_qrec[k], s_qr[k]);
+		__syncwarp();
+#pragma unroll
+		for (int h = 0; h < 2; ++h)
+			if (nln[h]) {
+				const uint32_t i = i0 + lane + 32 * h;
+				cell_add(cell + cells.qlig() + i, w * W.gq[lane + 32 * h], L.part + cells.qlig() + i);
+			}
 	}
+	__syncwarp();
+}
+
+/* The pose's outputs from the sum of its round totals in W.tot. */
+template <bool BACKWARD>
+__device__ __forceinline__ void pairwise_finish(const PairwiseLaunch& L, size_t p, float w, int lane, PairStage& W) {
+	__syncwarp();
+	const volatile float* t = W.tot;
+	if (!BACKWARD) {
+		if (lane == 0) L.E[p] = t[0];
+		return;
+	}
+	float T[9], ang[3], tx, ty, tz;
+#pragma unroll
+	for (int k = 0; k < 9; ++k) T[k] = t[4 + k];
+	torque_reduce(get_pose(W, tx, ty, tz), T, ang);
+	/* dE/dDOF = -(force, Euler torque), DOF_6D order (pos, ang) */
+	const float g[6] = {-w * t[1], -w * t[2], -w * t[3], -w * ang[0], -w * ang[1], -w * ang[2]};
+	float v = 0.f;
+#pragma unroll
+	for (int k = 0; k < 6; ++k) v = lane == k ? g[k] : v;
+	if (lane < 6) L.g_dofs[6 * p + lane] = v;
+}
+
+/* Backward: large blocks, so that few copies of the cells take shared memory
+ * (256 threads where they leave no room for more); forward: small ones. */
+constexpr int kPairwiseThreads = 512, kForwardThreads = 256;
+
+extern __shared__ __align__(16) unsigned char pairwise_smem[];
+
+/* A warp takes a pose -- or, by_round, one 64-bead round of a pose, the warp
+ * that finishes the last of them adding the totals -- from the counter.  Each
+ * round is reduced on its own and the totals are added in round order, so a
+ * pose's result does not depend on the launch (as in rigid_rounds_kernel). */
+template <bool BACKWARD>
+__global__ void __launch_bounds__(BACKWARD ? kPairwiseThreads : kForwardThreads, BACKWARD ? 2 : 5)
+		pairwise_kernel(const PairwiseLaunch L) {
+	PairStage* stage = reinterpret_cast<PairStage*>(pairwise_smem);
+	unsigned long long* cell = reinterpret_cast<unsigned long long*>(stage + (blockDim.x >> 5));
+	const PairCells cells{L.T * L.T, L.lig.n, L.rec.n};
+	if (BACKWARD) {
+		for (uint32_t k = threadIdx.x; k < cells.count(); k += blockDim.x) cell[k] = 0;
+		__syncthreads();
+	}
+	const int lane = threadIdx.x & 31;
+	PairStage& W = stage[threadIdx.x >> 5];
+	const uint32_t rounds = L.split.rounds;
+	const size_t units = L.by_round ? L.n * rounds : L.n;
+	for (size_t k = next_pose(L.next, lane); k < units; k = next_pose(L.next, lane)) {
+		const size_t at = L.by_round ? k / rounds : k;
+		const size_t p = L.order ? (size_t)L.order[at] : at;
+		if (lane < kPoseRecord / 4)
+			reinterpret_cast<float4*>(W.pose)[lane] = reinterpret_cast<const float4*>(L.split.pose + kPoseRecord * p)[lane];
+		if (lane == 0) W.slot = p;
+		__syncwarp();
+		const float w = BACKWARD ? __ldg(&L.gE[p]) : 0.f;
+		const uint32_t r0 = L.by_round ? (uint32_t)(k - at * rounds) : 0, r1 = L.by_round ? r0 + 1 : rounds;
+		clear_totals(W, lane);
+		for (uint32_t r = r0; r < r1; ++r) {
+			PoseSums S = held_sums();
+			pairwise_round<BACKWARD>(L, cells, r * kBeadsPerRound, lane, w, W, cell, S);
+			const float v = BACKWARD ? sums_total(S, reinterpret_cast<float*>(W.pq), lane) : warp_sum(S.E);
+			add_round(W, v, lane);
+		}
+		const size_t pose = *(volatile unsigned long long*)&W.slot;
+		if (L.by_round) {
+			/* the round's totals out; the pose's last round reads the others' back */
+			float* tot = L.split.totals + pose * rounds * 16 + (lane >> 1);
+			if ((lane & 1) == 0) __stcg(tot + 16 * r0, *(volatile float*)&W.tot[lane >> 1]);
+			__threadfence();
+			__syncwarp();
+			uint32_t before = 0;
+			if (lane == 0) before = atomicAdd(&L.split.done[pose], 1u);
+			before = __shfl_sync(GBA_FULL_MASK, before, 0);
+			if (before + 1 != rounds) continue;
+			__threadfence();
+			clear_totals(W, lane);
+			for (uint32_t q = 0; q < rounds; ++q) add_round(W, __ldcg(tot + 16 * q), lane);
+		}
+		pairwise_finish<BACKWARD>(L, pose, w, lane, W);
+		__syncwarp();
+	}
+	if (BACKWARD) {
+		__syncthreads();
+		double* out = L.part + (size_t)(1 + blockIdx.x) * cells.count();
+		for (uint32_t k = threadIdx.x; k < cells.count(); k += blockDim.x) {
+			const unsigned long long c = cell[k];
+			out[k] = (double)__uint_as_float((uint32_t)c) + (double)__uint_as_float((uint32_t)(c >> 32));
+		}
+	}
+}
+
+/* Adds the blocks' sums up and to the caller's gradients: with rc = eps r0^8
+ * and ac = eps r0^6, d/dr0 = eps (8 r0^7 d/drc + 6 r0^5 d/dac) and
+ * d/deps = r0^8 d/drc + r0^6 d/dac.  32 cells per block, eight warps a share
+ * of the blocks' sums each (one thread per cell waited 34 us for 456 loads in
+ * a row); the atomics are for callers that add several calls' gradients at
+ * once. */
+__device__ __forceinline__ double cell_sum(const PairwiseLaunch& L, const PairCells& cells, uint32_t k, uint32_t blocks,
+		double (*share)[32]) {
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	double v = 0.0;
+	if (k < cells.count())
+#pragma unroll 8
+		for (uint32_t b = w; b <= blocks; b += 8) v += L.part[(size_t)b * cells.count() + k];
+	share[w][lane] = v;
+	__syncthreads();
+	v = 0.0;
+#pragma unroll
+	for (int q = 0; q < 8; ++q) v += share[q][lane];
+	__syncthreads();
+	return v;
+}
+
+__global__ void __launch_bounds__(256) pairwise_gather_kernel(const PairwiseLaunch L, const uint32_t blocks) {
+	__shared__ double share[8][32];
+	const PairCells cells{L.T * L.T, L.lig.n, L.rec.n};
+	const uint32_t type_blocks = (cells.T2 + 31) / 32;
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	if (blockIdx.x < type_blocks) {
+		const uint32_t k = blockIdx.x * 32 + lane;
+		const bool in = k < cells.T2;
+		const double drc = cell_sum(L, cells, in ? 2 * k : cells.count(), blocks, share);
+		const double dac = cell_sum(L, cells, in ? 2 * k + 1 : cells.count(), blocks, share);
+		if (w != 0 || !in || (drc == 0.0 && dac == 0.0)) return;
+		const uint32_t to = L.T * (k % L.T) + k / L.T;
+		const double r0 = L.r0[to], eps = L.eps[to];
+		const double p2 = r0 * r0, p5 = p2 * p2 * r0, p6 = p5 * r0, p7 = p6 * r0;
+		atomicAdd(&L.g_r0[to], eps * (8.0 * p7 * drc + 6.0 * p5 * dac));
+		atomicAdd(&L.g_eps[to], p7 * r0 * drc + p6 * dac);
+		return;
+	}
+	const uint32_t q = (blockIdx.x - type_blocks) * 32 + lane;
+	const bool in = q < cells.lig + cells.rec;
+	const double g = cell_sum(L, cells, in ? cells.qlig() + q : cells.count(), blocks, share);
+	if (w != 0 || !in || g == 0.0) return;
+	if (q < cells.lig)
+		atomicAdd(&L.g_qlig[q], g);
+	else
+		atomicAdd(&L.g_qrec[q - cells.lig], g);
+}
+
+/* The cells of one block at most, and the shared memory a block may use. */
+constexpr size_t kPairwiseCellBytes = 200 * 1024 - 8 * 2624;
+constexpr size_t kPairwiseSmem = 227 * 1024;
+static_assert(kPairwiseCellBytes + 8 * sizeof(PairStage) <= kPairwiseSmem, "a block of 256 threads always fits");
+
+/* Launches of at most this many poses per resident warp take rounds (their
+ * totals within kPairwiseSplitBytes), larger ones whole poses.  The forward
+ * pass orders its poses nearest first, so its tail is short, and rounds cost
+ * it more sooner.  Measured, whole poses against rounds, 2000/700 beads:
+ * forward 1,000 poses (0.2 a warp) 169 -> 79 us, 10,000 (1.6) 220 -> 283;
+ * backward 10,000 (2.1) 745 -> 720, 30,000 (6.2, before cell_add2) 2,901 ->
+ * 2,999. */
+constexpr size_t kForwardPosesPerWarp = 1, kBackwardPosesPerWarp = 4;
+constexpr size_t kPairwiseSplitBytes = (size_t)64 << 20;
+
+/* Resident blocks per SM: the opt-in to the shared memory and the query once
+ * per device, kernel, block size and shared memory. */
+int pairwise_blocks_per_sm(const void* kernel, bool backward, int threads, size_t smem) {
+	static std::mutex mu;
+	static std::map<std::array<size_t, 4>, int> known;
+	int dev = 0;
+	check_cuda(cudaGetDevice(&dev), "pairwise: device");
+	std::lock_guard<std::mutex> g(mu);
+	const std::array<size_t, 4> key{(size_t)dev, (size_t)backward, (size_t)threads, smem};
+	auto it = known.find(key);
+	if (it != known.end()) return it->second;
+	/* the largest any launch may ask for: launches of other sizes may be in flight */
+	check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairwiseSmem),
+			"pairwise: shared memory");
+	int nb = 0;
+	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem), "pairwise: occupancy");
+	if (known.size() >= 256) known.clear();
+	return known[key] = std::max(nb, 1);
 }
 
 }  // namespace
@@ -387,44 +688,61 @@ extern "C" int gba_pairwise_6d(gba_ctx* ctx, gba_id rec, gba_id lig, gba_id grid
 		L.g_r0 = g_r0;
 		L.g_eps = g_eps;
 		cudaStream_t s = (cudaStream_t)stream;
-		/* per-call constants of the 8-6 term per type pair (r0, eps change per call) */
-		const uint32_t T2 = L.T * L.T;
-		StreamScratch scratch(ctx->scratch_pool);
-		float4* tab = (float4*)scratch.get(3 * (size_t)std::max<uint32_t>(T2, 1) * sizeof(float4), s);
-		L.next = (unsigned long long*)scratch.get(sizeof(unsigned long long), s);
-		check_cuda(cudaMemsetAsync(L.next, 0, sizeof(unsigned long long), s), "pairwise: pose counter");
-		/* a few poses per warp: the launch's end is set by its slowest poses */
-		/* the sort takes an int item count: larger batches keep submission order */
-		L.order = (n >= kNearFirstMinPoses && n <= 0x7fffffffu) ? near_first_order(dofs, n, scratch, s) : nullptr;
-		if (T2 > 0) {
-			lj_table_kernel<<<(T2 + 255) / 256, 256, 0, s>>>(T2, L.r0, L.eps, L.ipon, tab);
-			check_cuda(cudaGetLastError(), "pairwise: parameter table");
-		}
-		L.tab = tab;
-		float4* rq = (float4*)scratch.get((size_t)std::max<uint32_t>(L.rec.n, 1) * sizeof(float4), s);
-		if (L.rec.n > 0) {
-			pack_receptor_kernel<<<std::min<uint32_t>((L.rec.n + 255) / 256, 1024), 256, 0, s>>>(L.rec.n, L.rec.xyzq,
-					L.q_rec, rq);
-			check_cuda(cudaGetLastError(), "pairwise: receptor records");
-		}
-		L.rq = rq;
-		const int threads = kPairwiseThreads;
-		const size_t smem = backward ? sizeof(double) * (2 * (size_t)L.T * L.T + L.lig.n + L.rec.n) : 0;
-		if (smem + sizeof(PairStage) * (kPairwiseThreads / 32) > 200 * 1024)
+		const PairCells cells{L.T * L.T, L.lig.n, L.rec.n};
+		const size_t cell_bytes = backward ? (size_t)cells.count() * sizeof(unsigned long long) : 0;
+		if (cell_bytes > kPairwiseCellBytes)
 			throw ApiError(GBA_ERR_INVALID_ARGUMENT, "gba_pairwise_6d: proteins/types too large for the adjoint's shared partials");
-		size_t blocks;
+		const size_t rounds = (L.lig.n + kBeadsPerRound - 1) / kBeadsPerRound;
+		const int threads = !backward ? kForwardThreads
+				: cell_bytes + kPairwiseThreads / 32 * sizeof(PairStage) <= kPairwiseSmem ? kPairwiseThreads : 256;
+		const size_t warps = threads / 32, smem = cell_bytes + warps * sizeof(PairStage);
+		const void* kernel = backward ? (const void*)pairwise_kernel<true> : (const void*)pairwise_kernel<false>;
+		const size_t resident = (size_t)ctx->num_sms * pairwise_blocks_per_sm(kernel, backward, threads, smem);
+		L.by_round = rounds > 1 && n <= (backward ? kBackwardPosesPerWarp : kForwardPosesPerWarp) * resident * warps &&
+				n * rounds * 16 * sizeof(float) <= kPairwiseSplitBytes;
+		const size_t units = L.by_round ? n * rounds : n;
+		const size_t blocks = std::max<size_t>(1, std::min<size_t>((units + warps - 1) / warps, resident));
+		/* one block of scratch, every part 16-byte aligned */
+		StreamScratch scratch(ctx->scratch_pool);
+		const bool sorted = n >= kNearFirstMinPoses && n <= kNearOneBlock;
+		const size_t T2 = cells.T2;
+		size_t at = 0;
+		auto place = [&](size_t bytes) {
+			const size_t o = at;
+			at += (bytes + 15) & ~(size_t)15;
+			return o;
+		};
+		const size_t o_next = place(sizeof(unsigned long long)), o_tab = place(2 * T2 * sizeof(float4)),
+				o_rq = place(L.rec.n * sizeof(float4)), o_pose = place(n * kPoseRecord * sizeof(float)),
+				o_done = place(L.by_round ? n * sizeof(uint32_t) : 0),
+				o_tot = place(L.by_round ? n * rounds * 16 * sizeof(float) : 0),
+				o_order = place(sorted ? n * sizeof(uint32_t) : 0),
+				o_part = place(backward ? (blocks + 1) * cells.count() * sizeof(double) : 0);
+		char* base = (char*)scratch.get(at, s);
+		L.next = (unsigned long long*)(base + o_next);
+		L.tab = (float4*)(base + o_tab);
+		L.rq = (float4*)(base + o_rq);
+		L.split.pose = (float*)(base + o_pose);
+		L.split.done = (uint32_t*)(base + o_done);
+		L.split.totals = (float*)(base + o_tot);
+		L.split.rounds = (uint32_t)rounds;
+		L.part = (double*)(base + o_part);
+		/* the sort takes an int item count: larger batches keep submission order */
+		L.order = sorted ? (uint32_t*)(base + o_order)
+				: n > kNearOneBlock && n <= 0x7fffffffu ? near_first_order(dofs, n, scratch, s) : nullptr;
+		const uint32_t pose_blocks = (uint32_t)((4 * n + kSetupThreads - 1) / kSetupThreads);
+		const uint32_t table_blocks = (uint32_t)std::min<size_t>(
+				(std::max<size_t>(T2, backward ? cells.count() : L.rec.n) + kSetupThreads - 1) / kSetupThreads, 256);
+		pairwise_setup_kernel<<<1 + pose_blocks + std::max(1u, table_blocks), kSetupThreads, 0, s>>>(L, pose_blocks, sorted,
+				backward ? cells.count() : 0);
+		check_cuda(cudaGetLastError(), "pairwise: setup");
 		if (backward) {
-			check_cuda(cudaFuncSetAttribute(pairwise_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-					(int)smem), "adjoint smem");
-			int nb = 0;
-			cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pairwise_kernel<true>, threads, smem);
-			blocks = std::max<size_t>(1, std::min<size_t>((n + 7) / 8, (size_t)ctx->num_sms * std::max(nb, 1)));
 			pairwise_kernel<true><<<(unsigned)blocks, threads, smem, s>>>(L);
+			check_cuda(cudaGetLastError(), "pairwise launch");
+			pairwise_gather_kernel<<<(unsigned)((T2 + 31) / 32 + (L.lig.n + L.rec.n + 31) / 32), 256, 0, s>>>(L,
+					(uint32_t)blocks);
 		} else {
-			int nb = 0;
-			cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pairwise_kernel<false>, threads, 0);
-			blocks = std::max<size_t>(1, std::min<size_t>((n + 7) / 8, (size_t)ctx->num_sms * std::max(nb, 1)));
-			pairwise_kernel<false><<<(unsigned)blocks, threads, 0, s>>>(L);
+			pairwise_kernel<false><<<(unsigned)blocks, threads, smem, s>>>(L);
 		}
 		check_cuda(cudaGetLastError(), "pairwise launch");
 	} catch (const ApiError& e) {

@@ -53,33 +53,11 @@ __global__ void __launch_bounds__(256, BOUND4 ? 4 : 1) rigid_energy_kernel(const
 __global__ void __launch_bounds__(128) rigid_setup_kernel(const RigidLaunch L) {
 	const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
 	const size_t p = t >> 2;
-	const int lane = threadIdx.x & 31, j = lane & 3, base = lane & ~3;
 	const bool in = p < L.n;
-	const float* d = reinterpret_cast<const float*>(L.dofs + (in ? p : 0));
-	float s = 0.f, c = 1.f;
-	if (j < 3) angle_sincos(__ldg(d + 3 + j), L.m.trig, s, c);
-	PoseRot R;
-	R.cphi = __shfl_sync(GBA_FULL_MASK, c, base);
-	R.sphi = __shfl_sync(GBA_FULL_MASK, s, base);
-	R.cssi = __shfl_sync(GBA_FULL_MASK, c, base + 1);
-	R.sssi = __shfl_sync(GBA_FULL_MASK, s, base + 1);
-	R.crot = __shfl_sync(GBA_FULL_MASK, c, base + 2);
-	R.srot = __shfl_sync(GBA_FULL_MASK, s, base + 2);
-	rot_matrix(R);
 	if (t == 0) *L.next = 0;
-	if (!in) return;
-	float4* o = reinterpret_cast<float4*>(L.split.pose + kPoseRecord * p);
-	if (j == 0) {
-		o[0] = make_float4(R.m[0], R.m[1], R.m[2], R.m[3]);
-		L.split.done[p] = 0;
-	} else if (j == 1) {
-		o[1] = make_float4(R.m[4], R.m[5], R.m[6], R.m[7]);
-	} else if (j == 2) {
-		o[2] = make_float4(R.m[8], R.cphi, R.sphi, R.cssi);
-	} else {
-		o[3] = make_float4(R.sssi, R.crot, R.srot, __ldg(d));
-		o[4] = make_float4(__ldg(d + 1), __ldg(d + 2), 0.f, 0.f);
-	}
+	if (in && (t & 3) == 0) L.split.done[p] = 0;
+	write_pose_record(reinterpret_cast<const float*>(L.dofs + (in ? p : 0)), L.m.trig, in, threadIdx.x & 31,
+			L.split.pose + kPoseRecord * p);
 }
 
 /* A warp takes one 64-bead round of a pose at a time; the warp that finishes

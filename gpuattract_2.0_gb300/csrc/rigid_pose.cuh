@@ -79,7 +79,8 @@ __device__ __forceinline__ void put_pose(WarpStage& W, const PoseRot& R, float t
 
 /* Reads back what put_pose stored; the volatile reads keep the compiler from
  * holding these 18 values in registers across the bead rounds. */
-__device__ __forceinline__ PoseRot get_pose(const WarpStage& W, float& tx, float& ty, float& tz) {
+template <class Stage>
+__device__ __forceinline__ PoseRot get_pose(const Stage& W, float& tx, float& ty, float& tz) {
 	const volatile float* v = W.pose;
 	PoseRot R;
 #pragma unroll
@@ -87,6 +88,37 @@ __device__ __forceinline__ PoseRot get_pose(const WarpStage& W, float& tx, float
 	R.cphi = v[9]; R.sphi = v[10]; R.cssi = v[11]; R.sssi = v[12]; R.crot = v[13]; R.srot = v[14];
 	tx = v[15]; ty = v[16]; tz = v[17];
 	return R;
+}
+
+/* A pose's record of kPoseRecord floats -- rotation, sin/cos and translation
+ * as put_pose stores them -- by four lanes, one Euler angle each; d: the
+ * pose's DOF_6D record, j: the lane of the four.  Every lane of the warp has
+ * to call it. */
+__device__ __forceinline__ void write_pose_record(const float* __restrict__ d, const DevTrig& T, bool store, int lane,
+		float* __restrict__ out) {
+	const int j = lane & 3, base = lane & ~3;
+	float s = 0.f, c = 1.f;
+	if (j < 3) angle_sincos(__ldg(d + 3 + j), T, s, c);
+	PoseRot R;
+	R.cphi = __shfl_sync(GBA_FULL_MASK, c, base);
+	R.sphi = __shfl_sync(GBA_FULL_MASK, s, base);
+	R.cssi = __shfl_sync(GBA_FULL_MASK, c, base + 1);
+	R.sssi = __shfl_sync(GBA_FULL_MASK, s, base + 1);
+	R.crot = __shfl_sync(GBA_FULL_MASK, c, base + 2);
+	R.srot = __shfl_sync(GBA_FULL_MASK, s, base + 2);
+	rot_matrix(R);
+	if (!store) return;
+	float4* o = reinterpret_cast<float4*>(out);
+	if (j == 0) {
+		o[0] = make_float4(R.m[0], R.m[1], R.m[2], R.m[3]);
+	} else if (j == 1) {
+		o[1] = make_float4(R.m[4], R.m[5], R.m[6], R.m[7]);
+	} else if (j == 2) {
+		o[2] = make_float4(R.m[8], R.cphi, R.sphi, R.cssi);
+	} else {
+		o[3] = make_float4(R.sssi, R.crot, R.srot, __ldg(d));
+		o[4] = make_float4(__ldg(d + 1), __ldg(d + 2), 0.f, 0.f);
+	}
 }
 
 /* Staged bead record of slot s: positions, charge, torque lever, type. */
@@ -624,7 +656,8 @@ __device__ __forceinline__ void eval_round(const RigidModel& M, uint32_t i0, int
 /* A round's lane sums added over the warp in a fixed butterfly (lane
  * distances 16, 8, 4, 2, 1): lanes 2c and 2c + 1 return component c of
  * (E, Fx, Fy, Fz, T[0..8]); lanes 26..31 nothing of use.  The 13 components go
- * through the round's corner weights, which nothing reads any more: even
+ * through shared memory (`area`, 13 rows of kTotalRow floats; for the rigid
+ * kernels the round's corner weights, which nothing reads any more): even
  * lanes' values of a component and odd lanes' lie in 16 floats each, which
  * one lane loads in four words and adds up, so the reduction costs 34
  * instructions a round against 95 for 31 shuffles with their selects (which
@@ -633,15 +666,15 @@ __device__ __forceinline__ void eval_round(const RigidModel& M, uint32_t i0, int
 constexpr int kTotalRow = 36;
 static_assert(13 * kTotalRow <= kBeadsPerRound * kCornerStride, "round_total overlays the corner weights");
 static_assert(offsetof(WarpStage, cw) % 16 == 0, "round_total loads float4");
-__device__ __forceinline__ float round_total(const PoseSums& S, WarpStage& W, int lane) {
-	float* to = W.cw + (lane & 1) * 16 + (lane >> 1);
+__device__ __forceinline__ float sums_total(const PoseSums& S, float* area, int lane) {
+	float* to = area + (lane & 1) * 16 + (lane >> 1);
 	to[0] = S.E;
 	to[kTotalRow] = S.Fx; to[2 * kTotalRow] = S.Fy; to[3 * kTotalRow] = S.Fz;
 #pragma unroll
 	for (int k = 0; k < 9; ++k) to[(4 + k) * kTotalRow] = S.T[k];
 	__syncwarp();
 	const int c = min(lane >> 1, 12);
-	const float4* from = reinterpret_cast<const float4*>(W.cw + c * kTotalRow + (lane & 1) * 16);
+	const float4* from = reinterpret_cast<const float4*>(area + c * kTotalRow + (lane & 1) * 16);
 	const float4 a = from[0], b = from[1], x = from[2], y = from[3];
 	/* lanes l and l + 16 lie 8 floats apart, l and l + 8 four, ... */
 	const float4 m = make_float4(fadd(fadd(a.x, x.x), fadd(b.x, y.x)), fadd(fadd(a.y, x.y), fadd(b.y, y.y)),
@@ -651,15 +684,20 @@ __device__ __forceinline__ float round_total(const PoseSums& S, WarpStage& W, in
 	__syncwarp();   /* read before the next round's weights */
 	return t;
 }
+__device__ __forceinline__ float round_total(const PoseSums& S, WarpStage& W, int lane) {
+	return sums_total(S, W.cw, lane);
+}
 
 /* Clears the warp's running totals. */
-__device__ __forceinline__ void clear_totals(WarpStage& W, int lane) {
+template <class Stage>
+__device__ __forceinline__ void clear_totals(Stage& W, int lane) {
 	if (lane < 16) W.tot[lane] = 0.f;
 	__syncwarp();
 }
 
 /* Adds a round's component (lane 2c holds component c) to the totals. */
-__device__ __forceinline__ void add_round(WarpStage& W, float v, int lane) {
+template <class Stage>
+__device__ __forceinline__ void add_round(Stage& W, float v, int lane) {
 	if ((lane & 1) == 0) W.tot[lane >> 1] = fadd(W.tot[lane >> 1], v);
 }
 
