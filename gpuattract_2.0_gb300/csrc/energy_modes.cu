@@ -842,7 +842,7 @@ __global__ void __launch_bounds__(kModesMinThreads) minimize_modes_kernel(const 
 		const size_t p = (size_t)slot;
 		VA13<6 + 2 * MM>& va = vas[wib];
 		/* lane k holds DOF float k (pos, ang, modesRec[10], modesLig[10]) */
-		float dv = lane < 26 ? __ldg(reinterpret_cast<const float*>(M.start + p) + lane) : 0.f;
+		float dv = 0.f;
 		if (lane == 0) {
 			double x0[6 + 2 * MM];
 			const float* s = reinterpret_cast<const float*>(M.start + p);
@@ -851,23 +851,20 @@ __global__ void __launch_bounds__(kModesMinThreads) minimize_modes_kernel(const 
 			for (uint32_t m = 0; m < Ml; ++m) x0[6 + Mr + m] = s[16 + m];
 			va.start(x0, jn, M.max_evals);
 		}
+		__syncwarp();
 		float v = 0.f;
 		int nev = 0;
 		for (;;) {
-			/* lane 0 scatters the point to be evaluated into the record layout */
-			float rec[26];
-			if (lane == 0) {
-				const double* pt = va.point();
-				for (int k = 0; k < 26; ++k) rec[k] = 0.f;
-				for (int k = 0; k < 3; ++k) { rec[3 + k] = (float)pt[k]; rec[k] = (float)pt[3 + k]; }
-				for (uint32_t m = 0; m < Mr; ++m) rec[6 + m] = (float)pt[6 + m];
-				for (uint32_t m = 0; m < Ml; ++m) rec[16 + m] = (float)pt[6 + Mr + m];
-			}
-#pragma unroll
-			for (int k = 0; k < 26; ++k) {
-				const float t = __shfl_sync(GBA_FULL_MASK, lane == 0 ? rec[k] : 0.f, 0);
-				if (lane == k) dv = t;
-			}
+			/* lane j converts element j of the point (one FP64 instruction for
+			 * all); lane k takes float k of the record from its lane */
+			const float pf = lane < jn ? (float)va.point()[lane] : 0.f;
+			int from = -1;
+			if (lane < 3) from = 3 + lane;
+			else if (lane < 6) from = lane - 3;
+			else if (lane < 6 + (int)Mr) from = lane;
+			else if (lane >= 16 && lane < 16 + (int)Ml) from = lane - 10 + (int)Mr;
+			const float xf = __shfl_sync(GBA_FULL_MASK, pf, max(from, 0));
+			dv = from >= 0 ? xf : 0.f;
 			if (REF)
 				v = eval_pose_modes_ref<MM>(L, dv, lane, stage[wib], *reinterpret_cast<RefModesExtra*>(&ms[wib]),
 						L.ref_rf + (((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * L.rec.n);
@@ -887,7 +884,7 @@ __global__ void __launch_bounds__(kModesMinThreads) minimize_modes_kernel(const 
 				else src = 17 + (k - 6 - (int)Mr);
 			}
 			const float gv = __shfl_sync(GBA_FULL_MASK, v, src);
-			const double gl = neg ? -(double)gv : (double)gv;
+			const double gl = (double)(neg ? -gv : gv);
 			const float e = __shfl_sync(GBA_FULL_MASK, v, 0);
 			va.provide_w((double)e, [&](int) { return gl; }, VaWarp{lane});
 			/* lane 0's reading for all: no lane may see a state that lane 0,

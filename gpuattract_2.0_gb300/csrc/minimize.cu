@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(256, REF ? 2 : 4) minimize_rigid_kernel(const 
 			const size_t p = L.order ? (size_t)__ldg(&L.order[slot]) : slot;
 			const RigidModel& M = L.models[L.pair_of ? __ldg(&L.pair_of[p]) : 0u];
 			VA13<6>& va = vas[threadIdx.x >> 5];
-			float cur[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 			float res[7];
+			float pf = 0.f;      /* lane j < 6: element j of the point, (ang xyz, pos xyz) */
 			int nev = 0;
 			if (lane == 0) {
 				const gba_dof6d s = L.start[p];
@@ -117,14 +117,13 @@ __global__ void __launch_bounds__(256, REF ? 2 : 4) minimize_rigid_kernel(const 
 				const double x0[6] = {s.ang[0], s.ang[1], s.ang[2], s.pos[0], s.pos[1], s.pos[2]};
 				va.start(x0, 6, L.max_evals);
 			}
+			__syncwarp();
 			for (;;) {
-				if (lane == 0) {
-					const double* pt = va.point();
-					cur[0] = (float)pt[3]; cur[1] = (float)pt[4]; cur[2] = (float)pt[5];
-					cur[3] = (float)pt[0]; cur[4] = (float)pt[1]; cur[5] = (float)pt[2];
-				}
+				/* one conversion for the six elements (an FP64 instruction) */
+				if (lane < 6) pf = (float)va.point()[lane];
+				float cur[6];
 #pragma unroll
-				for (int k = 0; k < 6; ++k) cur[k] = __shfl_sync(GBA_FULL_MASK, cur[k], 0);
+				for (int k = 0; k < 6; ++k) cur[k] = __shfl_sync(GBA_FULL_MASK, pf, k < 3 ? k + 3 : k - 3);
 				if (REF)
 					eval_pose_rigid_ref(M, cur[0], cur[1], cur[2], cur[3], cur[4], cur[5], lane, stage[threadIdx.x >> 5],
 							res);
@@ -134,7 +133,7 @@ __global__ void __launch_bounds__(256, REF ? 2 : 4) minimize_rigid_kernel(const 
 				++nev;
 				/* objective E, gradient -(ang, pos), src/apps/em/meta.h:114-121;
 				 * the whole warp steps the machine, lane j holding element j */
-				const double gl = -(double)rigid_grad_entry(res, lane);
+				const double gl = (double)-rigid_grad_entry(res, lane);
 				va.provide_w((double)res[0], [&](int) { return gl; }, VaWarp{lane});
 				/* lane 0's reading for all: no lane may see a state that lane 0,
 				 * gone on to the next pose, has already restarted */
@@ -151,7 +150,8 @@ __global__ void __launch_bounds__(256, REF ? 2 : 4) minimize_rigid_kernel(const 
 				}
 			}
 			store_result7(reinterpret_cast<float*>(L.out_result + p), res, lane);
-			if (lane < 6) reinterpret_cast<float*>(L.out_state + p)[lane] = cur[lane];
+			const float xf = __shfl_sync(GBA_FULL_MASK, pf, lane < 3 ? lane + 3 : lane - 3);
+			if (lane < 6) reinterpret_cast<float*>(L.out_state + p)[lane] = xf;
 			if (lane == 0 && L.out_nevals) L.out_nevals[p] = nev;
 			if (lane == 0 && L.done_ns) L.done_ns[p] = global_ns();
 		}
@@ -205,33 +205,36 @@ __device__ __forceinline__ void pipe_claim(const MinLaunch& L, PipeSlot& S, unsi
 }
 
 /* The control warp, every lane: hands the evaluation of slot S to its VA13
- * (the warp form); then lane 0 alone (t_start is its own) ends the pose --
- * outputs written, slot refilled -- or readies its next point. */
+ * (the warp form) and readies its next point, or lane 0 alone (t_start is its
+ * own) ends the pose -- outputs written, slot refilled. */
 __device__ __forceinline__ void pipe_consume(const MinLaunch& L, PipeSlot& S, unsigned long long t_start,
 		unsigned long long budget, int lane) {
 	/* objective E, gradient -(ang, pos), src/apps/em/meta.h:114-121 */
-	const double gl = -(double)rigid_grad_entry(S.res, lane);
+	const double gl = (double)-rigid_grad_entry(S.res, lane);
 	S.va.provide_w((double)S.res[0], [&](int) { return gl; }, VaWarp{lane});
-	if (lane != 0) return;
-	S.evaluated = 0;
-	++S.nev;
-	bool stop = S.va.done();
-	/* VA13 ends within max_evals + 1 evaluations; anything past that is a
-	 * broken machine, reported instead of looping */
-	if (!stop && S.nev > L.max_evals + 1) {
-		atomicExch(L.status, GBA_ERR_DEVICE_CHECK);
-		stop = true;
+	int stop = 0;
+	if (lane == 0) {
+		S.evaluated = 0;
+		++S.nev;
+		stop = S.va.done();
+		/* VA13 ends within max_evals + 1 evaluations; anything past that is a
+		 * broken machine, reported instead of looping */
+		if (!stop && S.nev > L.max_evals + 1) {
+			atomicExch(L.status, GBA_ERR_DEVICE_CHECK);
+			stop = 1;
+		}
+		if (!stop && (S.nev & 15) == 0 && global_ns() - t_start > budget) {
+			atomicExch(L.status, GBA_ERR_TIMEOUT);
+			stop = 1;
+		}
 	}
-	if (!stop && (S.nev & 15) == 0 && global_ns() - t_start > budget) {
-		atomicExch(L.status, GBA_ERR_TIMEOUT);
-		stop = true;
-	}
-	if (!stop) {
-		const double* pt = S.va.point();
-		S.cur[0] = (float)pt[3]; S.cur[1] = (float)pt[4]; S.cur[2] = (float)pt[5];
-		S.cur[3] = (float)pt[0]; S.cur[4] = (float)pt[1]; S.cur[5] = (float)pt[2];
+	if (!__shfl_sync(GBA_FULL_MASK, stop, 0)) {
+		/* one conversion for the six elements (an FP64 instruction) */
+		if (lane < 6) S.cur[lane < 3 ? lane + 3 : lane - 3] = (float)S.va.point()[lane];
+		__syncwarp();
 		return;
 	}
+	if (lane != 0) return;
 	float* r = reinterpret_cast<float*>(L.out_result + S.p);
 	float* x = reinterpret_cast<float*>(L.out_state + S.p);
 	for (int k = 0; k < 7; ++k) r[k] = S.res[k];

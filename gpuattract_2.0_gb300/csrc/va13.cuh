@@ -23,11 +23,16 @@
 #define GBA_HD inline
 #endif
 
-/* Device loops of the machine stay rolled: it runs between two evaluations
- * of the whole warp, and unrolled copies of its loops evicted the
- * evaluation's code from the instruction cache (measured with one lane
- * stepping it: instruction-fetch stalls; the minimizers ran 7-9 % slower
- * unrolled). */
+/* Device code of the machine stays small: its loops rolled, its divisions in
+ * one function (va_div), mc11a there once.  It runs between two evaluations,
+ * the warps of an SM are spread over both, and what the instruction cache
+ * does not hold every one of them waits for: with the warp form's loops
+ * unrolled by the compiler and its divisions inline the rigid kernel was
+ * 159 KB long (now 97 KB, the scoring kernel 39) and its warps spent 15 of 27
+ * cycles per instruction waiting for code (now 9 of 21; 8,000 poses of a
+ * 120-bead ligand, 40 evaluations: 13.4 -> 10.2 ms).  Fewer FP64
+ * instructions at the price of more code lost: divisions and comparisons in
+ * integer arithmetic 14.5 ms. */
 #ifdef __CUDA_ARCH__
 #define GBA_VA_LOOP _Pragma("unroll 1")
 #else
@@ -44,6 +49,19 @@ namespace gba {
 GBA_HD double va_max(double a, double b) { return a < b ? b : a; }
 GBA_HD double va_min(double a, double b) { return b < a ? b : a; }
 GBA_HD double va_abs(double a) { return fabs(a); }
+
+/* Division of the warp form: out of line on the device (sixteen places of a
+ * step divide). */
+#ifdef __CUDACC__
+static __device__ __noinline__ double va_div_device(double x, double y) { return x / y; }
+#endif
+GBA_HD double va_div(double x, double y) {
+#ifdef __CUDA_ARCH__
+	return va_div_device(x, y);
+#else
+	return x / y;
+#endif
+}
 
 /* Products are never contracted with a following add: the host build runs
  * with -ffp-contract=off and the device uses round-to-nearest multiplies, so
@@ -294,24 +312,26 @@ GBA_HD void mc11a_w(double* a, int n, double* z, double sig, double* w, int& ir,
 	int mm = 0;
 	if (sig > 0.0) goto L40;
 	if (sig == 0.0 || ir == 0) return;
-	ti = 1.0 / sig;
+	ti = va_div(1.0, sig);
 	if (mk == 0) goto L10;
 	if (ir > 0) {
 		ex.each(1, n, [&](int j) {
 			const double dj = a[va_diag(j, n)];
-			q[j] = dj != 0.0 ? vm(w[j], w[j]) / dj : 0.0;
+			q[j] = dj != 0.0 ? va_div(vm(w[j], w[j]), dj) : 0.0;
 		});
+		GBA_VA_LOOP
 		for (int i = 1; i <= n; ++i)
 			if (a[va_diag(i, n)] != 0.0) ti = ti + q[i];
 	}
 	goto L20;
 L10:
 	ex.each(1, n, [&](int j) { w[j] = z[j]; });
+	GBA_VA_LOOP
 	for (int i = 1; i <= n; ++i) {
 		const int ij = va_diag(i, n);
 		const double v = w[i];
 		if (a[ij] > 0.0) {
-			ti = ti + vm(v, v) / a[ij];
+			ti = ti + va_div(vm(v, v), a[ij]);
 			if (i != n) ex.each(i + 1, n, [&](int j) { w[j] = w[j] - vm(v, a[ij + j - i]); });
 		} else {
 			ex.each(i, i, [&](int) { w[i] = 0.0; });
@@ -324,7 +344,7 @@ L20:
 		goto L23;
 	}
 	if (ti > 0.0) {
-		ti = eps / sig;
+		ti = va_div(eps, sig);
 		if (eps == 0.0) ir = ir - 1;
 		goto L23;
 	}
@@ -333,9 +353,10 @@ L23:
 	mm = 1;
 	ex.each(1, n, [&](int j) {
 		const double dj = a[va_diag(j, n)];
-		q[j] = dj != 0.0 ? vm(w[j], w[j]) / dj : 0.0;
+		q[j] = dj != 0.0 ? va_div(vm(w[j], w[j]), dj) : 0.0;
 	});
 	tim = ti;
+	GBA_VA_LOOP
 	for (int i = 1; i <= n; ++i) {
 		const int j = np - i;
 		if (a[va_diag(j, n)] != 0.0) tim = ti - q[j];
@@ -346,10 +367,11 @@ L23:
 	goto L41;
 L40:
 	mm = 0;
-	tim = 1.0 / sig;
+	tim = va_div(1.0, sig);
 L41: {
 	bool have_al = false;
 	double al = 0.0;
+	GBA_VA_LOOP
 	for (int i = 1; i <= n; ++i) {
 		const int ij = va_diag(i, n);
 		const double v = z[i];
@@ -362,12 +384,12 @@ L41: {
 			}
 			ir = 1 - ir;
 			ex.each(i, n, [&](int j) {
-				if (j == i) a[ij] = vm(v, v) / tim;
-				else a[ij + j - i] = z[j] / v;
+				if (j == i) a[ij] = va_div(vm(v, v), tim);
+				else a[ij + j - i] = va_div(z[j], v);
 			});
 			return;
 		}
-		if (!have_al) al = v / aii;
+		if (!have_al) al = va_div(v, aii);
 		if (mm <= 0) ti = tim + vm(v, al);
 		else ti = w[i];
 		ex.each(0, 3, [&](int k) {
@@ -382,7 +404,7 @@ L41: {
 					de = a[va_diag(i + 1, n)];
 				}
 			}
-			q[k] = nu / de;
+			q[k] = va_div(nu, de);
 		});
 		const double r = q[0], b = q[1], gm = q[2];
 		al = q[3];
@@ -431,10 +453,11 @@ GBA_HD void mc11e_w(const double* a, int n, double* z, double* w, int ir, double
 	if (n <= 1) {
 		ex.each(1, 1, [&](int) {
 			w[1] = z[1];
-			z[1] = z[1] / a[1];
+			z[1] = va_div(z[1], a[1]);
 		});
 		return;
 	}
+	GBA_VA_LOOP
 	for (int j = 1; j < n; ++j) {
 		const double zj = z[j];
 		const int dj = va_diag(j, n);
@@ -447,14 +470,16 @@ GBA_HD void mc11e_w(const double* a, int n, double* z, double* w, int ir, double
 	const int dm = va_diag(n - 1, n);
 	ex.each(1, n, [&](int i) {
 		if (i == 1) w[1] = z[1];
-		q[i] = z[i] / a[va_diag(i, n)];
+		q[i] = va_div(z[i], a[va_diag(i, n)]);
 		if (i == n) {
 			z[n] = q[n];
 			t[n] = vm(a[dm + 1], q[n]);
 		}
 	});
+	GBA_VA_LOOP
 	for (int i = n - 1; i >= 1; --i) {
 		double v = q[i];
+		GBA_VA_LOOP
 		for (int j = i + 1; j <= n; ++j) v = v - t[j];
 		/* z_i final; the products of row i - 1 (z_i's from v) */
 		const int dp = i > 1 ? va_diag(i - 1, n) : 0;
@@ -679,8 +704,9 @@ struct VA13 {
 		});
 	L220:
 		dgb = xnull;
+		ex.each(1, jn, [&](int j) { t[j] = vm(gb[j], d[j]); });
 		GBA_VA_LOOP
-		for (i = 1; i <= jn; ++i) dgb = dgb + vm(gb[i], d[i]);
+		for (i = 1; i <= jn; ++i) dgb = dgb + t[i];
 		if (fb - fa <= vm(vm(0.1, c), dga)) goto L280;
 		if (step > steplb) goto L270;
 	L240:
@@ -689,8 +715,8 @@ struct VA13 {
 		goto Lsave;
 	L270:
 		stepbd = step;
-		c = gmin + dgb - vm(3.0, fb - fmin) / step;
-		c = gmin / (c + gmin - sqrt(vm(c, c) - vm(gmin, dgb)));
+		c = gmin + dgb - va_div(vm(3.0, fb - fmin), step);
+		c = va_div(gmin, c + gmin - sqrt(vm(c, c) - vm(gmin, dgb)));
 		step = vm(step, va_max(0.1, c));
 		goto L170;
 	L280:
@@ -700,8 +726,8 @@ struct VA13 {
 		gmin = dgb;
 		step = vm(9.0, stmin);
 		if (stepbd > xnull) step = vm(0.5, stepbd);
-		c = dga + vm(3.0, dgb) - vm(4.0, fb - fa) / stmin;
-		if (c > xnull) step = va_min(step, vm(stmin, va_max(1.0, -dgb / c)));
+		c = dga + vm(3.0, dgb) - va_div(vm(4.0, fb - fa), stmin);
+		if (c > xnull) step = va_min(step, vm(stmin, va_max(1.0, va_div(-dgb, c))));
 		if (dgb < vm(0.7, dga)) goto L170;
 		isfv = 4 - isfv;
 		if (stmin + step <= steplb) goto L240;
@@ -712,9 +738,13 @@ struct VA13 {
 			d[j] = gb[j] - ga[j];
 			ga[j] = gb[j];
 		});
-		mc11a_w(h, jn, xbb, 1.0 / dga, w, ir, 1, xnull, q, t, ex);
-		ir = -ir;
-		mc11a_w(h, jn, d, 1.0 / vm(stmin, dgb - dga), d, ir, 0, xnull, q, t, ex);
+		/* minfor's two updates in one loop, so that mc11a's code is there once */
+		GBA_VA_LOOP
+		for (int u = 0; u < 2; ++u) {
+			if (u == 1) ir = -ir;
+			mc11a_w(h, jn, u == 0 ? xbb : d, va_div(1.0, u == 0 ? dga : vm(stmin, dgb - dga)), u == 0 ? w : d, ir, 1 - u,
+					xnull, q, t, ex);
+		}
 		if (ir < jn) {
 			phase = kDone;
 			goto Lsave;
@@ -732,20 +762,21 @@ struct VA13 {
 		mc11e_w(h, jn, d, w, jn, q, t, ex);
 		c = xnull;
 		dga = xnull;
+		ex.each(1, jn, [&](int j) { t[j] = vm(ga[j], d[j]); });
 		GBA_VA_LOOP
 		for (i = 1; i <= jn; ++i) {
 			c = va_max(c, va_abs(d[i]));
-			dga = dga + vm(ga[i], d[i]);
+			dga = dga + t[i];
 		}
 		if (dga >= xnull) goto L240;
 		stmin = xnull;
 		stepbd = xnull;
-		steplb = acc / c;
+		steplb = va_div(acc, c);
 		fmin = fa;
 		gmin = dga;
 		step = 1.0;
-		if (dff <= xnull) step = va_min(step, 1.0 / c);
-		if (dff > xnull) step = va_min(step, (dff + dff) / (-dga));
+		if (dff <= xnull) step = va_min(step, va_div(1.0, c));
+		if (dff > xnull) step = va_min(step, va_div(dff + dff, -dga));
 	L170:
 		c = stmin + step;
 		if (nfun >= ivmax) {
