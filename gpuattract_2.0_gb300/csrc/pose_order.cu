@@ -121,36 +121,53 @@ __global__ void bucket_keys_kernel(const float* __restrict__ dofs, size_t stride
 	rank[p] = atomicAdd(&count[b], 1u);
 }
 
-/* Exclusive prefix sum of the kBuckets counts, one 1024-thread block. */
+/* Exclusive prefix sum of the kBuckets counts, one 1024-thread block.  Bound
+ * by the latency of its loads: a thread reading 32 counts in a row (128 bytes
+ * from its neighbour's) took 34 us; here the block reads eight tiles of
+ * 4,096 counts in 16-byte words, all in flight together: 6.3 us. */
 __global__ void __launch_bounds__(1024) bucket_scan_kernel(uint32_t* __restrict__ count) {
-	constexpr int per = kBuckets / 1024;
-	__shared__ uint32_t warp_tot[32];
+	constexpr int kTiles = kBuckets / 4096;
+	static_assert(kBuckets % 4096 == 0 && kTiles <= 32, "whole tiles, one warp each for their totals");
+	__shared__ uint32_t warp_tot[kTiles][32];
+	__shared__ uint32_t tile_tot[kTiles];
 	const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-	uint32_t v[per];
-	uint32_t sum = 0;
+	uint4* c = reinterpret_cast<uint4*>(count);
+	uint4 v[kTiles];
 #pragma unroll
-	for (int k = 0; k < per; ++k) { v[k] = count[t * per + k]; sum += v[k]; }
-	uint32_t incl = sum;
+	for (int k = 0; k < kTiles; ++k) v[k] = c[k * 1024 + t];
+	uint32_t incl[kTiles];
 #pragma unroll
-	for (int o = 1; o < 32; o <<= 1) {
-		const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
-		if (lane >= o) incl += x;
-	}
-	if (lane == 31) warp_tot[w] = incl;
+	for (int k = 0; k < kTiles; ++k) incl[k] = v[k].x + v[k].y + v[k].z + v[k].w;
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+		for (int k = 0; k < kTiles; ++k) {
+			const uint32_t x = __shfl_up_sync(0xffffffffu, incl[k], o);
+			if (lane >= o) incl[k] += x;
+		}
+	if (lane == 31)
+#pragma unroll
+		for (int k = 0; k < kTiles; ++k) warp_tot[k][w] = incl[k];
 	__syncthreads();
-	if (w == 0) {
-		uint32_t x = warp_tot[lane], xi = x;
+	if (w < kTiles) {
+		const uint32_t x = warp_tot[w][lane];
+		uint32_t xi = x;
 #pragma unroll
 		for (int o = 1; o < 32; o <<= 1) {
 			const uint32_t y = __shfl_up_sync(0xffffffffu, xi, o);
 			if (lane >= o) xi += y;
 		}
-		warp_tot[lane] = xi - x;
+		warp_tot[w][lane] = xi - x;
+		if (lane == 31) tile_tot[w] = xi;
 	}
 	__syncthreads();
-	uint32_t run = warp_tot[w] + incl - sum;
+	uint32_t before = 0;
 #pragma unroll
-	for (int k = 0; k < per; ++k) { count[t * per + k] = run; run += v[k]; }
+	for (int k = 0; k < kTiles; ++k) {
+		const uint32_t x = before + warp_tot[k][w] + incl[k] - (v[k].x + v[k].y + v[k].z + v[k].w);
+		c[k * 1024 + t] = make_uint4(x, x + v[k].x, x + v[k].x + v[k].y, x + v[k].x + v[k].y + v[k].z);
+		before += tile_tot[k];
+	}
 }
 
 __global__ void bucket_scatter_kernel(size_t n, const uint32_t* __restrict__ start,
