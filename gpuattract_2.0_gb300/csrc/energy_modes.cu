@@ -39,6 +39,9 @@
  * src/model/transform_modes.cu:154, src/model/reduction_modes.cu:68-69).
  */
 #include <algorithm>
+#include <array>
+#include <map>
+#include <mutex>
 
 #include "rigid_pose.cuh"
 #include "va13.cuh"
@@ -198,6 +201,45 @@ __device__ __forceinline__ ModesFrame modes_frame(const float dv, const int lane
 	return F;
 }
 
+/* Stages 64 receptor beads from j0: deformed, moved into the ligand frame,
+ * their lookups in the LIGAND grid queued, their mode vectors rotated for the
+ * cooperative lookups.  Returns the number of lookups. */
+template <int MM>
+__device__ __forceinline__ uint32_t modes_rec_stage(const ModesLaunch& L, const ModesFrame& F, const float ampR[MM],
+		const uint32_t j0, const int lane, WarpStage& W, ModeStage<MM>& MS) {
+	const uint32_t Mr = L.rec.n_modes;
+	uint32_t nlk[2];
+	BeadGrid bg[2];
+#pragma unroll
+	for (int h = 0; h < 2; ++h) {
+		const int s = lane + 32 * h;
+		const uint32_t j = j0 + s;
+		nlk[h] = 0;
+		bg[h] = BeadGrid{0u, 0u};
+		if (j < L.rec.n) {
+			const float4 r = __ldg(&L.rec.xyzq[j]);
+			const uint32_t mapped = __ldg(&L.rec.tm[j]) >> 16;
+			float vw[4 * kModeWords<MM>];
+			load_modes<MM>(L.rec_modes + (size_t)j * L.rec_ms, Mr, vw);
+			float x = r.x, y = r.y, z = r.z;
+			deform_w<MM>(vw, Mr, ampR, x, y, z);
+			float px, py, pz;
+			rot_apply(F.Ri, x, y, z, px, py, pz);
+			px = fadd(px, F.ip[0]); py = fadd(py, F.ip[1]); pz = fadd(pz, F.ip[2]);
+			put_bead(W, s, 0.f, 0.f, 0.f, px, py, pz, r.w, j);
+			nlk[h] = stage_grid(L.grid_lig, px, py, pz, mapped, r.w, s, W, bg[h]);
+			/* the ligand-frame force f is rotated back by R before the
+			 * projection: (R f) . v = f . (R^T v); staged for the
+			 * cooperative lookups only (one lookup per bead or two: the
+			 * per-lane form rotates f instead) */
+			if (nlk[h] && L.grid_lig.coop_lookup) stage_modes<MM>(MS, s, vw, Mr, F.R.m, true);
+		}
+	}
+	const uint32_t n_look = queue_lookups(W, nlk, bg, lane);
+	__syncwarp();
+	return n_look;
+}
+
 /* Receptor pass: the receptor beads, deformed and moved into the ligand
  * frame, in the LIGAND grid; each force rotated back by R and projected on
  * the receptor modes into the lane sums gR. */
@@ -205,40 +247,9 @@ template <int MM>
 __device__ __forceinline__ void modes_rec_pass(const ModesLaunch& L, const ModesFrame& F, const float ampR[MM],
 		const int lane, WarpStage& W, ModeStage<MM>& MS, float gR[MM]) {
 	const uint32_t Mr = L.rec.n_modes;
-	const PoseRot& R = F.R;
-	const float* Ri = F.Ri;
-	const float ipx = F.ip[0], ipy = F.ip[1], ipz = F.ip[2];
 	const int comp = coop_component(lane);
 	for (uint32_t j0 = 0; j0 < L.rec.n; j0 += kBeadsPerRound) {
-		uint32_t nlk[2];
-		BeadGrid bg[2];
-#pragma unroll
-		for (int h = 0; h < 2; ++h) {
-			const int s = lane + 32 * h;
-			const uint32_t j = j0 + s;
-			nlk[h] = 0;
-			bg[h] = BeadGrid{0u, 0u};
-			if (j < L.rec.n) {
-				const float4 r = __ldg(&L.rec.xyzq[j]);
-				const uint32_t mapped = __ldg(&L.rec.tm[j]) >> 16;
-				float vw[4 * kModeWords<MM>];
-				load_modes<MM>(L.rec_modes + (size_t)j * L.rec_ms, Mr, vw);
-				float x = r.x, y = r.y, z = r.z;
-				deform_w<MM>(vw, Mr, ampR, x, y, z);
-				float px, py, pz;
-				rot_apply(Ri, x, y, z, px, py, pz);
-				px = fadd(px, ipx); py = fadd(py, ipy); pz = fadd(pz, ipz);
-				put_bead(W, s, 0.f, 0.f, 0.f, px, py, pz, r.w, j);
-				nlk[h] = stage_grid(L.grid_lig, px, py, pz, mapped, r.w, s, W, bg[h]);
-				/* the ligand-frame force f is rotated back by R before the
-				 * projection: (R f) . v = f . (R^T v); staged for the
-				 * cooperative lookups only (one lookup per bead or two: the
-				 * per-lane form rotates f instead) */
-				if (nlk[h] && L.grid_lig.coop_lookup) stage_modes<MM>(MS, s, vw, Mr, R.m, true);
-			}
-		}
-		const uint32_t n_look = queue_lookups(W, nlk, bg, lane);
-		__syncwarp();
+		const uint32_t n_look = modes_rec_stage<MM>(L, F, ampR, j0, lane, W, MS);
 		if (L.grid_lig.coop_lookup) {
 			for (uint32_t k0 = 0; k0 < n_look; k0 += 16) {
 				CoopStep<2> st;
@@ -255,13 +266,97 @@ __device__ __forceinline__ void modes_rec_pass(const ModesLaunch& L, const Modes
 				const float4 v = grid_lookup(L.grid_lig, W, q);
 				/* back into the receptor frame, then -(force . mode) */
 				float fx, fy, fz;
-				rot_apply(R.m, v.x, v.y, v.z, fx, fy, fz);
+				rot_apply(F.R.m, v.x, v.y, v.z, fx, fy, fz);
 				project<MM>(L.rec_modes + (size_t)__float_as_uint(W.ut[s].w) * L.rec_ms, Mr, fx, fy, fz, -1.f, gR);
 			}
 		}
 		__syncwarp();
 	}
 
+}
+
+/* Stages 64 ligand beads from i0: deformed, moved into the receptor frame,
+ * lookups and neighbour lists queued, mode vectors rotated.  Returns the
+ * number of lookups; n_pair, nln, start as queue_pairs has them. */
+template <int MM>
+__device__ __forceinline__ uint32_t modes_lig_stage(const ModesLaunch& L, const ModesFrame& F, const float ampL[MM],
+		const uint32_t i0, const int lane, WarpStage& W, ModeStage<MM>& MS, uint32_t nln[2], uint32_t start[2],
+		uint32_t& n_pair) {
+	const uint32_t Ml = L.lig.n_modes;
+	uint32_t nlk[2];
+	BeadGrid bg[2];
+#pragma unroll
+	for (int h = 0; h < 2; ++h) {
+		const int s = lane + 32 * h;
+		const uint32_t i = i0 + s;
+		nlk[h] = 0;
+		nln[h] = 0;
+		bg[h] = BeadGrid{0u, 0u};
+		if (i < L.lig.n) {
+			const float4 b = __ldg(&L.lig.xyzq[i]);
+			const uint32_t tm = __ldg(&L.lig.tm[i]);
+			const uint32_t type = tm & 0xffffu, mapped = tm >> 16;
+			float vw[4 * kModeWords<MM>];
+			load_modes<MM>(L.lig_modes + (size_t)i * L.lig_ms, Ml, vw);
+			float x = b.x, y = b.y, z = b.z;
+			deform_w<MM>(vw, Ml, ampL, x, y, z);
+			float px, py, pz;
+			rot_apply(F.R.m, x, y, z, px, py, pz);
+			px = fadd(px, F.t[0]); py = fadd(py, F.t[1]); pz = fadd(pz, F.t[2]);
+			put_bead(W, s, b.x, b.y, b.z, px, py, pz, b.w, type);
+			nlk[h] = stage_grid(L.grid_rec, px, py, pz, mapped, b.w, s, W, bg[h]);
+			bool in_nl;
+			if (type != 0) nln[h] = stage_nl(L.grid_rec.nl, px, py, pz, s, W, in_nl);
+			/* the global-frame force f is projected in the ligand frame:
+			 * (R^T f) . v = f . (R v) */
+			if (nlk[h] | nln[h]) stage_modes<MM>(MS, s, vw, Ml, F.R.m, false);
+		}
+	}
+	const uint32_t n_look = queue_lookups(W, nlk, bg, lane);
+	n_pair = queue_pairs(W, nln, lane, start);
+	__syncwarp();
+	return n_look;
+}
+
+/* One flattened pair -- ligand bead staged in slot s, list entry at `at` --
+ * against the deformed receptor: receptor bead j, its mode vectors vw, force
+ * and energy; false outside the plateau. */
+template <int MM>
+__device__ __forceinline__ bool modes_pair(const ModesLaunch& L, const float ampR[MM], const WarpStage& W, uint32_t s,
+		uint32_t at, uint32_t& j, float (&vw)[4 * kModeWords<MM>], float& fx, float& fy, float& fz, float& e) {
+	const uint32_t Mr = L.rec.n_modes;
+	j = __ldg(&L.grid_rec.nl.list[at]);
+	const float4 r = __ldg(&L.rec.xyzq[j]);
+	float rx = r.x, ry = r.y, rz = r.z;
+	load_modes<MM>(L.rec_modes + (size_t)j * L.rec_ms, Mr, vw);
+	deform_w<MM>(vw, Mr, ampR, rx, ry, rz);
+	const uint32_t trec = __ldg(&L.rec.tm[j]) & 0xffffu;
+	const float4 b = W.pq[s];
+	return nl_pair(L.grid_rec.nl, L.par, __float_as_uint(W.ut[s].w), b.w, b.x, b.y, b.z, rx, ry, rz, r.w, trec, fx, fy,
+			fz, e);
+}
+
+/* gR[m] += f . v_m: the reaction on a receptor bead is -f, and its mode
+ * gradient gets -(-f . v). */
+template <int MM>
+__device__ __forceinline__ void project_reaction(const float (&vw)[4 * kModeWords<MM>], uint32_t Mr, float fx, float fy,
+		float fz, float gR[MM]) {
+#pragma unroll
+	for (int m = 0; m < MM; ++m)
+		if (m < (int)Mr)
+			gR[m] = ffma(1.f, ffma(fz, vw[3 * m + 2], ffma(fy, vw[3 * m + 1], fmul(fx, vw[3 * m]))), gR[m]);
+}
+
+/* A finished component f of a lookup in slot s, on the lane holding component
+ * comp: the cooperative sums without the ligand modes. */
+__device__ __forceinline__ void coop_add(const WarpStage& W, uint32_t s, int comp, float f, CoopSums& C) {
+	C.f = fadd(C.f, f);
+	if (comp != 3) {
+		const float4 u = W.ut[s];
+		C.t0 = ffma(u.x, f, C.t0);
+		C.t1 = ffma(u.y, f, C.t1);
+		C.t2 = ffma(u.z, f, C.t2);
+	}
 }
 
 /* Ligand pass: the ligand beads, deformed and moved into the receptor frame,
@@ -273,43 +368,10 @@ __device__ __forceinline__ void modes_lig_pass(const ModesLaunch& L, const Modes
 		const float ampL[MM], const int lane, WarpStage& W, ModeStage<MM>& MS, PoseSums& S, CoopSums& C,
 		float gL[MM], float gR[MM]) {
 	const uint32_t Mr = L.rec.n_modes, Ml = L.lig.n_modes;
-	const PoseRot& R = F.R;
-	const float tx = F.t[0], ty = F.t[1], tz = F.t[2];
 	const int comp = coop_component(lane);
 	for (uint32_t i0 = 0; i0 < L.lig.n; i0 += kBeadsPerRound) {
-		uint32_t nlk[2], nln[2];
-		BeadGrid bg[2];
-#pragma unroll
-		for (int h = 0; h < 2; ++h) {
-			const int s = lane + 32 * h;
-			const uint32_t i = i0 + s;
-			nlk[h] = 0;
-			nln[h] = 0;
-			bg[h] = BeadGrid{0u, 0u};
-			if (i < L.lig.n) {
-				const float4 b = __ldg(&L.lig.xyzq[i]);
-				const uint32_t tm = __ldg(&L.lig.tm[i]);
-				const uint32_t type = tm & 0xffffu, mapped = tm >> 16;
-				float vw[4 * kModeWords<MM>];
-				load_modes<MM>(L.lig_modes + (size_t)i * L.lig_ms, Ml, vw);
-				float x = b.x, y = b.y, z = b.z;
-				deform_w<MM>(vw, Ml, ampL, x, y, z);
-				float px, py, pz;
-				rot_apply(R.m, x, y, z, px, py, pz);
-				px = fadd(px, tx); py = fadd(py, ty); pz = fadd(pz, tz);
-				put_bead(W, s, b.x, b.y, b.z, px, py, pz, b.w, type);
-				nlk[h] = stage_grid(L.grid_rec, px, py, pz, mapped, b.w, s, W, bg[h]);
-				bool in_nl;
-				if (type != 0) nln[h] = stage_nl(L.grid_rec.nl, px, py, pz, s, W, in_nl);
-				/* the global-frame force f is projected in the ligand frame:
-				 * (R^T f) . v = f . (R v) */
-				if (nlk[h] | nln[h]) stage_modes<MM>(MS, s, vw, Ml, R.m, false);
-			}
-		}
-		const uint32_t n_look = queue_lookups(W, nlk, bg, lane);
-		uint32_t start[2];
-		const uint32_t n_pair = queue_pairs(W, nln, lane, start);
-		__syncwarp();
+		uint32_t nln[2], start[2], n_pair;
+		const uint32_t n_look = modes_lig_stage<MM>(L, F, ampL, i0, lane, W, MS, nln, start, n_pair);
 		if (L.grid_rec.coop_lookup) {
 			for (uint32_t k0 = 0; k0 < n_look; k0 += 16) {
 				CoopStep<2> st;
@@ -319,14 +381,8 @@ __device__ __forceinline__ void modes_lig_pass(const ModesLaunch& L, const Modes
 					const float v = st.component(b, lane);
 					if (st.ok[b]) {
 						const float f = fmul(v, st.sc[b]);
-						C.f = fadd(C.f, f);
-						if (comp != 3) {
-							const float4 u = W.ut[st.sl[b]];
-							C.t0 = ffma(u.x, f, C.t0);
-							C.t1 = ffma(u.y, f, C.t1);
-							C.t2 = ffma(u.z, f, C.t2);
-							project_component<MM>(MS, st.sl[b], comp, Ml, f, gL);
-						}
+						coop_add(W, st.sl[b], comp, f, C);
+						if (comp != 3) project_component<MM>(MS, st.sl[b], comp, Ml, f, gL);
 					}
 				}
 			}
@@ -350,25 +406,12 @@ __device__ __forceinline__ void modes_lig_pass(const ModesLaunch& L, const Modes
 				const uint32_t q = w + 32 * h + lane;
 				if (q >= n_pair) continue;
 				const uint32_t s = so[h];
-				const uint32_t j = __ldg(&L.grid_rec.nl.list[W.lbase[s] + q]);
-				const float4 r = __ldg(&L.rec.xyzq[j]);
-				float rx = r.x, ry = r.y, rz = r.z;
-				float vw[4 * kModeWords<MM>];
-				load_modes<MM>(L.rec_modes + (size_t)j * L.rec_ms, Mr, vw);
-				deform_w<MM>(vw, Mr, ampR, rx, ry, rz);
-				const uint32_t trec = __ldg(&L.rec.tm[j]) & 0xffffu;
-				const float4 b = W.pq[s];
+				uint32_t j;
+				float vw[4 * kModeWords<MM>], fx, fy, fz, e;
+				if (!modes_pair<MM>(L, ampR, W, s, W.lbase[s] + q, j, vw, fx, fy, fz, e)) continue;
 				const float4 u = W.ut[s];
-				float fx, fy, fz, e;
-				if (!nl_pair(L.grid_rec.nl, L.par, __float_as_uint(u.w), b.w, b.x, b.y, b.z, rx, ry, rz,
-						r.w, trec, fx, fy, fz, e))
-					continue;
 				S.add(e, fx, fy, fz, u.x, u.y, u.z);
-				/* reaction on receptor bead j is -f: its mode gradient gets -(-f . v) */
-#pragma unroll
-				for (int m = 0; m < MM; ++m)
-					if (m < (int)Mr)
-						gR[m] = ffma(1.f, ffma(fz, vw[3 * m + 2], ffma(fy, vw[3 * m + 1], fmul(fx, vw[3 * m]))), gR[m]);
+				project_reaction<MM>(vw, Mr, fx, fy, fz, gR);
 				project_staged<MM>(MS, s, Ml, fx, fy, fz, -1.f, gL);
 			}
 		}
@@ -376,29 +419,17 @@ __device__ __forceinline__ void modes_lig_pass(const ModesLaunch& L, const Modes
 	}
 }
 
-/* The Result_6D_Modes record from the ligand pass's sums and the two passes'
- * receptor-mode gradients (warp-summed, receptor pass first): warp sums,
- * correctModeForce (delta += 4 k delta^4, src/model/reduction_modes.h:101-115),
- * ForceLim, TorqueMat.  Lane k (k < 27) returns float k of the record. */
+/* The Result_6D_Modes record from the pose's sums (energy, force, torque
+ * matrix; gR and gL the modes' gradients): correctModeForce (delta += 4 k
+ * delta^4, src/model/reduction_modes.h:101-115), ForceLim, TorqueMat.  Lane k
+ * (k < 27) returns float k of the record. */
 template <int MM>
-__device__ __forceinline__ float modes_epilogue(const ModesLaunch& L, const ModesFrame& F, PoseSums& S,
-		const CoopSums& C, float gL[MM], const float gR_rec[MM], float gR_nl[MM], const int lane) {
+__device__ __forceinline__ float modes_record(const ModesLaunch& L, const PoseRot& R, float sE, float sFx, float sFy,
+		float sFz, const float T[9], float gL[MM], float gR[MM], const int lane) {
 	const uint32_t Mr = L.rec.n_modes, Ml = L.lig.n_modes;
-	fold_coop(C, S, lane);
-	float sE = warp_sum(S.E), sFx = warp_sum(S.Fx), sFy = warp_sum(S.Fy), sFz = warp_sum(S.Fz);
-	float T[9];
-#pragma unroll
-	for (int k = 0; k < 9; ++k) T[k] = warp_sum(S.T[k]);
-	float gR[MM];
-#pragma unroll
-	for (int m = 0; m < MM; ++m) {
-		gR[m] = 0.f;
-		if (m < (int)Mr) gR[m] = fadd(gR_rec[m], warp_sum(gR_nl[m]));
-		if (m < (int)Ml) gL[m] = warp_sum(gL[m]);
-	}
 	force_lim(sFx, sFy, sFz);
 	float ang[3];
-	torque_reduce(F.R, T, ang);
+	torque_reduce(R, T, ang);
 	/* correctModeForce: delta += (float)(4 k * delta^4) */
 #pragma unroll
 	for (int m = 0; m < MM; ++m) {
@@ -430,6 +461,27 @@ __device__ __forceinline__ float modes_epilogue(const ModesLaunch& L, const Mode
 	return v;
 }
 
+/* modes_record from the ligand pass's lane sums and the two passes'
+ * receptor-mode gradients (the receptor pass's warp-summed, added first). */
+template <int MM>
+__device__ __forceinline__ float modes_epilogue(const ModesLaunch& L, const ModesFrame& F, PoseSums& S,
+		const CoopSums& C, float gL[MM], const float gR_rec[MM], float gR_nl[MM], const int lane) {
+	const uint32_t Mr = L.rec.n_modes, Ml = L.lig.n_modes;
+	fold_coop(C, S, lane);
+	const float sE = warp_sum(S.E), sFx = warp_sum(S.Fx), sFy = warp_sum(S.Fy), sFz = warp_sum(S.Fz);
+	float T[9];
+#pragma unroll
+	for (int k = 0; k < 9; ++k) T[k] = warp_sum(S.T[k]);
+	float gR[MM];
+#pragma unroll
+	for (int m = 0; m < MM; ++m) {
+		gR[m] = 0.f;
+		if (m < (int)Mr) gR[m] = fadd(gR_rec[m], warp_sum(gR_nl[m]));
+		if (m < (int)Ml) gL[m] = warp_sum(gL[m]);
+	}
+	return modes_record<MM>(L, F.R, sE, sFx, sFy, sFz, T, gL, gR, lane);
+}
+
 /* Warp sums of the receptor pass's mode gradients (every lane). */
 template <int MM>
 __device__ __forceinline__ void sum_rec_modes(uint32_t Mr, float gR[MM]) {
@@ -458,6 +510,254 @@ __device__ __forceinline__ float eval_pose_modes(const ModesLaunch& L, const flo
 	CoopSums C;
 	modes_lig_pass<MM>(L, F, ampR, ampL, lane, W, MS, S, C, gL, gRn);
 	return modes_epilogue<MM>(L, F, S, C, gL, gRr, gRn, lane);
+}
+
+/* ---- a pose split over the warps of a block ---------------------------------
+ *
+ * One warp's evaluation is a chain of rounds (777/333 beads, 7 modes each: 13
+ * receptor and 6 ligand rounds, 112 + 135 us for a warp by itself), and every
+ * sum is a chain too: each lane adds its terms in round order, which the
+ * results' bits rest on.  The terms are independent, though, and most of the
+ * work.  A team takes as many rounds at a time as it has warps: warp t stages
+ * round t, drains its lookups and computes its pairs, leaving each lane's
+ * term (a lookup's finished component; a pair's force, energy, slot and
+ * receptor bead) in shared memory; then the sums are continued over the
+ * rounds in order, each by one warp -- the receptor modes dealt over all
+ * warps, and of the ligand pass energy, force and torque, the reactions on
+ * the receptor modes, and the ligand modes by up to three.  Where a round has
+ * more pairs than a warp's buffer holds (a clash), all warps compute pairs of
+ * one round at a time.  Bit for bit eval_pose_modes on octet grids. */
+constexpr int kModesMaxTeam = 8;
+constexpr int kTeamHalves = 4;      /* half-windows (32 pairs) of a round held at once */
+
+template <int MM>
+struct ModesTeamWarp {
+	WarpStage W;
+	ModeStage<MM> MS;
+	float f[2 * kBeadsPerRound / 8][32];     /* component of the lane's lookup in block b */
+	float4 pv[kTeamHalves][32];              /* force and energy of the lane's pair */
+	uint32_t pj[kTeamHalves][32];            /* receptor bead | slot << 24 | 1 << 31; 0: no pair */
+	uint32_t start[kBeadsPerRound], len[kBeadsPerRound];   /* the round's flattened pairs by slot */
+};
+
+template <int MM>
+struct ModesTeamShared {
+	float gRr[MM], gRn[MM], gL[MM];          /* warp sums of the modes' gradients */
+	uint32_t n_look[kModesMaxTeam];
+	uint32_t halves[kModesMaxTeam];
+	float dof[26];
+	int stop;
+	unsigned long long pose;
+};
+
+/* The lane's lookup of block b (eight lookups), if there is one. */
+__device__ __forceinline__ uint32_t coop_lookup_index(uint32_t b, int lane) {
+	return 8 * b + 4 * (lane & 1) + (lane >> 3);
+}
+
+/* Drains the round's lookups into f. */
+template <int MM>
+__device__ __forceinline__ void team_lookups(const DevGrid& G, ModesTeamWarp<MM>& T, uint32_t n_look, int lane) {
+	for (uint32_t k0 = 0; k0 < n_look; k0 += 16) {
+		CoopStep<2> st;
+		st.load(G, T.W, k0, n_look, lane);
+#pragma unroll
+		for (int b = 0; b < 2; ++b) T.f[k0 / 8 + b][lane] = fmul(st.component(b, lane), st.sc[b]);
+	}
+}
+
+/* The pairs of half-windows [h0, h0 + kTeamHalves) of the round staged in R
+ * into the buffer of T (this warp's). */
+template <int MM>
+__device__ __forceinline__ void team_pairs(const ModesLaunch& L, const float ampR[MM], const ModesTeamWarp<MM>& R,
+		ModesTeamWarp<MM>& T, uint32_t h0, int lane) {
+	const uint32_t start[2] = {R.start[lane], R.start[lane + 32]}, len[2] = {R.len[lane], R.len[lane + 32]};
+	const uint32_t n_pair = __reduce_max_sync(GBA_FULL_MASK, max(len[0] ? start[0] + len[0] : 0u, len[1] ? start[1] + len[1] : 0u));
+	if (32 * h0 >= n_pair) return;
+	PairWindow win;
+	if (h0 > 0) {
+		/* the bead that covers the pair before the first window */
+		const uint32_t q = 32 * h0 - 1;
+		uint32_t slot = 0;
+#pragma unroll
+		for (int h = 0; h < 2; ++h)
+			if (q >= start[h] && q - start[h] < len[h]) slot = 1u + lane + 32 * h;
+		win.carry = __reduce_max_sync(GBA_FULL_MASK, slot) - 1u;
+	}
+	for (uint32_t hw = 0; hw < kTeamHalves && 32 * (h0 + hw) < n_pair; hw += 2) {
+		const uint32_t w = 32 * (h0 + hw);
+		uint32_t so[2];
+		win.owners(T.W, w, start, len, lane, so[0], so[1]);
+#pragma unroll
+		for (int h = 0; h < 2; ++h) {
+			const uint32_t q = w + 32 * h + lane;
+			uint32_t pj = 0;
+			if (q < n_pair) {
+				uint32_t j;
+				float vw[4 * kModeWords<MM>], fx, fy, fz, e;
+				if (modes_pair<MM>(L, ampR, R.W, so[h], R.W.lbase[so[h]] + q, j, vw, fx, fy, fz, e)) {
+					T.pv[hw + h][lane] = make_float4(fx, fy, fz, e);
+					pj = j | so[h] << 24 | 0x80000000u;
+				}
+			}
+			T.pj[hw + h][lane] = pj;
+		}
+	}
+}
+
+/* One pose by a block of G warps; every warp calls it with the pose's record
+ * in dv (lane k: float k).  Warp 0's lane k (k < 27) returns float k of the
+ * result. */
+template <int MM>
+__device__ __forceinline__ float eval_pose_modes_team(const ModesLaunch& L, const float dv, const int lane, const int t,
+		const int G, ModesTeamWarp<MM>* team, ModesTeamShared<MM>& sh) {
+	const uint32_t Mr = L.rec.n_modes, Ml = L.lig.n_modes;
+	const int comp = coop_component(lane);
+	ModesTeamWarp<MM>& me = team[t];
+	float ampR[MM], ampL[MM];
+	const ModesFrame F = modes_frame<MM>(dv, lane, ampR, ampL, L.trig);
+	uint32_t mine = 0;      /* the receptor modes this warp sums over the receptor pass */
+	for (int m = t; m < (int)Mr; m += G) mine |= 1u << m;
+
+	/* receptor pass */
+	{
+		const uint32_t rounds = (L.rec.n + kBeadsPerRound - 1) / kBeadsPerRound;
+		float gR[MM];
+#pragma unroll
+		for (int m = 0; m < MM; ++m) gR[m] = 0.f;
+		for (uint32_t r0 = 0; r0 < rounds; r0 += G) {
+			uint32_t n_look = 0;
+			if (r0 + t < rounds) {
+				n_look = modes_rec_stage<MM>(L, F, ampR, (r0 + t) * kBeadsPerRound, lane, me.W, me.MS);
+				team_lookups<MM>(L.grid_lig, me, n_look, lane);
+			}
+			if (lane == 0) sh.n_look[t] = n_look;
+			__syncthreads();
+			for (int u = 0; u < G; ++u) {
+				const uint32_t nl = sh.n_look[u];
+				for (uint32_t b = 0; 8 * b < nl; ++b) {
+					const uint32_t k = coop_lookup_index(b, lane);
+					if (k < nl && comp < 3) {
+						const uint32_t s = lookup_slot(team[u].W, k);
+						const float f = team[u].f[b][lane];
+#pragma unroll
+						for (int m = 0; m < MM; ++m)
+							if (mine >> m & 1u) gR[m] = ffma(-f, team[u].MS.w[s][comp][m], gR[m]);
+					}
+				}
+			}
+			__syncthreads();
+		}
+#pragma unroll
+		for (int m = 0; m < MM; ++m)
+			if (mine >> m & 1u) {
+				const float v = warp_sum(gR[m]);
+				if (lane == 0) sh.gRr[m] = v;
+			}
+	}
+
+	/* ligand pass: energy, force, torque on warp 0; reactions; ligand modes */
+	const bool do_nl = t == 1 % G, do_lig = t == 2 % G;
+	const uint32_t rounds = (L.lig.n + kBeadsPerRound - 1) / kBeadsPerRound;
+	PoseSums S;
+	CoopSums C;
+	float gRn[MM], gL[MM];
+#pragma unroll
+	for (int m = 0; m < MM; ++m) {
+		gRn[m] = 0.f;
+		gL[m] = 0.f;
+	}
+	for (uint32_t r0 = 0; r0 < rounds; r0 += G) {
+		uint32_t n_look = 0, n_pair = 0, nln[2] = {0, 0}, start[2] = {0, 0};
+		if (r0 + t < rounds) {
+			n_look = modes_lig_stage<MM>(L, F, ampL, (r0 + t) * kBeadsPerRound, lane, me.W, me.MS, nln, start, n_pair);
+			team_lookups<MM>(L.grid_rec, me, n_look, lane);
+		}
+#pragma unroll
+		for (int h = 0; h < 2; ++h) {
+			me.start[lane + 32 * h] = start[h];
+			me.len[lane + 32 * h] = nln[h];
+		}
+		if (lane == 0) {
+			sh.n_look[t] = n_look;
+			sh.halves[t] = (n_pair + 31) / 32;
+		}
+		__syncthreads();
+		uint32_t most = 0;
+		for (int u = 0; u < G; ++u) most = max(most, sh.halves[u]);
+		const bool apart = most <= kTeamHalves;      /* every warp holds its own round's pairs */
+		if (apart) {
+			team_pairs<MM>(L, ampR, me, me, 0, lane);
+			__syncthreads();
+		}
+		for (int u = 0; u < G; ++u) {
+			const ModesTeamWarp<MM>& you = team[u];
+			const uint32_t nl = sh.n_look[u], nh = sh.halves[u];
+			if (t == 0 || do_lig)
+				for (uint32_t b = 0; 8 * b < nl; ++b) {
+					const uint32_t k = coop_lookup_index(b, lane);
+					if (k < nl) {
+						const uint32_t s = lookup_slot(you.W, k);
+						const float f = you.f[b][lane];
+						if (t == 0) coop_add(you.W, s, comp, f, C);
+						if (do_lig && comp != 3) project_component<MM>(you.MS, s, comp, Ml, f, gL);
+					}
+				}
+			for (uint32_t h0 = 0; h0 < nh; h0 += kTeamHalves) {
+				const uint32_t part = h0 / kTeamHalves % G;
+				if (!apart && part == 0) {
+					__syncthreads();      /* the buffers have been read */
+					team_pairs<MM>(L, ampR, you, me, h0 + t * kTeamHalves, lane);
+					__syncthreads();
+				}
+				if (!(t == 0 || do_nl || do_lig)) continue;
+				const ModesTeamWarp<MM>& held = apart ? you : team[part];
+				const uint32_t n = min(nh - h0, (uint32_t)kTeamHalves);
+				for (uint32_t h = 0; h < n; ++h) {
+					const uint32_t pj = held.pj[h][lane];
+					if (!pj) continue;
+					const float4 v = held.pv[h][lane];
+					const uint32_t s = pj >> 24 & 0x7fu;
+					if (t == 0) {
+						const float4 x = you.W.ut[s];
+						S.add(v.w, v.x, v.y, v.z, x.x, x.y, x.z);
+					}
+					if (do_nl) {
+						float vw[4 * kModeWords<MM>];
+						load_modes<MM>(L.rec_modes + (size_t)(pj & 0xffffffu) * L.rec_ms, Mr, vw);
+						project_reaction<MM>(vw, Mr, v.x, v.y, v.z, gRn);
+					}
+					if (do_lig) project_staged<MM>(you.MS, s, Ml, v.x, v.y, v.z, -1.f, gL);
+				}
+			}
+		}
+		__syncthreads();
+	}
+#pragma unroll
+	for (int m = 0; m < MM; ++m) {
+		if (do_nl && m < (int)Mr) {
+			const float v = warp_sum(gRn[m]);
+			if (lane == 0) sh.gRn[m] = v;
+		}
+		if (do_lig && m < (int)Ml) {
+			const float v = warp_sum(gL[m]);
+			if (lane == 0) sh.gL[m] = v;
+		}
+	}
+	__syncthreads();
+	if (t != 0) return 0.f;
+	fold_coop(C, S, lane);
+	const float sE = warp_sum(S.E), sFx = warp_sum(S.Fx), sFy = warp_sum(S.Fy), sFz = warp_sum(S.Fz);
+	float T[9];
+#pragma unroll
+	for (int k = 0; k < 9; ++k) T[k] = warp_sum(S.T[k]);
+	float gRt[MM], gLt[MM];
+#pragma unroll
+	for (int m = 0; m < MM; ++m) {
+		gRt[m] = m < (int)Mr ? fadd(sh.gRr[m], sh.gRn[m]) : 0.f;
+		gLt[m] = m < (int)Ml ? sh.gL[m] : 0.f;
+	}
+	return modes_record<MM>(L, F.R, sE, sFx, sFy, sFz, T, gLt, gRt, lane);
 }
 
 /* ---- the reference CPU path's order (GBA_KOPT_REFERENCE_ORDER) ----------
@@ -782,6 +1082,19 @@ __global__ void __launch_bounds__(kModesThreads, 2) modes_lig_kernel(const Modes
 	}
 }
 
+/* Few poses: a block of warps each (eval_pose_modes_team). */
+template <int MM>
+__global__ void __launch_bounds__(32 * kModesMaxTeam, 2) modes_team_kernel(const ModesLaunch L) {
+	ModesTeamWarp<MM>* team = reinterpret_cast<ModesTeamWarp<MM>*>(modes_dyn_smem);
+	const int lane = threadIdx.x & 31, t = threadIdx.x >> 5, G = blockDim.x >> 5;
+	ModesTeamShared<MM>& sh = *reinterpret_cast<ModesTeamShared<MM>*>(team + G);
+	for (size_t p = blockIdx.x; p < L.n; p += gridDim.x) {
+		const float dv = lane < 26 ? __ldg(reinterpret_cast<const float*>(L.dofs + p) + lane) : 0.f;
+		const float v = eval_pose_modes_team<MM>(L, dv, lane, t, G, team, sh);
+		if (t == 0 && lane < 27) reinterpret_cast<float*>(L.out + p)[lane] = v;
+	}
+}
+
 /* GBA_KOPT_REFERENCE_ORDER scoring: a warp takes whole poses
  * (eval_pose_modes_ref) with its own receptor array in L.ref_rf. */
 template <int MM>
@@ -806,6 +1119,29 @@ __device__ __forceinline__ unsigned long long modes_global_ns() {
 	unsigned long long t;
 	asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
 	return t;
+}
+
+/* The record's float that element j of the machine's point belongs to is
+ * found from either side: the element behind float k (or -1), and the result
+ * entry behind gradient element j (1-based; neg: its sign turns). */
+__device__ __forceinline__ int modes_point_element(int k, int Mr, int Ml) {
+	if (k < 3) return 3 + k;
+	if (k < 6) return k - 3;
+	if (k < 6 + Mr) return k;
+	if (k >= 16 && k < 16 + Ml) return k - 10 + Mr;
+	return -1;
+}
+/* -(ang), -(pos), then the mode entries, which are gradients already
+ * (reduceModeForce) */
+__device__ __forceinline__ int modes_gradient_entry(int j, int Mr, int jn, bool& neg) {
+	neg = false;
+	const int k = j - 1;
+	if (j < 1 || j > jn) return 0;
+	if (k < 6) {
+		neg = true;
+		return k < 3 ? 4 + k : k - 2;
+	}
+	return k < 6 + Mr ? 7 + (k - 6) : 17 + (k - 6 - Mr);
 }
 
 template <int MM, bool REF>
@@ -858,11 +1194,7 @@ __global__ void __launch_bounds__(kModesMinThreads) minimize_modes_kernel(const 
 			/* lane j converts element j of the point (one FP64 instruction for
 			 * all); lane k takes float k of the record from its lane */
 			const float pf = lane < jn ? (float)va.point()[lane] : 0.f;
-			int from = -1;
-			if (lane < 3) from = 3 + lane;
-			else if (lane < 6) from = lane - 3;
-			else if (lane < 6 + (int)Mr) from = lane;
-			else if (lane >= 16 && lane < 16 + (int)Ml) from = lane - 10 + (int)Mr;
+			const int from = modes_point_element(lane, (int)Mr, (int)Ml);
 			const float xf = __shfl_sync(GBA_FULL_MASK, pf, max(from, 0));
 			dv = from >= 0 ? xf : 0.f;
 			if (REF)
@@ -872,17 +1204,9 @@ __global__ void __launch_bounds__(kModesMinThreads) minimize_modes_kernel(const 
 				v = eval_pose_modes<MM>(L, dv, lane, stage[wib], ms[wib]);
 			++nev;
 			/* lane j takes gradient element j from the lane holding its entry
-			 * of the result record: -(ang), -(pos), then the mode entries,
-			 * which are gradients already (reduceModeForce) */
-			const int k = lane - 1;
-			int src = 0;
-			bool neg = false;
-			if (lane >= 1 && lane <= jn) {
-				if (k < 3) { src = 4 + k; neg = true; }
-				else if (k < 6) { src = k - 2; neg = true; }
-				else if (k < 6 + (int)Mr) src = 7 + (k - 6);
-				else src = 17 + (k - 6 - (int)Mr);
-			}
+			 * of the result record */
+			bool neg;
+			const int src = modes_gradient_entry(lane, (int)Mr, jn, neg);
 			const float gv = __shfl_sync(GBA_FULL_MASK, v, src);
 			const double gl = (double)(neg ? -gv : gv);
 			const float e = __shfl_sync(GBA_FULL_MASK, v, 0);
@@ -905,6 +1229,81 @@ __global__ void __launch_bounds__(kModesMinThreads) minimize_modes_kernel(const 
 	}
 }
 
+/* The same with a block of warps per pose (eval_pose_modes_team), warp 0
+ * stepping its VA13: for jobs whose poses all get a block of their own. */
+template <int MM>
+__global__ void __launch_bounds__(32 * kModesMaxTeam, 2) minimize_modes_team_kernel(const ModesMinLaunch M) {
+	ModesTeamWarp<MM>* team = reinterpret_cast<ModesTeamWarp<MM>*>(modes_dyn_smem);
+	const int lane = threadIdx.x & 31, t = threadIdx.x >> 5, G = blockDim.x >> 5;
+	ModesTeamShared<MM>& sh = *reinterpret_cast<ModesTeamShared<MM>*>(team + G);
+	VA13<6 + 2 * MM>& va = *reinterpret_cast<VA13<6 + 2 * MM>*>(&sh + 1);
+	const ModesLaunch& L = M.m;
+	const int Mr = (int)L.rec.n_modes, Ml = (int)L.lig.n_modes, jn = 6 + Mr + Ml;
+	const unsigned long long t_start = modes_global_ns();
+	for (;;) {
+		if (threadIdx.x == 0) {
+			unsigned long long slot = atomicAdd(M.counter, 1ull);
+			if (slot < M.n && modes_global_ns() - t_start > kMinimizeHardCapNs) {
+				atomicExch(M.status, GBA_ERR_TIMEOUT);
+				slot = ~0ull;
+			}
+			sh.pose = slot;
+			if (slot < M.n) {
+				double x0[6 + 2 * MM];
+				const float* s = reinterpret_cast<const float*>(M.start + slot);
+				for (int k = 0; k < 3; ++k) { x0[k] = s[3 + k]; x0[3 + k] = s[k]; }
+				for (int m = 0; m < Mr; ++m) x0[6 + m] = s[6 + m];
+				for (int m = 0; m < Ml; ++m) x0[6 + Mr + m] = s[16 + m];
+				va.start(x0, jn, M.max_evals);
+			}
+		}
+		__syncthreads();
+		const size_t p = (size_t)sh.pose;
+		if (p >= M.n) break;
+		int nev = 0;
+		for (;;) {
+			if (t == 0) {
+				const float pf = lane < jn ? (float)va.point()[lane] : 0.f;
+				const int from = modes_point_element(lane, Mr, Ml);
+				const float xf = __shfl_sync(GBA_FULL_MASK, pf, max(from, 0));
+				if (lane < 26) sh.dof[lane] = from >= 0 ? xf : 0.f;
+			}
+			__syncthreads();
+			const float dv = lane < 26 ? sh.dof[lane] : 0.f;
+			const float v = eval_pose_modes_team<MM>(L, dv, lane, t, G, team, sh);
+			++nev;
+			if (t == 0) {
+				bool neg;
+				const int src = modes_gradient_entry(lane, Mr, jn, neg);
+				const float gv = __shfl_sync(GBA_FULL_MASK, v, src);
+				const double gl = (double)(neg ? -gv : gv);
+				const float e = __shfl_sync(GBA_FULL_MASK, v, 0);
+				va.provide_w((double)e, [&](int) { return gl; }, VaWarp{lane});
+				if (lane == 0) {
+					int stop = va.done();
+					if (!stop && nev > M.max_evals + 1) {
+						atomicExch(M.status, GBA_ERR_DEVICE_CHECK);
+						stop = 1;
+					}
+					if (!stop && (nev & 15) == 0 && modes_global_ns() - t_start > kMinimizeHardCapNs) {
+						atomicExch(M.status, GBA_ERR_TIMEOUT);
+						stop = 1;
+					}
+					sh.stop = stop;
+				}
+				__syncwarp();
+				if (sh.stop) {
+					if (lane < 27) reinterpret_cast<float*>(M.out_result + p)[lane] = v;
+					if (lane < 26) reinterpret_cast<float*>(M.out_state + p)[lane] = dv;
+					if (lane == 0 && M.out_nevals) M.out_nevals[p] = nev;
+				}
+			}
+			__syncthreads();
+			if (sh.stop) break;
+		}
+	}
+}
+
 namespace {
 
 template <int MM>
@@ -912,22 +1311,71 @@ size_t mode_stage_bytes(int threads) {
 	return (size_t)(threads / 32) * sizeof(ModeStage<MM>);
 }
 
-/* dynamic shared memory beyond the 48 KB default needs the opt-in */
+/* Resident blocks per SM (0: the kernel does not fit), with the opt-in to
+ * dynamic shared memory beyond the 48 KB default; queried once per device,
+ * kernel, block size and shared memory (the queries cost a small call more
+ * host time than its launches).  The opt-in only grows: launches of other
+ * sizes may be in flight. */
 template <class K>
-cudaError_t allow_smem(K kernel, size_t dyn) {
-	return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+int blocks_that_fit(K kernel, int threads, size_t dyn) {
+	static std::mutex mu;
+	static std::map<std::array<size_t, 4>, int> known;
+	static std::map<std::pair<size_t, size_t>, size_t> opted;
+	int dev = 0;
+	if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+	std::lock_guard<std::mutex> g(mu);
+	const std::array<size_t, 4> key{(size_t)dev, (size_t)kernel, (size_t)threads, dyn};
+	const auto it = known.find(key);
+	if (it != known.end()) return it->second;
+	size_t& most = opted[{(size_t)dev, (size_t)kernel}];
+	int nb = 0;
+	if (dyn <= most || cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) == cudaSuccess) {
+		most = std::max(most, dyn);
+		if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, dyn) != cudaSuccess) nb = 0;
+	}
+	cudaGetLastError();      /* a size that does not fit is an answer */
+	if (known.size() >= 256) known.clear();
+	return known[key] = nb;
 }
 
 template <class K>
 int resident_blocks(K kernel, int threads, size_t dyn) {
-	if (allow_smem(kernel, dyn) != cudaSuccess) return 1;
-	int nb = 0;
-	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, dyn);
-	return nb > 0 ? nb : 1;
+	return std::max(1, blocks_that_fit(kernel, threads, dyn));
+}
+
+/* shared memory of a team of G warps; the minimizer's VA13 state follows */
+template <int MM>
+size_t team_bytes(int G, bool minimize) {
+	static_assert(sizeof(ModesTeamWarp<MM>) % 16 == 0 && sizeof(ModesTeamShared<MM>) % 8 == 0, "laid out in a row");
+	return (size_t)G * sizeof(ModesTeamWarp<MM>) + sizeof(ModesTeamShared<MM>) +
+			(minimize ? sizeof(VA13<6 + 2 * MM>) : 0);
+}
+
+/* Warps per pose for n poses: the largest team with which every pose has a
+ * resident block of its own, or 0 (a pose then takes a warp by itself).  The
+ * terms' records hold 24 bits of a receptor bead's index and come from
+ * cooperative lookups.  Measured, a warp per pose against teams: scoring
+ * 777/333 beads, 7 modes, 100 poses 210 -> 73 us; 1500/600, 5 modes, 500 poses
+ * 317 -> 157, 1,000 poses 307 -> 205, and 1,200 poses, not all resident in
+ * teams of two, 308 against 370; minimizing 700/300, 5 modes, 50 evaluations
+ * 100 poses 16.6 -> 6.4 ms, 500 12.7 -> 7.0, 800 13.4 -> 10.2. */
+template <int MM, class K>
+int team_size(K kernel, bool minimize, const ModesLaunch& L, size_t n, int num_sms) {
+	if (!L.grid_rec.coop_lookup || !L.grid_lig.coop_lookup || L.rec.n > (1u << 24)) return 0;
+	const uint32_t rounds = std::max((L.rec.n + 63) / 64, (L.lig.n + 63) / 64);
+	if (n > (size_t)num_sms * 8) return 0;       /* 16 warps of 128 registers, two at least to a team */
+	for (int G = (int)std::min<uint32_t>(kModesMaxTeam, rounds); G >= 2; --G)
+		if (n <= (size_t)num_sms * blocks_that_fit(kernel, 32 * G, team_bytes<MM>(G, minimize))) return G;
+	return 0;
 }
 
 template <int MM>
 cudaError_t launch_modes_mm(const ModesLaunch& L, int num_sms, cudaStream_t s) {
+	const int team = team_size<MM>(modes_team_kernel<MM>, false, L, L.n, num_sms);
+	if (team > 0) {
+		modes_team_kernel<MM><<<(unsigned)L.n, 32 * team, team_bytes<MM>(team, false), s>>>(L);
+		return cudaGetLastError();
+	}
 	const size_t dyn_r = mode_stage_bytes<MM>(kModesRecThreads);
 	const size_t want_r = (L.n + kModesRecThreads / 32 - 1) / (kModesRecThreads / 32);
 	const size_t br = std::max<size_t>(1, std::min<size_t>(want_r,
@@ -964,20 +1412,23 @@ size_t min_modes_bytes(int threads) {
 
 template <int MM, bool REF>
 cudaError_t launch_min_mm(const ModesMinLaunch& M, int blocks, int threads, cudaStream_t s) {
+	if (!REF) {
+		const int team = team_size<MM>(minimize_modes_team_kernel<MM>, true, M.m, M.n, M.num_sms);
+		if (team > 0) {
+			const size_t dyn = team_bytes<MM>(team, true);
+			minimize_modes_team_kernel<MM><<<(unsigned)M.n, 32 * team, dyn, s>>>(M);
+			return cudaGetLastError();
+		}
+	}
 	const size_t dyn = min_modes_bytes<MM>(threads);
-	cudaError_t e = allow_smem(minimize_modes_kernel<MM, REF>, dyn);
-	if (e != cudaSuccess) return e;
+	resident_blocks(minimize_modes_kernel<MM, REF>, threads, dyn);      /* the opt-in */
 	minimize_modes_kernel<MM, REF><<<blocks, threads, dyn, s>>>(M);
 	return cudaGetLastError();
 }
 
 template <int MM, bool REF>
 int min_bps_mm(int threads) {
-	const size_t dyn = min_modes_bytes<MM>(threads);
-	if (allow_smem(minimize_modes_kernel<MM, REF>, dyn) != cudaSuccess) return 1;
-	int nb = 0;
-	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, minimize_modes_kernel<MM, REF>, threads, dyn);
-	return nb > 0 ? nb : 1;
+	return resident_blocks(minimize_modes_kernel<MM, REF>, threads, min_modes_bytes<MM>(threads));
 }
 
 }  // namespace

@@ -238,8 +238,11 @@ struct ModesMinLaunch {
 	int max_evals;
 	unsigned long long* counter;    /* zeroed before launch */
 	int* status;                    /* GBA_OK, set to TIMEOUT / DEVICE_CHECK by the kernel */
+	int num_sms;
 };
 
+/* blocks, threads: of the form with a warp per pose; small jobs take a block
+ * of warps per pose instead (the same results bit for bit) */
 cudaError_t launch_minimize_modes(const ModesMinLaunch& M, int blocks, int threads, cudaStream_t s);
 int minimize_modes_blocks_per_sm(int threads, const ModesLaunch& L);
 

@@ -632,6 +632,7 @@ int gba_minimize_6d_modes(gba_ctx* ctx, gba_id rec, gba_id lig, gba_id grid_rec,
 	const bool dev = is_device_pointer(start) && is_device_pointer(out_state) &&
 			is_device_pointer(out_result) && (!out_nevals || is_device_pointer(out_nevals));
 	M.n = n;
+	M.num_sms = ctx->num_sms;
 	M.max_evals = max_evals;
 	if (dev) {
 		M.start = start;
