@@ -50,6 +50,9 @@ namespace gba {
 
 namespace {
 
+/* The grid layout a pass is compiled for. */
+constexpr int kNative = 0, kOctets = 1, kAnyLayout = 2;
+
 /* Floats of a bead's mode record held in registers (mode_stride(MM)). */
 template <int MM>
 constexpr int kModeWords = (3 * MM + 3) / 4;
@@ -107,6 +110,34 @@ __device__ __forceinline__ void project(const float* __restrict__ v, uint32_t M,
 template <int MM>
 struct ModeStage {
 	float w[kBeadsPerRound][3][MM];
+	/* the pose: R [0, 9), its sin/cos [9, 15), R(-ang) [15, 24), t' [24, 27),
+	 * t [27, 30), then the receptor's and the ligand's amplitudes.  Kept here
+	 * rather than in registers (31 to 50 of them), read back where a round or
+	 * its pairs need some. */
+	float pose[(30 + 2 * MM + 3) & ~3];
+};
+
+/* What the receptor pass stages of a round: charges, lookups, weights and (for
+ * the native layout) bead indices, in the fields the lookups expect of a
+ * WarpStage, without its pairs and torque. */
+struct RecStage {
+	float cw[kBeadsPerRound * kCornerStride];
+	uint2 look[2 * kBeadsPerRound];
+	float q[kBeadsPerRound];
+	uint32_t j[kBeadsPerRound];
+	__device__ __forceinline__ float charge(uint32_t s) const { return q[s]; }
+	__device__ __forceinline__ void put_rec(int s, float charge, uint32_t bead) {
+		q[s] = charge;
+		j[s] = bead;
+	}
+	__device__ __forceinline__ uint32_t bead(uint32_t s) const { return j[s]; }
+};
+/* The same of a whole WarpStage. */
+struct FullStage : WarpStage {
+	__device__ __forceinline__ void put_rec(int s, float charge, uint32_t bead) {
+		put_bead(*this, s, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, charge, bead);
+	}
+	__device__ __forceinline__ uint32_t bead(uint32_t s) const { return __float_as_uint(ut[s].w); }
 };
 
 /* Rotated mode vectors of slot s: w_m = R v_m (transpose = false) or R^T v_m,
@@ -201,13 +232,54 @@ __device__ __forceinline__ ModesFrame modes_frame(const float dv, const int lane
 	return F;
 }
 
+/* The pose frame and amplitudes of record dv, parked in the warp's staging. */
+template <int MM>
+__device__ __forceinline__ void put_frame(const ModesLaunch& L, const float dv, const int lane, ModeStage<MM>& MS) {
+	float ampR[MM], ampL[MM];
+	const ModesFrame F = modes_frame<MM>(dv, lane, ampR, ampL, L.trig);
+	if (lane == 0) {
+		float* v = MS.pose;
+#pragma unroll
+		for (int k = 0; k < 9; ++k) {
+			v[k] = F.R.m[k];
+			v[15 + k] = F.Ri[k];
+		}
+		v[9] = F.R.cphi; v[10] = F.R.sphi; v[11] = F.R.cssi; v[12] = F.R.sssi; v[13] = F.R.crot; v[14] = F.R.srot;
+#pragma unroll
+		for (int k = 0; k < 3; ++k) {
+			v[24 + k] = F.ip[k];
+			v[27 + k] = F.t[k];
+		}
+#pragma unroll
+		for (int m = 0; m < MM; ++m) {
+			v[30 + m] = ampR[m];
+			v[30 + MM + m] = ampL[m];
+		}
+	}
+	__syncwarp();
+}
+
+/* N parked floats from `at`; volatile, so that the compiler does not keep
+ * them in registers from one use to the next. */
+template <int N, int MM>
+__device__ __forceinline__ void get_frame(const ModeStage<MM>& MS, int at, float (&out)[N]) {
+	const volatile float* v = MS.pose + at;
+#pragma unroll
+	for (int k = 0; k < N; ++k) out[k] = v[k];
+}
+
 /* Stages 64 receptor beads from j0: deformed, moved into the ligand frame,
  * their lookups in the LIGAND grid queued, their mode vectors rotated for the
  * cooperative lookups.  Returns the number of lookups. */
-template <int MM>
-__device__ __forceinline__ uint32_t modes_rec_stage(const ModesLaunch& L, const ModesFrame& F, const float ampR[MM],
-		const uint32_t j0, const int lane, WarpStage& W, ModeStage<MM>& MS) {
+template <int MM, class Stage>
+__device__ __forceinline__ uint32_t modes_rec_stage(const ModesLaunch& L, const uint32_t j0, const int lane, Stage& W,
+		ModeStage<MM>& MS) {
 	const uint32_t Mr = L.rec.n_modes;
+	float Rm[9], Ri[9], ip[3], ampR[MM];
+	get_frame(MS, 0, Rm);
+	get_frame(MS, 15, Ri);
+	get_frame(MS, 24, ip);
+	get_frame(MS, 30, ampR);
 	uint32_t nlk[2];
 	BeadGrid bg[2];
 #pragma unroll
@@ -224,15 +296,15 @@ __device__ __forceinline__ uint32_t modes_rec_stage(const ModesLaunch& L, const 
 			float x = r.x, y = r.y, z = r.z;
 			deform_w<MM>(vw, Mr, ampR, x, y, z);
 			float px, py, pz;
-			rot_apply(F.Ri, x, y, z, px, py, pz);
-			px = fadd(px, F.ip[0]); py = fadd(py, F.ip[1]); pz = fadd(pz, F.ip[2]);
-			put_bead(W, s, 0.f, 0.f, 0.f, px, py, pz, r.w, j);
+			rot_apply(Ri, x, y, z, px, py, pz);
+			px = fadd(px, ip[0]); py = fadd(py, ip[1]); pz = fadd(pz, ip[2]);
+			W.put_rec(s, r.w, j);
 			nlk[h] = stage_grid(L.grid_lig, px, py, pz, mapped, r.w, s, W, bg[h]);
 			/* the ligand-frame force f is rotated back by R before the
 			 * projection: (R f) . v = f . (R^T v); staged for the
 			 * cooperative lookups only (one lookup per bead or two: the
 			 * per-lane form rotates f instead) */
-			if (nlk[h] && L.grid_lig.coop_lookup) stage_modes<MM>(MS, s, vw, Mr, F.R.m, true);
+			if (nlk[h] && L.grid_lig.coop_lookup) stage_modes<MM>(MS, s, vw, Mr, Rm, true);
 		}
 	}
 	const uint32_t n_look = queue_lookups(W, nlk, bg, lane);
@@ -243,14 +315,14 @@ __device__ __forceinline__ uint32_t modes_rec_stage(const ModesLaunch& L, const 
 /* Receptor pass: the receptor beads, deformed and moved into the ligand
  * frame, in the LIGAND grid; each force rotated back by R and projected on
  * the receptor modes into the lane sums gR. */
-template <int MM>
-__device__ __forceinline__ void modes_rec_pass(const ModesLaunch& L, const ModesFrame& F, const float ampR[MM],
-		const int lane, WarpStage& W, ModeStage<MM>& MS, float gR[MM]) {
+template <int MM, int LAYOUT = kAnyLayout, class Stage>
+__device__ __forceinline__ void modes_rec_pass(const ModesLaunch& L, const int lane, Stage& W, ModeStage<MM>& MS,
+		float gR[MM]) {
 	const uint32_t Mr = L.rec.n_modes;
 	const int comp = coop_component(lane);
 	for (uint32_t j0 = 0; j0 < L.rec.n; j0 += kBeadsPerRound) {
-		const uint32_t n_look = modes_rec_stage<MM>(L, F, ampR, j0, lane, W, MS);
-		if (L.grid_lig.coop_lookup) {
+		const uint32_t n_look = modes_rec_stage<MM>(L, j0, lane, W, MS);
+		if (LAYOUT == kAnyLayout ? L.grid_lig.coop_lookup != 0 : LAYOUT == kOctets) {
 			for (uint32_t k0 = 0; k0 < n_look; k0 += 16) {
 				CoopStep<2> st;
 				st.load(L.grid_lig, W, k0, n_look, lane);
@@ -261,13 +333,15 @@ __device__ __forceinline__ void modes_rec_pass(const ModesLaunch& L, const Modes
 				}
 			}
 		} else {
+			float Rm[9];
+			get_frame(MS, 0, Rm);
 			for (uint32_t q = lane; q < n_look; q += 32) {
 				const uint32_t s = lookup_slot(W, q);
 				const float4 v = grid_lookup(L.grid_lig, W, q);
 				/* back into the receptor frame, then -(force . mode) */
 				float fx, fy, fz;
-				rot_apply(F.R.m, v.x, v.y, v.z, fx, fy, fz);
-				project<MM>(L.rec_modes + (size_t)__float_as_uint(W.ut[s].w) * L.rec_ms, Mr, fx, fy, fz, -1.f, gR);
+				rot_apply(Rm, v.x, v.y, v.z, fx, fy, fz);
+				project<MM>(L.rec_modes + (size_t)W.bead(s) * L.rec_ms, Mr, fx, fy, fz, -1.f, gR);
 			}
 		}
 		__syncwarp();
@@ -279,10 +353,13 @@ __device__ __forceinline__ void modes_rec_pass(const ModesLaunch& L, const Modes
  * lookups and neighbour lists queued, mode vectors rotated.  Returns the
  * number of lookups; n_pair, nln, start as queue_pairs has them. */
 template <int MM>
-__device__ __forceinline__ uint32_t modes_lig_stage(const ModesLaunch& L, const ModesFrame& F, const float ampL[MM],
-		const uint32_t i0, const int lane, WarpStage& W, ModeStage<MM>& MS, uint32_t nln[2], uint32_t start[2],
-		uint32_t& n_pair) {
+__device__ __forceinline__ uint32_t modes_lig_stage(const ModesLaunch& L, const uint32_t i0, const int lane,
+		WarpStage& W, ModeStage<MM>& MS, uint32_t nln[2], uint32_t start[2], uint32_t& n_pair) {
 	const uint32_t Ml = L.lig.n_modes;
+	float Rm[9], tr[3], ampL[MM];
+	get_frame(MS, 0, Rm);
+	get_frame(MS, 27, tr);
+	get_frame(MS, 30 + MM, ampL);
 	uint32_t nlk[2];
 	BeadGrid bg[2];
 #pragma unroll
@@ -301,15 +378,15 @@ __device__ __forceinline__ uint32_t modes_lig_stage(const ModesLaunch& L, const 
 			float x = b.x, y = b.y, z = b.z;
 			deform_w<MM>(vw, Ml, ampL, x, y, z);
 			float px, py, pz;
-			rot_apply(F.R.m, x, y, z, px, py, pz);
-			px = fadd(px, F.t[0]); py = fadd(py, F.t[1]); pz = fadd(pz, F.t[2]);
+			rot_apply(Rm, x, y, z, px, py, pz);
+			px = fadd(px, tr[0]); py = fadd(py, tr[1]); pz = fadd(pz, tr[2]);
 			put_bead(W, s, b.x, b.y, b.z, px, py, pz, b.w, type);
 			nlk[h] = stage_grid(L.grid_rec, px, py, pz, mapped, b.w, s, W, bg[h]);
 			bool in_nl;
 			if (type != 0) nln[h] = stage_nl(L.grid_rec.nl, px, py, pz, s, W, in_nl);
 			/* the global-frame force f is projected in the ligand frame:
 			 * (R^T f) . v = f . (R v) */
-			if (nlk[h] | nln[h]) stage_modes<MM>(MS, s, vw, Ml, F.R.m, false);
+			if (nlk[h] | nln[h]) stage_modes<MM>(MS, s, vw, Ml, Rm, false);
 		}
 	}
 	const uint32_t n_look = queue_lookups(W, nlk, bg, lane);
@@ -363,16 +440,15 @@ __device__ __forceinline__ void coop_add(const WarpStage& W, uint32_t s, int com
  * in the receptor grid, plus the NL pairs against the deformed receptor:
  * energy, force and torque into S and C, ligand mode projections into gL,
  * the pairs' reaction forces projected on the receptor modes into gR. */
-template <int MM>
-__device__ __forceinline__ void modes_lig_pass(const ModesLaunch& L, const ModesFrame& F, const float ampR[MM],
-		const float ampL[MM], const int lane, WarpStage& W, ModeStage<MM>& MS, PoseSums& S, CoopSums& C,
-		float gL[MM], float gR[MM]) {
+template <int MM, int LAYOUT = kAnyLayout>
+__device__ __forceinline__ void modes_lig_pass(const ModesLaunch& L, const int lane, WarpStage& W, ModeStage<MM>& MS,
+		PoseSums& S, CoopSums& C, float gL[MM], float gR[MM]) {
 	const uint32_t Mr = L.rec.n_modes, Ml = L.lig.n_modes;
 	const int comp = coop_component(lane);
 	for (uint32_t i0 = 0; i0 < L.lig.n; i0 += kBeadsPerRound) {
 		uint32_t nln[2], start[2], n_pair;
-		const uint32_t n_look = modes_lig_stage<MM>(L, F, ampL, i0, lane, W, MS, nln, start, n_pair);
-		if (L.grid_rec.coop_lookup) {
+		const uint32_t n_look = modes_lig_stage<MM>(L, i0, lane, W, MS, nln, start, n_pair);
+		if (LAYOUT == kAnyLayout ? L.grid_rec.coop_lookup != 0 : LAYOUT == kOctets) {
 			for (uint32_t k0 = 0; k0 < n_look; k0 += 16) {
 				CoopStep<2> st;
 				st.load(L.grid_rec, W, k0, n_look, lane);
@@ -397,6 +473,8 @@ __device__ __forceinline__ void modes_lig_pass(const ModesLaunch& L, const Modes
 		}
 		/* neighbour pairs after the lookups: measured faster here (the rigid
 		 * kernel measured the opposite) */
+		float ampR[MM];
+		get_frame(MS, 30, ampR);
 		PairWindow win;
 		for (uint32_t w = 0; w < n_pair; w += 64) {
 			uint32_t so[2];
@@ -461,10 +539,20 @@ __device__ __forceinline__ float modes_record(const ModesLaunch& L, const PoseRo
 	return v;
 }
 
+template <int MM>
+__device__ __forceinline__ PoseRot frame_rotation(const ModeStage<MM>& MS) {
+	PoseRot R;
+	float c[6];
+	get_frame(MS, 0, R.m);
+	get_frame(MS, 9, c);
+	R.cphi = c[0]; R.sphi = c[1]; R.cssi = c[2]; R.sssi = c[3]; R.crot = c[4]; R.srot = c[5];
+	return R;
+}
+
 /* modes_record from the ligand pass's lane sums and the two passes'
  * receptor-mode gradients (the receptor pass's warp-summed, added first). */
 template <int MM>
-__device__ __forceinline__ float modes_epilogue(const ModesLaunch& L, const ModesFrame& F, PoseSums& S,
+__device__ __forceinline__ float modes_epilogue(const ModesLaunch& L, const ModeStage<MM>& MS, PoseSums& S,
 		const CoopSums& C, float gL[MM], const float gR_rec[MM], float gR_nl[MM], const int lane) {
 	const uint32_t Mr = L.rec.n_modes, Ml = L.lig.n_modes;
 	fold_coop(C, S, lane);
@@ -479,7 +567,7 @@ __device__ __forceinline__ float modes_epilogue(const ModesLaunch& L, const Mode
 		if (m < (int)Mr) gR[m] = fadd(gR_rec[m], warp_sum(gR_nl[m]));
 		if (m < (int)Ml) gL[m] = warp_sum(gL[m]);
 	}
-	return modes_record<MM>(L, F.R, sE, sFx, sFy, sFz, T, gL, gR, lane);
+	return modes_record<MM>(L, frame_rotation(MS), sE, sFx, sFy, sFz, T, gL, gR, lane);
 }
 
 /* Warp sums of the receptor pass's mode gradients (every lane). */
@@ -496,20 +584,19 @@ __device__ __forceinline__ void sum_rec_modes(uint32_t Mr, float gR[MM]) {
  * Only the model fields of L are read.  MM >= the receptor's and the
  * ligand's mode counts.  Bit for bit the result of the split scoring
  * kernels (modes_rec_kernel then modes_lig_kernel). */
-template <int MM>
+template <int MM, int LAYOUT>
 __device__ __forceinline__ float eval_pose_modes(const ModesLaunch& L, const float dv, const int lane,
-		WarpStage& W, ModeStage<MM>& MS) {
-	float ampR[MM], ampL[MM];
-	const ModesFrame F = modes_frame<MM>(dv, lane, ampR, ampL, L.trig);
+		FullStage& W, ModeStage<MM>& MS) {
+	put_frame<MM>(L, dv, lane, MS);
 	float gRr[MM], gRn[MM], gL[MM];
 #pragma unroll
 	for (int m = 0; m < MM; ++m) { gRr[m] = 0.f; gRn[m] = 0.f; gL[m] = 0.f; }
-	modes_rec_pass<MM>(L, F, ampR, lane, W, MS, gRr);
+	modes_rec_pass<MM, LAYOUT>(L, lane, W, MS, gRr);
 	sum_rec_modes<MM>(L.rec.n_modes, gRr);
 	PoseSums S;
 	CoopSums C;
-	modes_lig_pass<MM>(L, F, ampR, ampL, lane, W, MS, S, C, gL, gRn);
-	return modes_epilogue<MM>(L, F, S, C, gL, gRr, gRn, lane);
+	modes_lig_pass<MM, LAYOUT>(L, lane, W, MS, S, C, gL, gRn);
+	return modes_epilogue<MM>(L, MS, S, C, gL, gRr, gRn, lane);
 }
 
 /* ---- a pose split over the warps of a block ---------------------------------
@@ -532,7 +619,7 @@ constexpr int kTeamHalves = 4;      /* half-windows (32 pairs) of a round held a
 
 template <int MM>
 struct ModesTeamWarp {
-	WarpStage W;
+	FullStage W;
 	ModeStage<MM> MS;
 	float f[2 * kBeadsPerRound / 8][32];     /* component of the lane's lookup in block b */
 	float4 pv[kTeamHalves][32];              /* force and energy of the lane's pair */
@@ -569,8 +656,10 @@ __device__ __forceinline__ void team_lookups(const DevGrid& G, ModesTeamWarp<MM>
 /* The pairs of half-windows [h0, h0 + kTeamHalves) of the round staged in R
  * into the buffer of T (this warp's). */
 template <int MM>
-__device__ __forceinline__ void team_pairs(const ModesLaunch& L, const float ampR[MM], const ModesTeamWarp<MM>& R,
+__device__ __forceinline__ void team_pairs(const ModesLaunch& L, const ModesTeamWarp<MM>& R,
 		ModesTeamWarp<MM>& T, uint32_t h0, int lane) {
+	float ampR[MM];
+	get_frame(T.MS, 30, ampR);
 	const uint32_t start[2] = {R.start[lane], R.start[lane + 32]}, len[2] = {R.len[lane], R.len[lane + 32]};
 	const uint32_t n_pair = __reduce_max_sync(GBA_FULL_MASK, max(len[0] ? start[0] + len[0] : 0u, len[1] ? start[1] + len[1] : 0u));
 	if (32 * h0 >= n_pair) return;
@@ -614,8 +703,7 @@ __device__ __forceinline__ float eval_pose_modes_team(const ModesLaunch& L, cons
 	const uint32_t Mr = L.rec.n_modes, Ml = L.lig.n_modes;
 	const int comp = coop_component(lane);
 	ModesTeamWarp<MM>& me = team[t];
-	float ampR[MM], ampL[MM];
-	const ModesFrame F = modes_frame<MM>(dv, lane, ampR, ampL, L.trig);
+	put_frame<MM>(L, dv, lane, me.MS);
 	uint32_t mine = 0;      /* the receptor modes this warp sums over the receptor pass */
 	for (int m = t; m < (int)Mr; m += G) mine |= 1u << m;
 
@@ -628,7 +716,7 @@ __device__ __forceinline__ float eval_pose_modes_team(const ModesLaunch& L, cons
 		for (uint32_t r0 = 0; r0 < rounds; r0 += G) {
 			uint32_t n_look = 0;
 			if (r0 + t < rounds) {
-				n_look = modes_rec_stage<MM>(L, F, ampR, (r0 + t) * kBeadsPerRound, lane, me.W, me.MS);
+				n_look = modes_rec_stage<MM>(L, (r0 + t) * kBeadsPerRound, lane, me.W, me.MS);
 				team_lookups<MM>(L.grid_lig, me, n_look, lane);
 			}
 			if (lane == 0) sh.n_look[t] = n_look;
@@ -670,7 +758,7 @@ __device__ __forceinline__ float eval_pose_modes_team(const ModesLaunch& L, cons
 	for (uint32_t r0 = 0; r0 < rounds; r0 += G) {
 		uint32_t n_look = 0, n_pair = 0, nln[2] = {0, 0}, start[2] = {0, 0};
 		if (r0 + t < rounds) {
-			n_look = modes_lig_stage<MM>(L, F, ampL, (r0 + t) * kBeadsPerRound, lane, me.W, me.MS, nln, start, n_pair);
+			n_look = modes_lig_stage<MM>(L, (r0 + t) * kBeadsPerRound, lane, me.W, me.MS, nln, start, n_pair);
 			team_lookups<MM>(L.grid_rec, me, n_look, lane);
 		}
 #pragma unroll
@@ -687,7 +775,7 @@ __device__ __forceinline__ float eval_pose_modes_team(const ModesLaunch& L, cons
 		for (int u = 0; u < G; ++u) most = max(most, sh.halves[u]);
 		const bool apart = most <= kTeamHalves;      /* every warp holds its own round's pairs */
 		if (apart) {
-			team_pairs<MM>(L, ampR, me, me, 0, lane);
+			team_pairs<MM>(L, me, me, 0, lane);
 			__syncthreads();
 		}
 		for (int u = 0; u < G; ++u) {
@@ -707,7 +795,7 @@ __device__ __forceinline__ float eval_pose_modes_team(const ModesLaunch& L, cons
 				const uint32_t part = h0 / kTeamHalves % G;
 				if (!apart && part == 0) {
 					__syncthreads();      /* the buffers have been read */
-					team_pairs<MM>(L, ampR, you, me, h0 + t * kTeamHalves, lane);
+					team_pairs<MM>(L, you, me, h0 + t * kTeamHalves, lane);
 					__syncthreads();
 				}
 				if (!(t == 0 || do_nl || do_lig)) continue;
@@ -757,7 +845,7 @@ __device__ __forceinline__ float eval_pose_modes_team(const ModesLaunch& L, cons
 		gRt[m] = m < (int)Mr ? fadd(sh.gRr[m], sh.gRn[m]) : 0.f;
 		gLt[m] = m < (int)Ml ? sh.gL[m] : 0.f;
 	}
-	return modes_record<MM>(L, F.R, sE, sFx, sFy, sFz, T, gLt, gRt, lane);
+	return modes_record<MM>(L, frame_rotation(me.MS), sE, sFx, sFy, sFz, T, gLt, gRt, lane);
 }
 
 /* ---- the reference CPU path's order (GBA_KOPT_REFERENCE_ORDER) ----------
@@ -1010,9 +1098,17 @@ __device__ __forceinline__ float eval_pose_modes_ref(const ModesLaunch& L, const
 
 namespace {
 
-constexpr int kModesThreads = 256;       /* ligand-pass scoring kernel's block */
-constexpr int kModesRecThreads = 128;    /* receptor-pass kernel: block, */
-constexpr int kModesRecBlocks = 5;       /* resident blocks per SM (shared memory allows five) */
+/* Scoring kernels' blocks and how many of them the registers are bounded for:
+ * latency bounds both passes, so warps count for more than registers until
+ * the compiler spills, which it does at five modes and octets above six
+ * receptor and five ligand blocks (20,000 poses, 1500/600 beads: 2,285 us at
+ * 5 and 4, 2,107 at 6 and 5, 2,159 at 6 and 6; ten modes 644 at 5 and 4, 697 at
+ * 6 and 5; native grids 187 against 268). */
+constexpr int kModesThreads = 128;
+template <int MM, int LAYOUT>
+constexpr int kModesRecBlocks = MM <= 5 && LAYOUT == kOctets ? 6 : 5;
+template <int MM, int LAYOUT>
+constexpr int kModesLigBlocks = MM <= 5 && LAYOUT == kOctets ? 5 : 4;
 constexpr int kModesMinThreads = 128;    /* minimizer kernel block */
 constexpr int kModesRefThreads = 128;    /* reference-order scoring kernel block */
 
@@ -1029,9 +1125,9 @@ extern __shared__ float4 modes_dyn_smem[];
  * registers allow: the receptor pass (most of the grid lookups) parks its
  * warp-summed receptor-mode gradients in the result record's modesRec slots;
  * the ligand pass reads them back, adds its own and writes the record. */
-template <int MM>
-__global__ void __launch_bounds__(kModesRecThreads, kModesRecBlocks) modes_rec_kernel(const ModesLaunch L) {
-	__shared__ WarpStage stage[kModesRecThreads / 32];
+template <int MM, int LAYOUT>
+__global__ void __launch_bounds__(kModesThreads, kModesRecBlocks<MM, LAYOUT>) modes_rec_kernel(const ModesLaunch L) {
+	__shared__ RecStage stage[kModesThreads / 32];
 	ModeStage<MM>* ms = reinterpret_cast<ModeStage<MM>*>(modes_dyn_smem);
 	const int lane = threadIdx.x & 31;
 	const int wib = threadIdx.x >> 5;
@@ -1039,13 +1135,13 @@ __global__ void __launch_bounds__(kModesRecThreads, kModesRecBlocks) modes_rec_k
 	for (size_t p = next_pose(L.next, lane); p < L.n; p = next_pose(L.next, lane)) {
 		const float* d = reinterpret_cast<const float*>(L.dofs + p);
 		const float dv = lane < 26 ? __ldg(d + lane) : 0.f;
-		float ampR[MM], ampL[MM];
-		const ModesFrame F = modes_frame<MM>(dv, lane, ampR, ampL, L.trig);
+		put_frame<MM>(L, dv, lane, ms[wib]);
 		float gR[MM];
 #pragma unroll
 		for (int m = 0; m < MM; ++m) gR[m] = 0.f;
-		modes_rec_pass<MM>(L, F, ampR, lane, stage[wib], ms[wib], gR);
+		modes_rec_pass<MM, LAYOUT>(L, lane, stage[wib], ms[wib], gR);
 		sum_rec_modes<MM>(Mr, gR);
+		__syncwarp();
 		float v = 0.f;
 #pragma unroll
 		for (int m = 0; m < MM; ++m) v = lane == m ? gR[m] : v;
@@ -1053,8 +1149,8 @@ __global__ void __launch_bounds__(kModesRecThreads, kModesRecBlocks) modes_rec_k
 	}
 }
 
-template <int MM>
-__global__ void __launch_bounds__(kModesThreads, 2) modes_lig_kernel(const ModesLaunch L) {
+template <int MM, int LAYOUT>
+__global__ void __launch_bounds__(kModesThreads, kModesLigBlocks<MM, LAYOUT>) modes_lig_kernel(const ModesLaunch L) {
 	__shared__ WarpStage stage[kModesThreads / 32];
 	ModeStage<MM>* ms = reinterpret_cast<ModeStage<MM>*>(modes_dyn_smem);
 	const int lane = threadIdx.x & 31;
@@ -1063,8 +1159,7 @@ __global__ void __launch_bounds__(kModesThreads, 2) modes_lig_kernel(const Modes
 	for (size_t p = next_pose(L.next2, lane); p < L.n; p = next_pose(L.next2, lane)) {
 		const float* d = reinterpret_cast<const float*>(L.dofs + p);
 		const float dv = lane < 26 ? __ldg(d + lane) : 0.f;
-		float ampR[MM], ampL[MM];
-		const ModesFrame F = modes_frame<MM>(dv, lane, ampR, ampL, L.trig);
+		put_frame<MM>(L, dv, lane, ms[wib]);
 		float gRr[MM], gRn[MM], gL[MM];
 		const float* o = reinterpret_cast<const float*>(L.out + p);
 #pragma unroll
@@ -1076,8 +1171,9 @@ __global__ void __launch_bounds__(kModesThreads, 2) modes_lig_kernel(const Modes
 		__syncwarp();
 		PoseSums S;
 		CoopSums C;
-		modes_lig_pass<MM>(L, F, ampR, ampL, lane, stage[wib], ms[wib], S, C, gL, gRn);
-		const float v = modes_epilogue<MM>(L, F, S, C, gL, gRr, gRn, lane);
+		modes_lig_pass<MM, LAYOUT>(L, lane, stage[wib], ms[wib], S, C, gL, gRn);
+		const float v = modes_epilogue<MM>(L, ms[wib], S, C, gL, gRr, gRn, lane);
+		__syncwarp();
 		if (lane < 27) reinterpret_cast<float*>(L.out + p)[lane] = v;
 	}
 }
@@ -1144,9 +1240,12 @@ __device__ __forceinline__ int modes_gradient_entry(int j, int Mr, int jn, bool&
 	return k < 6 + Mr ? 7 + (k - 6) : 17 + (k - 6 - Mr);
 }
 
-template <int MM, bool REF>
+/* LAYOUT: compiled for octets where both grids have them, which leaves the
+ * native lookups' code out (6,000 poses, 700/300 beads, 20 evaluations: 17.6 ->
+ * 16.9 ms). */
+template <int MM, bool REF, int LAYOUT>
 __global__ void __launch_bounds__(kModesMinThreads) minimize_modes_kernel(const ModesMinLaunch M) {
-	__shared__ WarpStage stage[kModesMinThreads / 32];
+	__shared__ FullStage stage[kModesMinThreads / 32];
 	ModeStage<MM>* ms = reinterpret_cast<ModeStage<MM>*>(modes_dyn_smem);
 	/* per warp, after the mode staging areas: its pose's VA13 state, which
 	 * every lane of the warp steps (the warp form) */
@@ -1201,7 +1300,7 @@ __global__ void __launch_bounds__(kModesMinThreads) minimize_modes_kernel(const 
 				v = eval_pose_modes_ref<MM>(L, dv, lane, stage[wib], *reinterpret_cast<RefModesExtra*>(&ms[wib]),
 						L.ref_rf + (((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * L.rec.n);
 			else
-				v = eval_pose_modes<MM>(L, dv, lane, stage[wib], ms[wib]);
+				v = eval_pose_modes<MM, LAYOUT>(L, dv, lane, stage[wib], ms[wib]);
 			++nev;
 			/* lane j takes gradient element j from the lane holding its entry
 			 * of the result record */
@@ -1376,18 +1475,22 @@ cudaError_t launch_modes_mm(const ModesLaunch& L, int num_sms, cudaStream_t s) {
 		modes_team_kernel<MM><<<(unsigned)L.n, 32 * team, team_bytes<MM>(team, false), s>>>(L);
 		return cudaGetLastError();
 	}
-	const size_t dyn_r = mode_stage_bytes<MM>(kModesRecThreads);
-	const size_t want_r = (L.n + kModesRecThreads / 32 - 1) / (kModesRecThreads / 32);
-	const size_t br = std::max<size_t>(1, std::min<size_t>(want_r,
-			(size_t)num_sms * resident_blocks(modes_rec_kernel<MM>, kModesRecThreads, dyn_r)));
-	modes_rec_kernel<MM><<<(unsigned)br, kModesRecThreads, dyn_r, s>>>(L);
+	/* each pass by its own grid's layout */
+	const size_t dyn = mode_stage_bytes<MM>(kModesThreads), warps = kModesThreads / 32;
+	auto blocks = [&](auto kernel) {
+		return (unsigned)std::max<size_t>(1, std::min<size_t>((L.n + warps - 1) / warps,
+				(size_t)num_sms * resident_blocks(kernel, kModesThreads, dyn)));
+	};
+	if (L.grid_lig.coop_lookup)
+		modes_rec_kernel<MM, kOctets><<<blocks(modes_rec_kernel<MM, kOctets>), kModesThreads, dyn, s>>>(L);
+	else
+		modes_rec_kernel<MM, kNative><<<blocks(modes_rec_kernel<MM, kNative>), kModesThreads, dyn, s>>>(L);
 	cudaError_t e = cudaGetLastError();
 	if (e != cudaSuccess) return e;
-	const size_t dyn = mode_stage_bytes<MM>(kModesThreads);
-	const size_t want = (L.n + kModesThreads / 32 - 1) / (kModesThreads / 32);
-	const size_t bl = std::max<size_t>(1, std::min<size_t>(want,
-			(size_t)num_sms * resident_blocks(modes_lig_kernel<MM>, kModesThreads, dyn)));
-	modes_lig_kernel<MM><<<(unsigned)bl, kModesThreads, dyn, s>>>(L);
+	if (L.grid_rec.coop_lookup)
+		modes_lig_kernel<MM, kOctets><<<blocks(modes_lig_kernel<MM, kOctets>), kModesThreads, dyn, s>>>(L);
+	else
+		modes_lig_kernel<MM, kNative><<<blocks(modes_lig_kernel<MM, kNative>), kModesThreads, dyn, s>>>(L);
 	return cudaGetLastError();
 }
 
@@ -1421,14 +1524,23 @@ cudaError_t launch_min_mm(const ModesMinLaunch& M, int blocks, int threads, cuda
 		}
 	}
 	const size_t dyn = min_modes_bytes<MM>(threads);
-	resident_blocks(minimize_modes_kernel<MM, REF>, threads, dyn);      /* the opt-in */
-	minimize_modes_kernel<MM, REF><<<blocks, threads, dyn, s>>>(M);
+	/* resident_blocks: the opt-in to the shared memory */
+	if (!REF && M.m.grid_rec.coop_lookup && M.m.grid_lig.coop_lookup) {
+		resident_blocks(minimize_modes_kernel<MM, false, kOctets>, threads, dyn);
+		minimize_modes_kernel<MM, false, kOctets><<<blocks, threads, dyn, s>>>(M);
+	} else {
+		resident_blocks(minimize_modes_kernel<MM, REF, kAnyLayout>, threads, dyn);
+		minimize_modes_kernel<MM, REF, kAnyLayout><<<blocks, threads, dyn, s>>>(M);
+	}
 	return cudaGetLastError();
 }
 
 template <int MM, bool REF>
-int min_bps_mm(int threads) {
-	return resident_blocks(minimize_modes_kernel<MM, REF>, threads, min_modes_bytes<MM>(threads));
+int min_bps_mm(int threads, const ModesLaunch& L) {
+	const size_t dyn = min_modes_bytes<MM>(threads);
+	return !REF && L.grid_rec.coop_lookup && L.grid_lig.coop_lookup
+			? resident_blocks(minimize_modes_kernel<MM, false, kOctets>, threads, dyn)
+			: resident_blocks(minimize_modes_kernel<MM, REF, kAnyLayout>, threads, dyn);
 }
 
 }  // namespace
@@ -1459,8 +1571,8 @@ cudaError_t launch_minimize_modes(const ModesMinLaunch& M, int blocks, int threa
 
 int minimize_modes_blocks_per_sm(int threads, const ModesLaunch& L) {
 	if (L.ref_order)
-		return mode_capacity(L) == 5 ? min_bps_mm<5, true>(threads) : min_bps_mm<GBA_MODES_MAX, true>(threads);
-	return mode_capacity(L) == 5 ? min_bps_mm<5, false>(threads) : min_bps_mm<GBA_MODES_MAX, false>(threads);
+		return mode_capacity(L) == 5 ? min_bps_mm<5, true>(threads, L) : min_bps_mm<GBA_MODES_MAX, true>(threads, L);
+	return mode_capacity(L) == 5 ? min_bps_mm<5, false>(threads, L) : min_bps_mm<GBA_MODES_MAX, false>(threads, L);
 }
 
 }  // namespace gba

@@ -62,6 +62,7 @@ struct WarpStage {
 	 * comes from the loads in flight */
 	float tot[16];
 	unsigned long long slot;           /* the pose's index, for the same reason */
+	__device__ __forceinline__ float charge(uint32_t s) const { return pq[s].w; }
 };
 
 /* Stores the pose rotation and translation in the warp's staging area. */
@@ -150,8 +151,9 @@ struct BeadGrid {
  * (src/model/IntrplGrid.h:96-104,130-163): picks inner or outer grid, stores
  * the eight trilinear corner weights of slot s, sets the element indices and
  * returns the number of lookups (0, 1, or 2 with the charge channel). */
+template <class Stage>
 __device__ __forceinline__ uint32_t stage_grid(const DevGrid& G, float px, float py, float pz,
-		uint32_t mapped, float q, int s, WarpStage& W, BeadGrid& bg) {
+		uint32_t mapped, float q, int s, Stage& W, BeadGrid& bg) {
 	if (mapped == 0) return 0;
 	const bool inner = !grid_out(G.inner, px, py, pz);
 	const bool outer = !inner && !grid_out(G.outer, px, py, pz);
@@ -202,23 +204,26 @@ __device__ __forceinline__ uint32_t stage_nl(const DevNL& nl, float px, float py
 }
 
 /* Bead slot of queued lookup k. */
-__device__ __forceinline__ uint32_t lookup_slot(const WarpStage& W, uint32_t k) { return W.look[k].y & 0x7fu; }
+template <class Stage>
+__device__ __forceinline__ uint32_t lookup_slot(const Stage& W, uint32_t k) { return W.look[k].y & 0x7fu; }
 
 /* Grid, element, slot and scale of queued lookup k: 1/voxelVol, times the
  * bead charge for the charge channel. */
-__device__ __forceinline__ const DevIntrpl& lookup_grid(const DevGrid& G, const WarpStage& W, uint32_t k,
+template <class Stage>
+__device__ __forceinline__ const DevIntrpl& lookup_grid(const DevGrid& G, const Stage& W, uint32_t k,
 		uint32_t& elem, uint32_t& s, float& sc) {
 	const uint2 e = W.look[k];
 	const DevIntrpl& g = (e.x & 0x80000000u) ? G.outer : G.inner;
 	elem = e.x & 0x7fffffffu;
 	s = e.y & 0x7fu;
-	sc = (e.y & 0x80u) ? fmul(g.voxelVol_inv, W.pq[s].w) : g.voxelVol_inv;
+	sc = (e.y & 0x80u) ? fmul(g.voxelVol_inv, W.charge(s)) : g.voxelVol_inv;
 	return g;
 }
 
 /* One queued lookup by one lane: the channel's interpolated (fx, fy, fz, E),
  * scaled. */
-__device__ __forceinline__ float4 grid_lookup(const DevGrid& G, const WarpStage& W, uint32_t k) {
+template <class Stage>
+__device__ __forceinline__ float4 grid_lookup(const DevGrid& G, const Stage& W, uint32_t k) {
 	uint32_t elem, s;
 	float sc;
 	const DevIntrpl& g = lookup_grid(G, W, k, elem, s, sc);
@@ -232,7 +237,8 @@ __device__ __forceinline__ float4 grid_lookup(const DevGrid& G, const WarpStage&
 }
 
 /* Writes the lookup queue entries of slot s (n = 0..2) at position k. */
-__device__ __forceinline__ void enqueue_lookups(WarpStage& W, uint32_t k, int s, uint32_t n, const BeadGrid& bg) {
+template <class Stage>
+__device__ __forceinline__ void enqueue_lookups(Stage& W, uint32_t k, int s, uint32_t n, const BeadGrid& bg) {
 	if (n > 0) W.look[k] = make_uint2(bg.t, (uint32_t)s);
 	if (n > 1) W.look[k + 1] = make_uint2(bg.q, (uint32_t)s | 0x80u);
 }
@@ -241,7 +247,8 @@ __device__ __forceinline__ void enqueue_lookups(WarpStage& W, uint32_t k, int s,
  * bead slot lane, nlk[1] for slot lane + 32): slots 0..31 first, then 32..63,
  * so that neighbouring queue entries belong to neighbouring slots.  Returns
  * the queue length. */
-__device__ __forceinline__ uint32_t queue_lookups(WarpStage& W, const uint32_t nlk[2], const BeadGrid bg[2],
+template <class Stage>
+__device__ __forceinline__ uint32_t queue_lookups(Stage& W, const uint32_t nlk[2], const BeadGrid bg[2],
 		int lane) {
 	const uint32_t incl = warp_incl_scan(nlk[0] | (nlk[1] << 16), lane);
 	const uint32_t tot = __shfl_sync(GBA_FULL_MASK, incl, 31);
@@ -371,7 +378,8 @@ struct CoopStep {
 	bool ok[NB];
 
 	/* block b, lane (g, c): own lookup k0 + 8 b + 4 mine + g, then the partner's */
-	__device__ __forceinline__ void load(const DevGrid& G, const WarpStage& W, uint32_t k0, uint32_t n_look,
+	template <class Stage>
+	__device__ __forceinline__ void load(const DevGrid& G, const Stage& W, uint32_t k0, uint32_t n_look,
 			int lane) {
 		const int grp = lane >> 3, cor = lane & 7, mine = cor & 1;
 #pragma unroll
