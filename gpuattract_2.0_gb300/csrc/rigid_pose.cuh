@@ -17,7 +17,7 @@
  *      of 64 pairs, two per lane (owners from per-window start masks);
  *   3. the warp drains the lookup queue: one lookup per lane (8 gathered
  *      float4 corners), or with the octet layout and GBA_KOPT_COOP_LOOKUP
- *      eight lanes per lookup, one corner each (one 128-byte line per
+ *      four lanes per lookup, two corners each (one 128-byte line per
  *      lookup, sixteen lookups per step, loaded without L1 allocation so
  *      that L1 keeps the receptor and parameter data).  Pairs come first:
  *      measured on GB300, this order is faster.
@@ -358,72 +358,74 @@ struct CoopSums {
 /* Drains the lookup queue of a round.  Per-lane form: one lookup per lane
  * into S.  Cooperative form (octet layout), sixteen lookups per step in two
  * blocks of eight: in block b, lane group g = lane / 8 takes lookups
- * k0 + 8 b + g and k0 + 8 b + 4 + g, lane c = lane % 8 loads octet corner c
- * of both (one 128-byte line per lookup, read without L1 allocation) times
- * its trilinear weight (src/model/trilinIntrpl.h:29-66); all four loads of a
- * lane are issued before the first is used.  A three-step reduce-scatter over
- * the group leaves lane c holding one finished component -- lookup (c & 1),
- * component 2 * ((c >> 1) & 1) + (c >> 2) -- summed in octet_sum's pairwise
- * order, so both forms give the same value per lookup.  Each lane loads its
- * own lookup first, which makes the first step select-free.  The lane scales
- * the component and adds it to its CoopSums role. */
+ * k0 + 8 b + g (its even lanes) and k0 + 8 b + 4 + g (its odd lanes); lane
+ * c = lane % 8 loads the octet's corners 2 (c / 2) and 2 (c / 2) + 1, 32 bytes
+ * in one load (one 128-byte line per lookup, read without L1 allocation),
+ * times their trilinear weights (src/model/trilinIntrpl.h:29-66); the loads
+ * of a step are all issued before the first is used.  A two-step
+ * reduce-scatter over the lookup's four lanes leaves lane c holding one
+ * finished component, 2 * ((c >> 1) & 1) + (c >> 2), summed in octet_sum's
+ * pairwise order, so both forms give the same value per lookup.  The lane
+ * scales the component and adds it to its CoopSums role.  (Eight lanes a
+ * lookup with a 16-byte corner each computed every address twice and took
+ * four more shuffles a block: 4.25 -> 3.75 ms for 100,000 poses of 2000/700
+ * beads.  Four blocks a step instead of two spill: 4.17 ms.) */
 /* One cooperative step of drain_lookups: the loads and the reduce-scatter of
  * lookups k0 .. k0 + 8 NB - 1, kept apart so that other work can run between
  * them. */
 template <int NB>
 struct CoopStep {
-	float c[NB][8];   /* per block b: own lookup x y z w, partner's x y z w */
+	float m[NB][4];   /* per block: x y z w of the lane's two corners, weighted and added */
 	uint32_t sl[NB];
 	float sc[NB];
 	bool ok[NB];
 
-	/* block b, lane (g, c): own lookup k0 + 8 b + 4 mine + g, then the partner's */
+	/* block b, lane (g, c): lookup k0 + 8 b + 4 (c & 1) + g */
 	template <class Stage>
 	__device__ __forceinline__ void load(const DevGrid& G, const Stage& W, uint32_t k0, uint32_t n_look,
 			int lane) {
-		const int grp = lane >> 3, cor = lane & 7, mine = cor & 1;
+		const int pair = lane & 6;      /* the lane's first corner */
+		float d[NB][8];
 #pragma unroll
 		for (int b = 0; b < NB; ++b) {
+			const uint32_t k = k0 + 8 * b + 4 * (lane & 1) + (lane >> 3);
 			sl[b] = 0;
 			sc[b] = 0.f;
-			ok[b] = false;
+			ok[b] = k < n_look;
+			if (ok[b]) {
+				uint32_t elem;
+				const DevIntrpl& g = lookup_grid(G, W, k, elem, sl[b], sc[b]);
+				ldg_no_l1(g.oct + 8 * (size_t)elem + pair, d[b]);
+			} else {
 #pragma unroll
-			for (int h = 0; h < 2; ++h) {
-				const uint32_t k = k0 + 8 * b + 4 * (h ^ mine) + grp;
-				float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
-				float w = 0.f;
-				if (k < n_look) {
-					uint32_t elem, s;
-					float scale;
-					const DevIntrpl& g = lookup_grid(G, W, k, elem, s, scale);
-					d = ldg_no_l1(g.oct + 8 * (size_t)elem + cor);
-					w = W.cw[kCornerStride * s + cor];
-					if (h == 0) { sl[b] = s; sc[b] = scale; ok[b] = true; }
-				}
-				c[b][4 * h] = fmul(d.x, w); c[b][4 * h + 1] = fmul(d.y, w);
-				c[b][4 * h + 2] = fmul(d.z, w); c[b][4 * h + 3] = fmul(d.w, w);
+				for (int j = 0; j < 8; ++j) d[b][j] = 0.f;
 			}
+		}
+#pragma unroll
+		for (int b = 0; b < NB; ++b) {
+			float w0 = 0.f, w1 = 0.f;
+			if (ok[b]) {
+				w0 = W.cw[kCornerStride * sl[b] + pair];
+				w1 = W.cw[kCornerStride * sl[b] + pair + 1];
+			}
+#pragma unroll
+			for (int j = 0; j < 4; ++j) m[b][j] = fadd(fmul(d[b][j], w0), fmul(d[b][4 + j], w1));
 		}
 	}
 
-	/* the reduce-scatter of block b: the lane's finished, unscaled component
-	 * (lane c: lookup c & 1, component 2 * ((c >> 1) & 1) + (c >> 2)) */
+	/* the reduce-scatter of block b: the lane's finished, unscaled component */
 	__device__ __forceinline__ float component(int b, int lane) const {
 		const int cor = lane & 7;
 		const int hi2 = (cor >> 1) & 1, hi4 = cor >> 2;
-		/* step 1 (partner c ^ 1): keep the own lookup */
-		float m4[4];
-#pragma unroll
-		for (int j = 0; j < 4; ++j) m4[j] = fadd(c[b][j], __shfl_xor_sync(GBA_FULL_MASK, c[b][4 + j], 1));
-		/* step 2 (partner c ^ 2): keep components {0,1} or {2,3} */
+		/* partner c ^ 2: keep components {0,1} or {2,3} */
 		float m2[2];
 #pragma unroll
 		for (int j = 0; j < 2; ++j) {
-			const float keep = hi2 ? m4[2 + j] : m4[j];
-			const float send = hi2 ? m4[j] : m4[2 + j];
+			const float keep = hi2 ? m[b][2 + j] : m[b][j];
+			const float send = hi2 ? m[b][j] : m[b][2 + j];
 			m2[j] = fadd(keep, __shfl_xor_sync(GBA_FULL_MASK, send, 2));
 		}
-		/* step 3 (partner c ^ 4): keep one */
+		/* partner c ^ 4: keep one */
 		const float keep = hi4 ? m2[1] : m2[0];
 		const float send = hi4 ? m2[0] : m2[1];
 		return fadd(keep, __shfl_xor_sync(GBA_FULL_MASK, send, 4));
