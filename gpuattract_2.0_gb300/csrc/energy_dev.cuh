@@ -128,6 +128,13 @@ __device__ __forceinline__ bool nl_out(const DevNL& g, float x, float y, float z
 			(z >= g.pos[2]) & (z <= g.maxDim[2]));
 }
 
+/* Read-only 32-byte load; p: 32-byte aligned. */
+__device__ __forceinline__ void ldg_32(const float* p, float (&v)[8]) {
+	asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+			: "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+			: "l"(p));
+}
+
 /* Read-only 32-byte load that does not allocate in L1 (the line still goes
  * through L2): grid corners are streamed, so L1 stays with the receptor and
  * parameter data the pair term re-reads.  p: 32-byte aligned. */

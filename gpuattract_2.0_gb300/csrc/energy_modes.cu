@@ -55,19 +55,21 @@ constexpr int kNative = 0, kOctets = 1, kAnyLayout = 2;
 
 /* Floats of a bead's mode record held in registers (mode_stride(MM)). */
 template <int MM>
-constexpr int kModeWords = (3 * MM + 3) / 4;
+constexpr int kModeWords = (3 * MM + 7) / 8 * 2;
 
-/* The bead's M mode vectors from its 16-byte aligned record v (padded to
- * whole float4s): one 16-byte load per four floats instead of one load per
- * float -- the records of a warp's beads lie apart, so every load is a
- * separate L1 wavefront. */
+/* The bead's M mode vectors from its 32-byte aligned record v (padded to
+ * eights of floats): one 32-byte load per eight floats -- the records of a
+ * warp's beads lie apart, so every load is an L1 wavefront per lane (16-byte
+ * loads: 20,000 poses at 5 modes 1,837 against 1,803 us, 5,000 at 10 modes 598
+ * against 533). */
 template <int MM>
 __device__ __forceinline__ void load_modes(const float* __restrict__ v, uint32_t M, float (&w)[4 * kModeWords<MM>]) {
-	const float4* q = reinterpret_cast<const float4*>(v);
 #pragma unroll
-	for (int k = 0; k < kModeWords<MM>; ++k) {
-		const float4 t = 4 * k < 3 * (int)M ? __ldg(q + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-		w[4 * k] = t.x; w[4 * k + 1] = t.y; w[4 * k + 2] = t.z; w[4 * k + 3] = t.w;
+	for (int k = 0; k < kModeWords<MM>; k += 2) {
+		float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+		if (4 * k < 3 * (int)M) ldg_32(v + 4 * k, t);
+#pragma unroll
+		for (int j = 0; j < 8; ++j) w[4 * k + j] = t[j];
 	}
 }
 
@@ -314,8 +316,11 @@ __device__ __forceinline__ uint32_t modes_rec_stage(const ModesLaunch& L, const 
 
 /* Receptor pass: the receptor beads, deformed and moved into the ligand
  * frame, in the LIGAND grid; each force rotated back by R and projected on
- * the receptor modes into the lane sums gR. */
-template <int MM, int LAYOUT = kAnyLayout, class Stage>
+ * the receptor modes into the lane sums gR.  BLOCKS: lookup blocks in flight
+ * per cooperative step; the scoring kernel has the registers for four (20,000
+ * poses, 1500/600 beads: 1,837 -> 1,765 us), the minimizer's code has not
+ * (15.0 -> 16.0 ms for 6,000 poses). */
+template <int MM, int LAYOUT = kAnyLayout, int BLOCKS = 2, class Stage>
 __device__ __forceinline__ void modes_rec_pass(const ModesLaunch& L, const int lane, Stage& W, ModeStage<MM>& MS,
 		float gR[MM]) {
 	const uint32_t Mr = L.rec.n_modes;
@@ -323,11 +328,11 @@ __device__ __forceinline__ void modes_rec_pass(const ModesLaunch& L, const int l
 	for (uint32_t j0 = 0; j0 < L.rec.n; j0 += kBeadsPerRound) {
 		const uint32_t n_look = modes_rec_stage<MM>(L, j0, lane, W, MS);
 		if (LAYOUT == kAnyLayout ? L.grid_lig.coop_lookup != 0 : LAYOUT == kOctets) {
-			for (uint32_t k0 = 0; k0 < n_look; k0 += 16) {
-				CoopStep<2> st;
+			for (uint32_t k0 = 0; k0 < n_look; k0 += 8 * BLOCKS) {
+				CoopStep<BLOCKS> st;
 				st.load(L.grid_lig, W, k0, n_look, lane);
 #pragma unroll
-				for (int b = 0; b < 2; ++b) {
+				for (int b = 0; b < BLOCKS; ++b) {
 					const float v = st.component(b, lane);
 					if (st.ok[b] && comp < 3) project_component<MM>(MS, st.sl[b], comp, Mr, fmul(v, st.sc[b]), gR);
 				}
@@ -1139,7 +1144,7 @@ __global__ void __launch_bounds__(kModesThreads, kModesRecBlocks<MM, LAYOUT>) mo
 		float gR[MM];
 #pragma unroll
 		for (int m = 0; m < MM; ++m) gR[m] = 0.f;
-		modes_rec_pass<MM, LAYOUT>(L, lane, stage[wib], ms[wib], gR);
+		modes_rec_pass<MM, LAYOUT, 4>(L, lane, stage[wib], ms[wib], gR);
 		sum_rec_modes<MM>(Mr, gR);
 		__syncwarp();
 		float v = 0.f;

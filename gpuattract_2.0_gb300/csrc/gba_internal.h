@@ -32,9 +32,9 @@ struct DevProtein {
 	float mode_force[GBA_MODES_MAX];
 };
 
-/* Floats per bead of a device mode array: 3 per mode, padded to whole
- * float4s so that a bead's vectors load as 16-byte words. */
-constexpr uint32_t mode_stride(uint32_t n_modes) { return (3 * n_modes + 3) & ~3u; }
+/* Floats per bead of a device mode array: 3 per mode, padded to eights so that
+ * a bead's vectors load as 32-byte words. */
+constexpr uint32_t mode_stride(uint32_t n_modes) { return (3 * n_modes + 7) & ~7u; }
 
 struct DevIntrpl {
 	uint32_t dimN[3];
