@@ -60,6 +60,7 @@ struct PairwiseLaunch {
 	uint32_t* order;            /* visiting order (nearest ligands first), or nullptr */
 	RoundSplit split;           /* pose records; totals and done only when split */
 	int by_round;               /* units are 64-bead rounds, else poses */
+	uint32_t copies;            /* backward: of the type pairs' cells in a block, 1 or 2 */
 	double* part;               /* backward: per block, then once for what no TwoFloat holds, the sums of
 	                               every cell (PairCells) */
 };
@@ -309,6 +310,8 @@ template <bool BACKWARD>
 __device__ __forceinline__ void pairwise_round(const PairwiseLaunch& L, const PairCells& cells, uint32_t i0, int lane,
 		float w, PairStage& W, unsigned long long* cell, PoseSums& S) {
 	const bool cdiel = L.dielec == GBA_DIELEC_CONSTANT;
+	/* odd lanes add to the second copy of the type pairs' cells, where there is one */
+	const uint32_t pair_cells = BACKWARD && L.copies > 1 && (lane & 1) ? (cells.count() + 1) & ~1u : 0;
 	uint32_t nln[2];
 	{
 		float tx, ty, tz;
@@ -419,7 +422,7 @@ __device__ __forceinline__ void pairwise_round(const PairwiseLaunch& L, const Pa
 						S.T[6] += u.x * fz; S.T[7] += u.y * fz; S.T[8] += u.z * fz;
 						gqv = L.ffelec * qj * dd;
 						cell_add(cell + cells.qrec() + j, w * (L.ffelec * qi * dd), L.part + cells.qrec() + j);
-						cell_add2(reinterpret_cast<TwoFloat2*>(cell) + tp, w * drc, w * dac, L.part + 2 * tp, L.part + 2 * tp + 1);
+						cell_add2(reinterpret_cast<TwoFloat2*>(cell + pair_cells) + tp, w * drc, w * dac, L.part + 2 * tp, L.part + 2 * tp + 1);
 					}
 				}
 			}
@@ -487,8 +490,11 @@ __global__ void __launch_bounds__(BACKWARD ? kPairwiseThreads : kForwardThreads,
 	PairStage* stage = reinterpret_cast<PairStage*>(pairwise_smem);
 	unsigned long long* cell = reinterpret_cast<unsigned long long*>(stage + (blockDim.x >> 5));
 	const PairCells cells{L.T * L.T, L.lig.n, L.rec.n};
+	/* a second copy of the type pairs' cells lies behind the rest, an even
+	 * number of cells from the first */
+	const uint32_t second = (cells.count() + 1) & ~1u, spare = L.copies > 1 ? 2 * cells.T2 : 0;
 	if (BACKWARD) {
-		for (uint32_t k = threadIdx.x; k < cells.count(); k += blockDim.x) cell[k] = 0;
+		for (uint32_t k = threadIdx.x; k < second + spare; k += blockDim.x) cell[k] = 0;
 		__syncthreads();
 	}
 	const int lane = threadIdx.x & 31;
@@ -534,7 +540,12 @@ __global__ void __launch_bounds__(BACKWARD ? kPairwiseThreads : kForwardThreads,
 		double* out = L.part + (size_t)(1 + blockIdx.x) * cells.count();
 		for (uint32_t k = threadIdx.x; k < cells.count(); k += blockDim.x) {
 			const unsigned long long c = cell[k];
-			out[k] = (double)__uint_as_float((uint32_t)c) + (double)__uint_as_float((uint32_t)(c >> 32));
+			double v = (double)__uint_as_float((uint32_t)c) + (double)__uint_as_float((uint32_t)(c >> 32));
+			if (k < spare) {
+				const unsigned long long d = cell[second + k];
+				v += (double)__uint_as_float((uint32_t)d) + (double)__uint_as_float((uint32_t)(d >> 32));
+			}
+			out[k] = v;
 		}
 	}
 }
@@ -695,7 +706,15 @@ extern "C" int gba_pairwise_6d(gba_ctx* ctx, gba_id rec, gba_id lig, gba_id grid
 		const size_t rounds = (L.lig.n + kBeadsPerRound - 1) / kBeadsPerRound;
 		const int threads = !backward ? kForwardThreads
 				: cell_bytes + kPairwiseThreads / 32 * sizeof(PairStage) <= kPairwiseSmem ? kPairwiseThreads : 256;
-		const size_t warps = threads / 32, smem = cell_bytes + warps * sizeof(PairStage);
+		const size_t warps = threads / 32;
+		/* a second copy of the type pairs' cells where two blocks still fit an
+		 * SM: half as many lanes meet in a cell.  2000/700 beads, 32 types, forward
+		 * and backward, one copy against two: 10,000 poses 901 -> 876 us, 30,000
+		 * 2,312 -> 2,218; 500/200, 30,000 poses: 887 -> 825. */
+		const size_t two_copies = (cell_bytes + 15) / 16 * 16 + (size_t)2 * L.T * L.T * sizeof(unsigned long long);
+		L.copies = backward && threads == kPairwiseThreads &&
+				2 * (two_copies + warps * sizeof(PairStage) + 1024) <= kPairwiseSmem ? 2 : 1;
+		const size_t smem = (L.copies > 1 ? two_copies : (cell_bytes + 15) / 16 * 16) + warps * sizeof(PairStage);
 		const void* kernel = backward ? (const void*)pairwise_kernel<true> : (const void*)pairwise_kernel<false>;
 		const size_t resident = (size_t)ctx->num_sms * pairwise_blocks_per_sm(kernel, backward, threads, smem);
 		L.by_round = rounds > 1 && n <= (backward ? kBackwardPosesPerWarp : kForwardPosesPerWarp) * resident * warps &&

@@ -78,6 +78,26 @@ def test_large_type_table(pkg):
         assert np.abs(a - b).max() <= 1e-9 * np.abs(a).max()
 
 
+@pytest.mark.parametrize("T", [46, 47])
+def test_copies_of_the_type_cells(pkg, T):
+    """At 46 types the last blocks with two copies of the type pairs' cells, at
+    47 the first with one; 32 types have two.  An odd number of charge cells
+    lies between the copies.  48-bit sums that differ in order alone."""
+    import torch
+    res = {}
+    for t in (32, T):
+        sysm, d, *par = _system(pkg, 131, t)
+        res[t] = _backward(sysm, d, *par, torch.linspace(0.5, 2.0, len(d), device="cuda"))
+        sysm.ctx.close()
+    assert np.array_equal(res[32][0], res[T][0]) and np.array_equal(res[32][1], res[T][1])
+    for k in range(2, 6):
+        a, b = res[32][k], res[T][k]
+        if k >= 4:
+            assert not b[32:].any() and not b[:, 32:].any()
+            b = b[:32, :32]
+        assert np.abs(a - b).max() <= 1e-9 * np.abs(a).max()
+
+
 def test_sums_beyond_a_float(pkg):
     """A power of two on the weights scales every gradient exactly; the terms
     then pass 1e37 and are added up in double.  Only a sum one of whose terms
