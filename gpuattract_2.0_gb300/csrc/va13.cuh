@@ -28,11 +28,12 @@
  * the warps of an SM are spread over both, and what the instruction cache
  * does not hold every one of them waits for: with the warp form's loops
  * unrolled by the compiler and its divisions inline the rigid kernel was
- * 159 KB long (now 97 KB, the scoring kernel 39) and its warps spent 15 of 27
- * cycles per instruction waiting for code (now 9 of 21; 8,000 poses of a
- * 120-bead ligand, 40 evaluations: 13.4 -> 10.2 ms).  Fewer FP64
- * instructions at the price of more code lost: divisions and comparisons in
- * integer arithmetic 14.5 ms. */
+ * 159 KB long (now 106 KB, the scoring kernel 39) and its warps spent 15 of 27
+ * cycles per instruction waiting for code (then 97 KB and 9 of 21; 8,000 poses
+ * of a 120-bead ligand, 40 evaluations: 13.4 -> 10.2 ms).  Fewer FP64
+ * instructions at the price of more code in the step's way lost: divisions and
+ * comparisons in integer arithmetic 14.5 ms.  mc11a_pair_w's 8 KB take the
+ * place of mc11a_w's, which then seldom runs. */
 #ifdef __CUDA_ARCH__
 #define GBA_VA_LOOP _Pragma("unroll 1")
 #else
@@ -253,7 +254,10 @@ GBA_HD void mc11e(const double* a, int n, double* z, double* w, int ir) {
  * Executors.  `each(lo, hi, f)` runs f(j) for the elements j in [lo, hi]:
  * on the device on lanes lo..hi between two __syncwarp()s; on the host (the
  * tests) in DESCENDING order, so that an element that depended on another
- * element of the same section would change the trajectory.  Shared state is
+ * element of the same section would change the trajectory.  `halves(f)` runs
+ * f(h, k) on lane k of each half warp h, `per_half(f)` f(h) on every lane of
+ * it; what a half keeps between sections is its lanes' own (state(h): the
+ * host keeps both), and second() is half 1's value for all.  Shared state is
  * written only inside `each` (so no lane can read a location in scalar code
  * while another lane writes it); scalar code between sections only reads. */
 struct VaSerial {
@@ -262,10 +266,55 @@ struct VaSerial {
 	GBA_HD void each(int lo, int hi, F f) const {
 		for (int j = hi; j >= lo; --j) f(j);
 	}
+	template <class F>
+	GBA_HD void halves(F f) const {
+		for (int h = 1; h >= 0; --h)
+			for (int k = 15; k >= 0; --k) f(h, k);
+	}
+	template <class F>
+	GBA_HD void per_half(F f) const {
+		f(1);
+		f(0);
+	}
+	GBA_HD int state(int h) const { return h; }
+	GBA_HD int second(int, int of1) const { return of1; }
 };
 
 struct VaWarp {
 	int lane;
+	/* lane k of half h; on the host as VaSerial */
+	template <class F>
+	GBA_HD void halves(F f) const {
+#ifdef __CUDA_ARCH__
+		__syncwarp();
+		f(lane >> 4, lane & 15);
+		__syncwarp();
+#else
+		VaSerial{}.halves(f);
+#endif
+	}
+	template <class F>
+	GBA_HD void per_half(F f) const {
+#ifdef __CUDA_ARCH__
+		f(lane >> 4);
+#else
+		VaSerial{}.per_half(f);
+#endif
+	}
+	GBA_HD int state(int h) const {
+#ifdef __CUDA_ARCH__
+		return 0;
+#else
+		return h;
+#endif
+	}
+	GBA_HD int second(int own, int of1) const {
+#ifdef __CUDA_ARCH__
+		return __shfl_sync(0xffffffffu, own, 16);
+#else
+		return of1;
+#endif
+	}
 	GBA_HD void sync() const {
 #ifdef __CUDA_ARCH__
 		__syncwarp();
@@ -439,6 +488,144 @@ L41: {
 	}
 }
 	if (ir < 0) ir = -ir;
+}
+
+/* minfor's two updates of one step, mc11a(a, n, z0, 1 / dga, w, ir = -n, 1, 0)
+ * and, with its ir negated, mc11a(a, n, z1, 1 / den, z1, ir, 0, 0), side by side: the
+ * first on half warp 0, the second two rows behind it on half 1, so that a
+ * row's division and its elements' updates are one instruction for both.
+ * Returns the second's ir.  For n >= 2 and 0 > dga, den > 0, both finite, when
+ * - the first starts with ir = -n: ti is 0 at L23 (its 1 / sig is not needed),
+ *   ir is n - 1 > 0 from there on, and a row whose diagonal entry is not
+ *   positive is passed over;
+ * - the second starts at L40 with ir = 1 - n: such a row ends it (with ir = n)
+ *   unless z_i is 0.
+ * Every element sees the operations of mc11a in their order.  A row's
+ * al = z_i / a_ii comes with the row before it (row 0: z_1 / a_11); half 1
+ * reads rows that half 0 has left.  w and q, t: its results are not used after.
+ * About 21 FP64 instructions a row, nine of them the division: 8 rows and one
+ * division before them a step for n = 6, where one update after the other took
+ * 12 rows and seven.  1,000 poses, 500/200 beads, 100 evaluations 4.84 ->
+ * 4.61 ms; 8,000, 400/120, 40: 9.80 -> 9.19; 12,000 of four pairs, 1,500/600,
+ * 40: 23.7 -> 22.8. */
+template <class X>
+GBA_HD int mc11a_pair_w(double* a, int n, double* z0, double* z1, double den, double* w, double* q, double* t,
+		const X& ex) {
+	enum Mode { kIdle, kStart, kSkip, kRow, kFill };
+	struct Half {
+		double tim, al, v, aii, ti;
+		Mode mode;
+		int ij, ir;
+		bool active;
+	} st[2];
+	/* L23's quotients; z_1 / a_11; sig of the second */
+	ex.each(0, n + 1, [&](int j) {
+		const double dj = a[va_diag(j < 1 || j > n ? 1 : j, n)];
+		double nu = j > n ? 1.0 : z0[1], de = j > n ? den : dj;
+		if (j >= 1 && j <= n) nu = vm(w[j], w[j]);
+		const double x = va_div(nu, de);
+		if (j > n) t[0] = x;
+		else q[j] = j == 0 || dj != 0.0 ? x : 0.0;
+	});
+	const double sig = t[0], al0 = q[0];
+	/* L23: t_j = the ti of row j, t_0 the tim that the rows begin with */
+	ex.each(0, n, [&](int j) {
+		double ti = 0.0;
+		GBA_VA_LOOP
+		for (int m = n; m > j; --m) ti = ti - q[m];
+		t[j] = ti;
+	});
+	ex.per_half([&](int h) {
+		Half& S = st[ex.state(h)];
+		S.tim = h == 0 ? t[0] : sig;
+		S.al = al0;
+		S.v = S.aii = S.ti = 0.0;
+		S.mode = kIdle;
+		S.ij = 0;
+		S.ir = 1 - n;
+		S.active = true;
+	});
+	GBA_VA_LOOP
+	for (int s = 1; s <= n + 2; ++s) {
+		ex.per_half([&](int h) {
+			Half& S = st[ex.state(h)];
+			const int i = s - 2 * h;
+			S.mode = !S.active || i > n ? kIdle : i < 0 ? kStart : kSkip;
+			if (S.mode != kSkip || i < 1) return;
+			const double* z = h == 0 ? z0 : z1;
+			S.ij = va_diag(i, n);
+			S.v = z[i];
+			S.aii = a[S.ij];
+			if (S.aii > 0.0) {
+				S.mode = kRow;
+				S.ti = h == 0 ? t[i] : S.tim + vm(S.v, S.al);
+			} else if (h == 1 && S.v != 0.0) {
+				S.mode = kFill;
+			}
+		});
+		ex.halves([&](int h, int k) {
+			const Half& S = st[ex.state(h)];
+			const int i = s - 2 * h, j = k + 1;
+			const bool fill = S.mode == kFill;
+			if (S.mode == kIdle || (fill ? j < i || j > n : k > 3)) return;
+			const double* z = h == 0 ? z0 : z1;
+			double nu = S.ti, de = S.tim;                          /* r; kStart: tim */
+			if (fill) {
+				nu = j == i ? vm(S.v, S.v) : z[j];
+				if (j != i) de = S.v;
+			} else if (S.mode == kStart) {
+				nu = 1.0;
+			} else if (k == 1) {                                   /* b */
+				nu = S.al;
+				de = S.ti;
+			} else if (k == 2) {                                   /* gm */
+				nu = S.tim;
+				de = S.ti;
+			} else if (k == 3) {                                   /* the next row's al */
+				nu = 0.0;
+				de = 1.0;
+				if (i < n) {
+					nu = z[i + 1];
+					if (S.mode == kRow) nu = nu - vm(S.v, a[S.ij + 1]);
+					de = a[va_diag(i + 1, n)];
+				}
+			}
+			(fill ? a + S.ij + j - i : (h == 0 ? q : w) + k)[0] = va_div(nu, de);
+		});
+		ex.halves([&](int h, int k) {
+			const Half& S = st[ex.state(h)];
+			const int i = s - 2 * h, j = k + 1;
+			if (S.mode != kRow || j < i || j > n) return;
+			const double* out = h == 0 ? q : w;
+			double* z = h == 0 ? z0 : z1;
+			const double r = out[0], b = out[1], gm = out[2];
+			double* aj = a + S.ij + j - i;
+			if (j == i) {
+				*aj = vm(S.aii, r);
+				return;
+			}
+			if (r == 0.0) return;
+			const double y = *aj, zj = z[j] - vm(S.v, y);
+			*aj = r > 4.0 ? vm(b, z[j]) + vm(y, gm) : y + vm(b, zj);
+			z[j] = zj;
+		});
+		ex.per_half([&](int h) {
+			Half& S = st[ex.state(h)];
+			const double* out = h == 0 ? q : w;
+			if (S.mode == kStart) S.tim = out[0];
+			if (S.mode == kFill) {
+				S.active = false;
+				S.ir = n;
+			}
+			if (S.mode == kRow || S.mode == kSkip) S.al = out[3];
+			if (S.mode == kRow) {
+				if (out[0] == 0.0) S.active = false;
+				S.tim = S.ti;
+			}
+		});
+	}
+	const int ir = ex.second(st[ex.state(0)].ir, st[ex.state(1)].ir);
+	return ir < 0 ? -ir : ir;
 }
 
 /* mc11e in the warp form (q, t: scratch of n + 1 doubles).  The forward
@@ -738,12 +925,18 @@ struct VA13 {
 			d[j] = gb[j] - ga[j];
 			ga[j] = gb[j];
 		});
-		/* minfor's two updates in one loop, so that mc11a's code is there once */
-		GBA_VA_LOOP
-		for (int u = 0; u < 2; ++u) {
-			if (u == 1) ir = -ir;
-			mc11a_w(h, jn, u == 0 ? xbb : d, va_div(1.0, u == 0 ? dga : vm(stmin, dgb - dga)), u == 0 ? w : d, ir, 1 - u,
-					xnull, q, t, ex);
+		{
+			const double den = vm(stmin, dgb - dga), most = 1.7976931348623157e308;
+			if (jn >= 2 && jn <= 16 && dga < 0.0 && dga >= -most && den > 0.0 && den <= most) {
+				ir = mc11a_pair_w(h, jn, xbb, d, den, w, q, t, ex);
+			} else {
+				/* one after the other, in a loop so that mc11a's code is there once */
+				GBA_VA_LOOP
+				for (int u = 0; u < 2; ++u) {
+					if (u == 1) ir = -ir;
+					mc11a_w(h, jn, u == 0 ? xbb : d, va_div(1.0, u == 0 ? dga : den), u == 0 ? w : d, ir, 1 - u, xnull, q, t, ex);
+				}
+			}
 		}
 		if (ir < jn) {
 			phase = kDone;
