@@ -321,7 +321,7 @@ class GbaContext:
         self._check(self.lib.gba_set_pose_order(self.h, int(bool(enable))))
 
     def set_kernel_options(self, flags: int):
-        """GBA_KOPT_* flags: 1 = computed plateau ratio, 2 = 8 lanes per grid
+        """GBA_KOPT_* flags: 1 = computed plateau ratio, 2 = 4 lanes per grid
         lookup, 4 = four-block instantiation, 8 = list entries carrying the
         receptor type, 16 = the reference CPU path's summation order (bit for
         bit the reference's results, slower); the default is 15."""

@@ -154,7 +154,7 @@ __device__ __forceinline__ float corner_weight(int c, float pmn_x, float pmn_y, 
 
 /* Sum of the eight corner products p[c] in the fixed pairwise order
  * ((p0 + p1) + (p2 + p3)) + ((p4 + p5) + (p6 + p7)) -- the order the
- * cooperative 8-lane butterfly produces, so both lookup forms give the same
+ * cooperative butterfly produces, so both lookup forms give the same
  * value bit for bit. */
 __device__ __forceinline__ float octet_sum(const float p[8]) {
 	return fadd(fadd(fadd(p[0], p[1]), fadd(p[2], p[3])), fadd(fadd(p[4], p[5]), fadd(p[6], p[7])));

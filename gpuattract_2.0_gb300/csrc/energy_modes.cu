@@ -30,7 +30,7 @@
  * (R f) . v and f . (R v) replaces (R^T f) . v, so each staged bead's mode
  * vectors are rotated once per round into shared memory (ModeStage) and a
  * projection costs no global load and no rotation.  On octet grids the grid
- * lookups of both passes take the rigid kernel's 8-lane cooperative form
+ * lookups of both passes take the rigid kernel's cooperative form
  * (CoopStep): the lane holding force component c adds f_c times component
  * c of the staged vector.  Kernels are compiled for mode capacities 5 and 10
  * (arrays sized to the capacity, not to GBA_MODES_MAX).

@@ -74,7 +74,7 @@ struct DevNL {
 struct DevGrid {
 	DevIntrpl inner, outer;
 	DevNL nl;
-	/* 8 lanes per grid lookup, one octet corner each (needs both octet copies) */
+	/* 4 lanes per grid lookup, two octet corners each (needs both octet copies) */
 	int coop_lookup;
 };
 

@@ -170,7 +170,7 @@ int gba_set_pose_order(gba_ctx* ctx, int enable);
  *                            within one ulp of the table entry -- instead of
  *                            being gathered from the 4 MB table;
  *   GBA_KOPT_COOP_LOOKUP     on grids with the octet layout (gba_grid_octets),
- *                            8 lanes share one grid lookup, one corner each,
+ *                            4 lanes share one grid lookup, two corners each,
  *                            loaded without L1 allocation;
  *   GBA_KOPT_FOUR_BLOCKS     the scoring kernel is compiled for four resident
  *                            256-thread blocks per SM (64 registers a thread);
@@ -361,10 +361,9 @@ int gba_minimize_6d_modes_plain(gba_ctx* ctx, gba_id rec, gba_id lig, gba_id gri
  * after each evaluation, when every pose of the job fits resident that way;
  * otherwise two poses per block and a control warp that runs one pose's
  * VA13 step while the team evaluates the other.  The result of
- * every pose is the same bit for bit whatever the setting: the minimizers
- * reduce each 64-bead round on its own and add the rounds in order (the
- * plain per-step form's launches do the same; gba_energy_6d reduces once
- * per pose, which differs in the last bits). */
+ * every pose is the same bit for bit whatever the setting: each 64-bead
+ * round is reduced on its own and the rounds are added in order, as in
+ * gba_energy_6d and the plain per-step form's launches. */
 int gba_set_minimize_team(gba_ctx* ctx, int warps_per_pose);
 
 /* Wall-time budget for device minimization (0 = none): warps stop claiming
