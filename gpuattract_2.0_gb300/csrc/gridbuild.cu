@@ -65,17 +65,25 @@ struct BuildArgs {
  * another division -- nine times per voxel and bead and took 77.7 ms.  Here a
  * block holds a brick of 4 x 4 x 4 voxels and up to 32 channels: two warps
  * compute the brick's geometry for 16 beads at a time into shared memory
- * (one also sums the charge channel), eight warps of four channels each read it
+ * (one also sums the charge channel), warps of four or eight channels each read it
  * back, two voxels per lane in packed FP32 instructions, which halve the
  * issue slots.  Double-buffered, one barrier per 16 beads (8: 6 % slower).
  * Measured for the 1,500 beads: 36.8 ms with one geometry warp, which the
- * others waited for; 27.5 ms with two. */
+ * others waited for; 27.5 ms with two (three: 29.0, four: 28.8).
+ *   What the channel warps read then bound it (the L1 data pipe 81 % busy,
+ * FP32 36 % of its issue): per bead five 8-byte words a lane and a 16-byte row
+ * per channel.  Now four words (1/d^6 is two products away), and rows of 16 bytes
+ * for two channels; the double sums, touched every 256 beads, lie in local memory,
+ * where they had pushed other registers out.  With the lists and descriptors
+ * 28.2 -> 26.6 ms with four channels a warp and 25.1 with eight, which share a
+ * word among more channels but leave fewer warps: 600 beads and 8, 16, 20, 28, 32
+ * and 33 channels 2.58, 3.64, 5.24, 6.05, 6.35 and 11.98 ms with four, 2.90,
+ * 4.65, 5.89, 6.22, 6.25 and 11.75 with eight (3.15, 3.86, 5.45, 6.37, 6.84 and
+ * 13.00 before).  Three blocks of eight-channel warps per SM: 27.4. */
 
-constexpr int kChan = 4;                      /* type channels per warp */
-constexpr int kLjWarps = 8;                   /* most warps of type channels per block */
+constexpr int kBlockChan = 32;                /* most type channels per block */
 constexpr int kCube = 4;                      /* voxels per axis of a block */
 constexpr int kChunk = 16;                    /* beads per barrier */
-constexpr int kRowAhead = 4;                  /* beads whose rows a warp loads together */
 static_assert(kTile % kChunk == 0, "a partial sum ends with a chunk");
 
 /* Two voxels of a lane (z and z + 2 of its column): packed FP32, each half
@@ -103,8 +111,8 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
 	return r;
 }
 
-/* One bead's geometry for a lane's two voxels: 1/d^2, the direction over d^2
- * and 1/d^6 at d = max(r, plateau), and d^2 itself. */
+/* One bead's geometry for a lane's two voxels: 1/d^2 and the direction over d^2
+ * at d = max(r, plateau); for the general form 1/d^6 and d^2 too. */
 struct VoxelGeo {
 	f2 rr2[32], ux[32], uy[32], uz[32], rr23[32], d2[32];
 };
@@ -114,10 +122,11 @@ struct Chunk {
 	float qf[kChunk];          /* charge times ffelec, 0: no contribution */
 };
 
-/* out[2 k] = {rc, rc, -ac, -ac}, out[2 k + 1] = {ipon, ipon, rmin2, emin} for
- * k = receptor type * n_lj + channel */
+/* For k = receptor type * n_lj + channel: plain, the k-th pair of floats is
+ * {rc, -ac}; else out[2 k] = {rc, rc, -ac, -ac} and out[2 k + 1] = {ipon, ipon,
+ * rmin2, emin}. */
 __global__ void pair_rows_kernel(DevParams par, const uint32_t* __restrict__ alphabet, uint32_t n_alphabet,
-		uint32_t n_lj, float4* __restrict__ out) {
+		uint32_t n_lj, int plain, float4* __restrict__ out) {
 	const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (k >= (size_t)(par.num_types + 1) * n_lj) return;
 	const uint32_t tr = (uint32_t)(k / n_lj), c = (uint32_t)(k % n_lj);
@@ -128,6 +137,10 @@ __global__ void pair_rows_kernel(DevParams par, const uint32_t* __restrict__ alp
 		const size_t t = (size_t)par.num_types * (tr - 1) + (tl - 1);
 		p = par.lj[t];
 		iv = par.ivor[t];
+	}
+	if (plain) {
+		reinterpret_cast<float2*>(out)[k] = make_float2(p.x, -p.y);
+		return;
 	}
 	out[2 * k] = make_float4(p.x, p.x, -p.y, -p.y);
 	out[2 * k + 1] = make_float4(iv, iv, p.z, p.w);
@@ -155,6 +168,7 @@ __device__ __forceinline__ Bead load_bead(const BuildArgs& a, uint32_t j) {
 /* The geometry of the bead pairs [i0, i1) of a chunk for the brick, by one
  * warp: lane = column (x, y) of the brick and half = bead of the pair; lane b
  * (< kChunk) brings bead b of the chunk. */
+template <bool PLAIN>
 __device__ __forceinline__ void fill_chunk(const BuildArgs& a, const Bead& mine, int i0, int i1, float px, float py,
 		const float pz[kCube], int lane, Chunk& C) {
 	const int col = lane & 15, half = lane >> 4;
@@ -202,14 +216,17 @@ __device__ __forceinline__ void fill_chunk(const BuildArgs& a, const Bead& mine,
 			g.ux[l] = mul2(pack2(ex[h], ex[h + 2]), i2);
 			g.uy[l] = mul2(pack2(ey[h], ey[h + 2]), i2);
 			g.uz[l] = mul2(pack2(ez[h], ez[h + 2]), i2);
-			g.rr23[l] = mul2(mul2(i2, i2), i2);
-			g.d2[l] = pack2(e2[h], e2[h + 2]);
+			if (!PLAIN) {
+				g.rr23[l] = mul2(mul2(i2, i2), i2);
+				g.d2[l] = pack2(e2[h], e2[h + 2]);
+			}
 		}
 	}
 }
 
 /* Adds a partial sum's packed pair to the two voxels' double sums. */
-__device__ __forceinline__ void fold2(f2& part, double acc[2]) {
+template <class Acc>
+__device__ __forceinline__ void fold2(f2& part, Acc* acc) {
 	float lo, hi;
 	unpack2(part, lo, hi);
 	acc[0] = __dadd_rn(acc[0], (double)lo);
@@ -219,9 +236,10 @@ __device__ __forceinline__ void fold2(f2& part, double acc[2]) {
 
 /* PLAIN: every pair's ipon is 1, its minimum lies inside the plateau (no
  * branch on d^2 < rmin2) and 2 (rep rr23) = rep (2 rr23) without underflow;
- * the host checks all three (plain_pairs).  8-6 shape only. */
-template <bool PLAIN>
-__global__ void __launch_bounds__(32 * (kLjWarps + 2), 2) grid_potential_kernel(const BuildArgs a,
+ * the host checks all three (plain_pairs).  8-6 shape only.  CH: type channels
+ * per warp. */
+template <bool PLAIN, int CH>
+__global__ void __launch_bounds__(32 * (kBlockChan / CH + 2), 2) grid_potential_kernel(const BuildArgs a,
 		const gba_intrpl_desc d, float4* __restrict__ out) {
 	__shared__ Chunk buf[2];
 	const uint32_t Nx = d.dimN[0], Ny = d.dimN[1], Nz = d.dimN[2];
@@ -252,14 +270,14 @@ __global__ void __launch_bounds__(32 * (kLjWarps + 2), 2) grid_potential_kernel(
 		f2 part[4] = {0, 0, 0, 0};
 		/* lanes past the chunk load its beads again: inside the receptor or nothing */
 		Bead mine = load_bead(a, lane & (kChunk - 1));
-		fill_chunk(a, mine, i0, i1, px, py, pz, lane, buf[0]);
+		fill_chunk<PLAIN>(a, mine, i0, i1, px, py, pz, lane, buf[0]);
 		mine = load_bead(a, kChunk + (lane & (kChunk - 1)));
 		__syncthreads();
 		for (uint32_t k = 0; k < chunks; ++k) {
 			if (k + 1 < chunks) {
 				const Bead now = mine;
 				mine = load_bead(a, (k + 2) * kChunk + (lane & (kChunk - 1)));
-				fill_chunk(a, now, i0, i1, px, py, pz, lane, buf[(k + 1) & 1]);
+				fill_chunk<PLAIN>(a, now, i0, i1, px, py, pz, lane, buf[(k + 1) & 1]);
 			}
 			if (charge) {
 				const Chunk& C = buf[k & 1];
@@ -292,42 +310,58 @@ __global__ void __launch_bounds__(32 * (kLjWarps + 2), 2) grid_potential_kernel(
 		}
 		return;
 	}
+	constexpr int kAhead = PLAIN ? 2 : 4;      /* beads whose rows a warp loads together */
 	const bool shape86 = PLAIN || a.par.potshape == GBA_POTSHAPE_8_6;
-	const uint32_t c0 = blockIdx.y * (kLjWarps * kChan) + warp * kChan;   /* first type channel */
-	const float4* rows = a.rows + 2 * (size_t)c0;
+	const uint32_t c0 = blockIdx.y * kBlockChan + warp * CH;   /* first type channel */
+	const float4* rows = PLAIN ? a.rows + c0 / 2 : a.rows + 2 * (size_t)c0;
 	/* The assembler fuses a packed product into a packed sum that follows it,
 	 * although both round; a factor of one that it cannot see keeps them apart. */
 	const f2 six = pack2(6.f, 6.f), one = pack2(a.one, a.one);
-	double acc[kChan][4][2] = {};
-	f2 part[kChan][4] = {};
+	/* in local memory, read and written every 256 beads: the registers are the
+	 * partial sums' */
+	volatile double acc[CH][4][2];
+#pragma unroll
+	for (int i = 0; i < CH; ++i)
+#pragma unroll
+		for (int c = 0; c < 4; ++c) acc[i][c][0] = acc[i][c][1] = 0.0;
+	f2 part[CH][4] = {};
 	__syncthreads();
 	for (uint32_t k = 0; k < chunks; ++k) {
 		const Chunk& C = buf[k & 1];
-#pragma unroll kRowAhead
-		for (int b = 0; b < kChunk; ++b) {
-			const float4* row = rows + 2 * (size_t)(C.row[b] * a.n_lj);
-			const VoxelGeo& g = C.geo[b];
-			const f2 rr2 = g.rr2[lane], ux = g.ux[lane], uy = g.uy[lane], uz = g.uz[lane], rr23 = g.rr23[lane];
-			if (PLAIN) {
-				const f2 dbl = add2(rr23, rr23);
+		if (PLAIN) {
+#pragma unroll kAhead
+			for (int b = 0; b < kChunk; ++b) {
+				const VoxelGeo& g = C.geo[b];
+				const f2 rr2 = g.rr2[lane], ux = g.ux[lane], uy = g.uy[lane], uz = g.uz[lane];
+				const f2 rr23 = mul2(mul2(rr2, rr2), rr2), dbl = add2(rr23, rr23);
+				const float4* row = rows + (size_t)(C.row[b] * (a.n_lj / 2));
+				float4 q[CH / 2];
 #pragma unroll
-				for (int i = 0; i < kChan; ++i) {
-					const float4 p = __ldg(row + 2 * i);
-					const f2 rep = mul2(pack2(p.x, p.y), rr2);
-					const f2 vlj = mul2(add2(rep, pack2(p.z, p.w)), rr23);
+				for (int i = 0; i < CH / 2; ++i) q[i] = __ldg(row + i);
+#pragma unroll
+				for (int i = 0; i < CH; ++i) {
+					const float rc = i & 1 ? q[i / 2].z : q[i / 2].x, ac = i & 1 ? q[i / 2].w : q[i / 2].y;
+					const f2 rep = mul2(pack2(rc, rc), rr2);
+					const f2 vlj = mul2(add2(rep, pack2(ac, ac)), rr23);
 					const f2 fb = fma2(six, vlj, mul2(rep, dbl));
 					part[i][0] = fma2(mul2(fb, ux), one, part[i][0]);
 					part[i][1] = fma2(mul2(fb, uy), one, part[i][1]);
 					part[i][2] = fma2(mul2(fb, uz), one, part[i][2]);
 					part[i][3] = add2(part[i][3], vlj);
 				}
-			} else {
+			}
+		} else {
+#pragma unroll kAhead
+			for (int b = 0; b < kChunk; ++b) {
+				const float4* row = rows + 2 * (size_t)(C.row[b] * a.n_lj);
+				const VoxelGeo& g = C.geo[b];
+				const f2 rr2 = g.rr2[lane], ux = g.ux[lane], uy = g.uy[lane], uz = g.uz[lane], rr23 = g.rr23[lane];
 				const f2 sd = shape86 ? pack2(2.f, 2.f) : six;
 				const f2 rrd = shape86 ? rr2 : rr23;
 				float da, db;
 				unpack2(g.d2[lane], da, db);
 #pragma unroll
-				for (int i = 0; i < kChan; ++i) {
+				for (int i = 0; i < CH; ++i) {
 					const float4 p = __ldg(row + 2 * i), m = __ldg(row + 2 * i + 1);   /* m: ipon, ipon, rmin2, emin */
 					const f2 rep = mul2(pack2(p.x, p.y), rrd);
 					const f2 vlj = mul2(add2(rep, pack2(p.z, p.w)), rr23);
@@ -349,13 +383,13 @@ __global__ void __launch_bounds__(32 * (kLjWarps + 2), 2) grid_potential_kernel(
 		}
 		if ((k + 1) % (kTile / kChunk) == 0 || k + 1 == chunks)
 #pragma unroll
-			for (int i = 0; i < kChan; ++i)
+			for (int i = 0; i < CH; ++i)
 #pragma unroll
 				for (int c = 0; c < 4; ++c) fold2(part[i][c], acc[i][c]);
 		__syncthreads();
 	}
 #pragma unroll
-	for (int i = 0; i < kChan; ++i)
+	for (int i = 0; i < CH; ++i)
 		if (c0 + i < a.n_alphabet) {
 			float4* o = out + (size_t)(1 + c0 + i) * N;
 			if (in0) o[v0] = make_float4((float)acc[i][0][0], (float)acc[i][1][0], (float)acc[i][2][0], (float)acc[i][3][0]);
@@ -378,13 +412,18 @@ bool plain_pairs(const std::vector<gba_ffparam>& table, int potshape, float plat
 void launch_potentials(const BuildArgs& a, bool plain, const gba_intrpl_desc& d, float4* out, cudaStream_t s) {
 	uint64_t bricks = 1;
 	for (int k = 0; k < 3; ++k) bricks *= (d.dimN[k] + kCube - 1) / kCube;
-	const uint32_t warps = (a.n_alphabet + kChan - 1) / kChan;      /* type channels, in warps */
-	const unsigned groups = std::max<uint32_t>(1, (warps + kLjWarps - 1) / kLjWarps);
-	const unsigned threads = 32 * (std::min<uint32_t>(warps, kLjWarps) + 2);
-	if (plain)
-		grid_potential_kernel<true><<<dim3((unsigned)bricks, groups), threads, 0, s>>>(a, d, out);
+	const unsigned groups = std::max<uint32_t>(1, (a.n_alphabet + kBlockChan - 1) / kBlockChan);
+	const uint32_t chan = std::min<uint32_t>(a.n_alphabet, kBlockChan);
+	/* eight channels a warp where they fill the block's warps (grid_potential_kernel) */
+	auto launch = [&](auto kernel, uint32_t per) {
+		kernel<<<dim3((unsigned)bricks, groups), 32 * ((chan + per - 1) / per + 2), 0, s>>>(a, d, out);
+	};
+	if (!plain)
+		launch(grid_potential_kernel<false, 4>, 4);
+	else if (a.n_alphabet > 28)
+		launch(grid_potential_kernel<true, 8>, 8);
 	else
-		grid_potential_kernel<false><<<dim3((unsigned)bricks, groups), threads, 0, s>>>(a, d, out);
+		launch(grid_potential_kernel<true, 4>, 4);
 	check_cuda(cudaGetLastError(), "grid build: potentials");
 }
 
@@ -652,22 +691,22 @@ extern "C" int gba_build_grid(gba_ctx* ctx, gba_id rec, gba_id params,
 		a.cut2 = (double)opt->nl_cutoff * opt->nl_cutoff;
 		cudaStream_t s = 0;
 		/* whole blocks of channel warps, so that every warp's row loads stay inside */
-		a.n_lj = (opt->n_alphabet + kLjWarps * kChan - 1) / (kLjWarps * kChan) * (kLjWarps * kChan);
+		a.n_lj = (opt->n_alphabet + kBlockChan - 1) / kBlockChan * kBlockChan;
 		const size_t nrow = (size_t)(a.par.num_types + 1) * a.n_lj;
 		DevBuffer rows;
 		rows.alloc(std::max<size_t>(1, nrow) * 2 * sizeof(float4));
 		a.rows = (const float4*)rows.ptr;
-		if (nrow > 0) {
-			pair_rows_kernel<<<(unsigned)((nrow + 255) / 256), 256, 0, s>>>(a.par, (const uint32_t*)alpha.ptr, a.n_alphabet,
-					a.n_lj, (float4*)rows.ptr);
-			check_cuda(cudaGetLastError(), "grid build: pair rows");
-		}
 		double reach2 = 0.0;      /* beads lie inside the outer grid's box */
 		for (int k = 0; k < 3; ++k) {
 			const double e = (item->outer_desc.dimN[k] + kCube) * (double)item->outer_desc.gridSpacing;
 			reach2 += e * e;
 		}
 		const bool plain = plain_pairs(P->host_table, a.par.potshape, a.plat2, reach2);
+		if (nrow > 0) {
+			pair_rows_kernel<<<(unsigned)((nrow + 255) / 256), 256, 0, s>>>(a.par, (const uint32_t*)alpha.ptr, a.n_alphabet,
+					a.n_lj, plain, (float4*)rows.ptr);
+			check_cuda(cudaGetLastError(), "grid build: pair rows");
+		}
 		launch_potentials(a, plain, item->inner_desc, (float4*)item->inner.ptr, s);
 		launch_potentials(a, plain, item->outer_desc, (float4*)item->outer.ptr, s);
 		DevBuffer counts, sums;

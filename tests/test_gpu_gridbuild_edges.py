@@ -44,6 +44,8 @@ def test_lists_at_tile_edges(pkg, oracle, n, spacing, cutoff, offset):
     (1, 3, 1, 1, 1, 10.0, 2.0),          # one bead: partial chunk and tile
     (16, 4, 1, 1, 0, 10.0, 1.9),         # exactly a chunk, a full channel warp, constant dielectric
     (17, 5, 1, 1, 1, 10.0, 2.1),         # one channel past a warp
+    (31, 8, 1, 1, 1, 10.0, 2.0),         # a full eight-channel warp
+    (48, 9, 1, 1, 0, 10.0, 2.2),         # one channel past it
     (256, 32, 1, 1, 1, 10.0, 3.1),       # exactly a tile and a block of channels
     (257, 33, 1, 1, 1, 10.0, 3.3),       # one past both
     (300, 32, 1, -1, 1, 10.0, 3.0),      # repulsive pairs: the general form
