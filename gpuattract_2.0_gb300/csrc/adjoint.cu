@@ -609,9 +609,8 @@ static_assert(kPairwiseCellBytes + 8 * sizeof(PairStage) <= kPairwiseSmem, "a bl
  * totals within kPairwiseSplitBytes), larger ones whole poses.  The forward
  * pass orders its poses nearest first, so its tail is short, and rounds cost
  * it more sooner.  Measured, whole poses against rounds, 2000/700 beads:
- * forward 1,000 poses (0.2 a warp) 169 -> 79 us, 10,000 (1.6) 220 -> 283;
- * backward 10,000 (2.1) 745 -> 720, 30,000 (6.2, before cell_add2) 2,901 ->
- * 2,999. */
+ * forward 1,000 poses (0.2 a warp) 164 -> 69 us, 10,000 (1.6) 216 -> 285;
+ * backward 10,000 (2.1) 722 -> 657, 30,000 (6.2) 1,716 -> 1,828. */
 constexpr size_t kForwardPosesPerWarp = 1, kBackwardPosesPerWarp = 4;
 constexpr size_t kPairwiseSplitBytes = (size_t)64 << 20;
 

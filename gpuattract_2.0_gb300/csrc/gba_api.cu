@@ -796,9 +796,9 @@ namespace {
  * brings at most this many poses per resident warp: there the slowest warp's
  * whole poses set the time, beyond it the rounds' extra records and totals
  * cost more than the shorter tail saves.  Measured, whole poses against rounds
- * (4,864 warps): 2000/700 beads 100 poses 302 -> 48 us, 2,000 318 -> 137,
- * 10,000 (2.1 a warp) 692 -> 572, 30,000 (6.2) 1572 -> 1567, 100,000 4658 ->
- * 5057; 500/200 beads 10,000 248 -> 237, 30,000 523 -> 547. */
+ * (4,864 warps): 2000/700 beads 100 poses 201 -> 41 us, 2,000 296 -> 127,
+ * 10,000 (2.1 a warp) 566 -> 469, 30,000 (6.2) 1,282 both; 500/200 beads 10,000
+ * 190 -> 189, 30,000 416 -> 451. */
 constexpr size_t kSplitPosesPerWarp = 4;
 /* and its totals stay below this (ligands of thousands of beads) */
 constexpr size_t kSplitBytes = (size_t)64 << 20;
