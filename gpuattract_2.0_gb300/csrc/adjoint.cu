@@ -28,6 +28,7 @@
 #include <cub/cub.cuh>
 
 #include "gba_context.h"
+#include "pairwise_limits.h"
 #include "rigid_pose.cuh"
 
 namespace gba {
@@ -226,18 +227,19 @@ __global__ void __launch_bounds__(kSetupThreads) pairwise_setup_kernel(const Pai
 	}
 	const uint32_t stride = (gridDim.x - 1 - pose_blocks) * kSetupThreads;
 	const uint32_t first = (blockIdx.x - 1 - pose_blocks) * kSetupThreads + threadIdx.x;
-	for (uint32_t k = first; k < L.T * L.T; k += stride) {
-		const uint32_t from = L.T * (k % L.T) + k / L.T;      /* the caller's: receptor type major */
+	const size_t T2 = (size_t)L.T * L.T;
+	for (size_t k = first; k < T2; k += stride) {
+		const uint32_t from = L.T * ((uint32_t)k % L.T) + (uint32_t)k / L.T;      /* the caller's: receptor type major */
 		const float r0 = L.r0[from], eps = L.eps[from];
 		const float r0_2 = r0 * r0, r0_6 = r0_2 * r0_2 * r0_2, r0_8 = r0_6 * r0_2;
 		const float rc = eps * r0_8, ac = eps * r0_6;
 		const bool ok = ac > 0.f && rc > 0.f;
 		const float emin = ok ? -27.f * (ac * ac) * (ac * ac) / (256.f * rc * rc * rc) : 0.f;
 		L.tab[k] = make_float4(rc, ac, (float)L.ipon[from], 0.f);
-		L.tab[L.T * L.T + k] = make_float4(emin, ok ? 4.f * rc / (3.f * ac) : 0.f, ok ? -3.f * emin / rc : 0.f,
+		L.tab[T2 + k] = make_float4(emin, ok ? 4.f * rc / (3.f * ac) : 0.f, ok ? -3.f * emin / rc : 0.f,
 				ok ? 4.f * emin / ac : 0.f);
 	}
-	for (uint32_t j = first; j < L.rec.n; j += stride) {
+	for (size_t j = first; j < L.rec.n; j += stride) {
 		const float4 r = L.rec.xyzq[j];
 		L.rq[j] = make_float4(r.x, r.y, r.z, L.q_rec[j]);
 	}
@@ -386,7 +388,7 @@ __device__ __forceinline__ void pairwise_round(const PairwiseLaunch& L, const Pa
 					float e = vlj, fb = 6.f * vlj + 2.f * c.x * ir8;      /* force factor: f = fb d / r^2 */
 					float drc = ir8, dac = -ir6;
 					if (c.z != 1.f) {
-						const float4 m = __ldg(&L.tab[L.T * L.T + tp]);   /* emin, rmin2, -3 emin / rc, 4 emin / ac */
+						const float4 m = __ldg(&L.tab[(size_t)L.T * L.T + tp]);   /* emin, rmin2, -3 emin / rc, 4 emin / ac */
 						if (r2 < m.y) {
 							e = vlj + (c.z - 1.f) * m.x;
 							drc = ir8 + (c.z - 1.f) * m.z;
@@ -600,8 +602,7 @@ __global__ void __launch_bounds__(256) pairwise_gather_kernel(const PairwiseLaun
 		atomicAdd(&L.g_qrec[q - cells.lig], g);
 }
 
-/* The cells of one block at most, and the shared memory a block may use. */
-constexpr size_t kPairwiseCellBytes = 200 * 1024 - 8 * 2624;
+/* The shared memory a block may use. */
 constexpr size_t kPairwiseSmem = 227 * 1024;
 static_assert(kPairwiseCellBytes + 8 * sizeof(PairStage) <= kPairwiseSmem, "a block of 256 threads always fits");
 
@@ -698,10 +699,10 @@ extern "C" int gba_pairwise_6d(gba_ctx* ctx, gba_id rec, gba_id lig, gba_id grid
 		L.g_r0 = g_r0;
 		L.g_eps = g_eps;
 		cudaStream_t s = (cudaStream_t)stream;
+		if (const char* why = pairwise_refused(backward, L.T, L.lig.n, L.rec.n))
+			throw ApiError(GBA_ERR_INVALID_ARGUMENT, why);
 		const PairCells cells{L.T * L.T, L.lig.n, L.rec.n};
-		const size_t cell_bytes = backward ? (size_t)cells.count() * sizeof(unsigned long long) : 0;
-		if (cell_bytes > kPairwiseCellBytes)
-			throw ApiError(GBA_ERR_INVALID_ARGUMENT, "gba_pairwise_6d: proteins/types too large for the adjoint's shared partials");
+		const size_t cell_bytes = backward ? pairwise_cell_bytes(L.T, L.lig.n, L.rec.n) : 0;
 		const size_t rounds = (L.lig.n + kBeadsPerRound - 1) / kBeadsPerRound;
 		const int threads = !backward ? kForwardThreads
 				: cell_bytes + kPairwiseThreads / 32 * sizeof(PairStage) <= kPairwiseSmem ? kPairwiseThreads : 256;
