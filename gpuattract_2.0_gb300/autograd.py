@@ -6,6 +6,8 @@ PairwiseEnergy  forward: exact ATTRACT pair energy per pose (pairs within the
                 which recomputes the transformed coordinates and returns
                 dE/dDOF, dE/d(ligand / receptor charges) and dE/d(r0, eps) per
                 type pair -- the parameters of a scoring-function refit.
+                Their FP32 terms are summed to 48 bits within a block and in
+                FP64 between blocks, then rounded to float32.
 GridEnergy      forward: the reference-equivalent grid + NL energy
                 (gba_energy_6d); backward: -Result, i.e. the reference's own
                 analytic forces and Euler torques (src/apps/em/meta.h:114-121).

@@ -22,8 +22,9 @@
  *   dE/dq     per ligand and per receptor bead
  *   dE/dr0, dE/deps per type pair [rec type - 1][lig type - 1]
  * Parameter gradients accumulate in the block's shared memory as unevaluated
- * sums of two floats (TwoFloat), are written out per block in double and added
- * up by a last kernel.
+ * sums of two floats (TwoFloat: 48 bits; a block adds some hundred FP32 terms
+ * to a cell), are written out per block in double and added up by a last
+ * kernel.
  */
 #include <cub/cub.cuh>
 
@@ -98,18 +99,25 @@ __device__ __forceinline__ TwoFloat two_add(TwoFloat a, float v) {
 	return TwoFloat{hi, __fsub_rn(l, __fsub_rn(hi, s))};
 }
 
-/* Adds v to a shared cell; what would overflow a TwoFloat (or is no number)
- * goes to the launch's double cell instead.  There is no shared FP64
- * reduction: atomicAdd loops over a compare-and-swap too.  26 M adds to each
- * of two random cells of 1,024: 0.28 ms as doubles, 0.14 ms as TwoFloats;
- * global FP64 reductions 0.34-1.3 ms.  In the kernel lanes meet in cells
- * (a ligand bead's 32 type pairs), and the loops repeat: cell_add2 halves
- * them (10,000 poses, 2000/700 beads, forward and backward: 1,193 -> 966 us). */
-__device__ __forceinline__ void cell_add(unsigned long long* cell, float v, double* beyond) {
+/* Terms enter the cells times 2^40 (exactly): a term is a pair's derivative
+ * times the pose's weight, derivatives go down to 1e-8, and with weights of
+ * 1e-30 the terms themselves would leave FP32's normal range. */
+constexpr float kCellScale = 0x1p40f;
+constexpr double kCellUnscale = 0x1p-40;
+
+/* Adds w x to a shared cell; what would overflow a TwoFloat (or is no number)
+ * goes, unscaled, to the launch's double cell instead.  There is no shared
+ * FP64 reduction: atomicAdd loops over a compare-and-swap too.  26 M adds to
+ * each of two random cells of 1,024: 0.28 ms as doubles, 0.14 ms as
+ * TwoFloats; global FP64 reductions 0.34-1.3 ms.  In the kernel lanes meet in
+ * cells (a ligand bead's 32 type pairs), and the loops repeat: cell_add2
+ * halves them. */
+__device__ __forceinline__ void cell_add(unsigned long long* cell, float w, float x, double* beyond) {
 	constexpr float kBig = 1e37f;
+	const float v = w * kCellScale * x;
 	if (v == 0.f) return;
 	if (!(fabsf(v) < kBig)) {
-		atomicAdd(beyond, (double)v);
+		atomicAdd(beyond, (double)(w * x));
 		return;
 	}
 	unsigned long long old = *(volatile unsigned long long*)cell, was;
@@ -117,7 +125,7 @@ __device__ __forceinline__ void cell_add(unsigned long long* cell, float v, doub
 		was = old;
 		const TwoFloat a{__uint_as_float((uint32_t)was), __uint_as_float((uint32_t)(was >> 32))};
 		if (!(fabsf(a.hi) < kBig)) {
-			atomicAdd(beyond, (double)v);
+			atomicAdd(beyond, (double)(w * x));
 			return;
 		}
 		const TwoFloat t = two_add(a, v);
@@ -130,12 +138,13 @@ __device__ __forceinline__ void cell_add(unsigned long long* cell, float v, doub
 struct __align__(16) TwoFloat2 {
 	TwoFloat a, b;
 };
-__device__ __forceinline__ void cell_add2(TwoFloat2* cell, float va, float vb, double* beyond_a, double* beyond_b) {
+__device__ __forceinline__ void cell_add2(TwoFloat2* cell, float w, float xa, float xb, double* beyond_a, double* beyond_b) {
 	constexpr float kBig = 1e37f;
+	const float va = w * kCellScale * xa, vb = w * kCellScale * xb;
 	if (va == 0.f && vb == 0.f) return;
 	if (!(fabsf(va) < kBig && fabsf(vb) < kBig)) {
-		atomicAdd(beyond_a, (double)va);
-		atomicAdd(beyond_b, (double)vb);
+		atomicAdd(beyond_a, (double)(w * xa));
+		atomicAdd(beyond_b, (double)(w * xb));
 		return;
 	}
 	TwoFloat2 old = *cell, was;
@@ -143,8 +152,8 @@ __device__ __forceinline__ void cell_add2(TwoFloat2* cell, float va, float vb, d
 	do {
 		was = old;
 		if (!(fabsf(was.a.hi) < kBig && fabsf(was.b.hi) < kBig)) {
-			atomicAdd(beyond_a, (double)va);
-			atomicAdd(beyond_b, (double)vb);
+			atomicAdd(beyond_a, (double)(w * xa));
+			atomicAdd(beyond_b, (double)(w * xb));
 			return;
 		}
 		old = atomicCAS(cell, was, TwoFloat2{two_add(was.a, va), two_add(was.b, vb)});
@@ -423,8 +432,8 @@ __device__ __forceinline__ void pairwise_round(const PairwiseLaunch& L, const Pa
 						S.T[3] += u.x * fy; S.T[4] += u.y * fy; S.T[5] += u.z * fy;
 						S.T[6] += u.x * fz; S.T[7] += u.y * fz; S.T[8] += u.z * fz;
 						gqv = L.ffelec * qj * dd;
-						cell_add(cell + cells.qrec() + j, w * (L.ffelec * qi * dd), L.part + cells.qrec() + j);
-						cell_add2(reinterpret_cast<TwoFloat2*>(cell + pair_cells) + tp, w * drc, w * dac, L.part + 2 * tp, L.part + 2 * tp + 1);
+						cell_add(cell + cells.qrec() + j, w, L.ffelec * qi * dd, L.part + cells.qrec() + j);
+						cell_add2(reinterpret_cast<TwoFloat2*>(cell + pair_cells) + tp, w, drc, dac, L.part + 2 * tp, L.part + 2 * tp + 1);
 					}
 				}
 			}
@@ -449,7 +458,7 @@ __device__ __forceinline__ void pairwise_round(const PairwiseLaunch& L, const Pa
 		for (int h = 0; h < 2; ++h)
 			if (nln[h]) {
 				const uint32_t i = i0 + lane + 32 * h;
-				cell_add(cell + cells.qlig() + i, w * W.gq[lane + 32 * h], L.part + cells.qlig() + i);
+				cell_add(cell + cells.qlig() + i, w, W.gq[lane + 32 * h], L.part + cells.qlig() + i);
 			}
 	}
 	__syncwarp();
@@ -547,7 +556,7 @@ __global__ void __launch_bounds__(BACKWARD ? kPairwiseThreads : kForwardThreads,
 				const unsigned long long d = cell[second + k];
 				v += (double)__uint_as_float((uint32_t)d) + (double)__uint_as_float((uint32_t)(d >> 32));
 			}
-			out[k] = v;
+			out[k] = v * kCellUnscale;
 		}
 	}
 }

@@ -399,7 +399,11 @@ typedef struct {
  *  backward (gE != NULL): recomputes everything and writes g_dofs[n*6]
  *           = gE * dE/dDOF in (pos, ang) order -- i.e. -gE * Result, the
  *           convention of src/apps/em/meta.h:114-121 -- and ADDS gE-weighted
- *           dE/dq_lig, dE/dq_rec, dE/dr0, dE/deps into the FP64 arrays. */
+ *           dE/dq_lig, dE/dq_rec, dE/dr0, dE/deps into the FP64 arrays.
+ *           A term is an FP32 product of gE and a pair's FP32 derivative;
+ *           a block of the launch sums its terms to 48 bits (a pair of
+ *           floats; in FP64 where those would overflow), and the blocks'
+ *           sums are added in FP64.  num_types <= 65535. */
 int gba_pairwise_6d(gba_ctx* ctx, gba_id rec, gba_id lig, gba_id grid,
 		const gba_pairwise_params* pp, const gba_dof6d* dofs, size_t n, float* E_out,
 		const float* gE, float* g_dofs, double* g_qlig, double* g_qrec, double* g_r0,
