@@ -128,23 +128,22 @@ extern "C" int gba_autotune(gba_ctx* ctx, gba_id rec, gba_id lig, gba_id grid, g
 			check_cuda(cudaMemcpy(d, sample, n * sizeof(gba_dof6d), cudaMemcpyDefault), "sample");
 			gba_result6d* r = (gba_result6d*)ctx->staging(1, n * sizeof(gba_result6d));
 			EventTimer T;
-			StreamScratch scratch(ctx->scratch_pool);
-			unsigned long long* next = (unsigned long long*)scratch.get(sizeof(unsigned long long), s);
 			if (!have_e) {
 				best_e = 1e30f;
+				StreamScratch scratch(ctx->scratch_pool);
+				RigidLaunch L = base;
+				L.dofs = d;
+				L.out = r;
+				L.n = n;
+				/* the form that a batch of this size takes */
+				RigidPlan plan = ctx->plan_rigid(L, TuneParams{256, 64, 1}, scratch, s);
 				for (int threads : {128, 256}) {
-					const int maxb = rigid_blocks_per_sm(threads, false, base.bound4 != 0, base.ref_order != 0);
+					const int maxb = rigid_blocks_per_sm(threads, false, base.bound4 != 0, base.ref_order != 0, plan.split);
 					for (int bps = 1; bps <= maxb; ++bps) {
-						RigidLaunch L = base;
-						L.dofs = d;
-						L.out = r;
-						L.n = n;
-						L.next = next;
-						const size_t blocks = std::max<size_t>(1, std::min<size_t>(
-								(n + threads / 32 - 1) / (threads / 32), (size_t)ctx->num_sms * bps));
+						plan = rigid_plan(plan.split, n, rounds, ctx->num_sms, threads, bps, maxb);
 						const float ms = T.best_ms([&] {
-							check_cuda(cudaMemsetAsync(next, 0, sizeof(unsigned long long), s), "tune: pose counter");
-							check_cuda(launch_rigid_energy(L, (int)blocks, threads, s), "tune launch");
+							Context::clear_rigid(L, plan, s);
+							Context::launch_rigid(L, plan, s);
 						}, s);
 						if (ms < best_e) {
 							best_e = ms;

@@ -790,35 +790,12 @@ void Context::run_modes(ModesLaunch& L, cudaStream_t s) {
 	check_cuda(launch_modes_energy(L, num_sms, s), "modes energy launch");
 }
 
-namespace {
-
-/* A scoring launch is split into 64-bead rounds (rigid_rounds_kernel) while it
- * brings at most this many poses per resident warp: there the slowest warp's
- * whole poses set the time, beyond it the rounds' extra records and totals
- * cost more than the shorter tail saves.  Measured, whole poses against rounds
- * (4,864 warps): 2000/700 beads 100 poses 201 -> 41 us, 2,000 296 -> 127,
- * 10,000 (2.1 a warp) 566 -> 469, 30,000 (6.2) 1,282 both; 500/200 beads 10,000
- * 190 -> 189, 30,000 416 -> 451. */
-constexpr size_t kSplitPosesPerWarp = 4;
-/* and its totals stay below this (ligands of thousands of beads) */
-constexpr size_t kSplitBytes = (size_t)64 << 20;
-
-}  // namespace
-
-void Context::run_rigid(RigidLaunch& L, cudaStream_t s, const TuneParams* shape) {
-	StreamScratch scratch(scratch_pool);
-	L.order = pose_order(L.dofs, 6, L.n, L.m.grid.outer, s, scratch);
-	const TuneParams tp = shape ? *shape : tuned("energy", L.n);
+RigidPlan Context::plan_rigid(RigidLaunch& L, const TuneParams& tp, StreamScratch& scratch, cudaStream_t s) const {
 	const size_t rounds = (L.m.lig.n + 63) / 64;
-	const bool split = !L.census && !L.ref_order && rounds > 1 &&
-			L.n <= kSplitPosesPerWarp * num_sms * 8 * rigid_blocks_per_sm(256, false, false, false, true) &&
-			L.n * rounds * 16 * sizeof(float) <= kSplitBytes;
-	/* a tuned shape was timed on the launch of whole poses */
-	const int threads = split ? 256 : tp.threads;
-	const size_t warps_per_block = threads / 32;
-	const int bps = split ? rigid_blocks_per_sm(256, false, false, false, true)
-			: std::min(tp.blocks_per_sm, rigid_blocks_per_sm(threads, L.census != nullptr, L.bound4 && !L.census,
-					L.ref_order && !L.census));
+	const bool bound4 = L.bound4 && !L.census;
+	const bool split = !L.census && !L.ref_order &&
+			rigid_splits(L.n, rounds, num_sms, rigid_blocks_per_sm(256, false, bound4, false, true));
+	const int resident = rigid_blocks_per_sm(tp.threads, L.census != nullptr, bound4, L.ref_order && !L.census, split);
 	if (split) {
 		/* one block: the records, the totals, the counts, the counter */
 		const size_t rec = L.n * kPoseRecord * sizeof(float), tot = L.n * rounds * 16 * sizeof(float);
@@ -830,14 +807,25 @@ void Context::run_rigid(RigidLaunch& L, cudaStream_t s, const TuneParams* shape)
 		L.split.rounds = (uint32_t)rounds;
 	} else {
 		L.next = (unsigned long long*)scratch.get(sizeof(unsigned long long), s);
-		check_cuda(cudaMemsetAsync(L.next, 0, sizeof(unsigned long long), s), "rigid energy: pose counter");
 	}
-	const size_t want = (L.n * (split ? rounds : 1) + warps_per_block - 1) / warps_per_block;
-	const int blocks = (int)std::max<size_t>(1, std::min<size_t>(want, (size_t)num_sms * bps));
-	auto launch = [&] {
-		check_cuda(split ? launch_rigid_rounds(L, blocks, threads, s) : launch_rigid_energy(L, blocks, threads, s),
-				"rigid energy launch");
-	};
+	return rigid_plan(split, L.n, rounds, num_sms, tp.threads, tp.blocks_per_sm, resident);
+}
+
+void Context::clear_rigid(const RigidLaunch& L, const RigidPlan& plan, cudaStream_t s) {
+	if (!plan.split) check_cuda(cudaMemsetAsync(L.next, 0, sizeof(unsigned long long), s), "rigid energy: pose counter");
+}
+
+void Context::launch_rigid(const RigidLaunch& L, const RigidPlan& plan, cudaStream_t s) {
+	check_cuda(plan.split ? launch_rigid_rounds(L, plan.blocks, plan.threads, s)
+			: launch_rigid_energy(L, plan.blocks, plan.threads, s), "rigid energy launch");
+}
+
+void Context::run_rigid(RigidLaunch& L, cudaStream_t s, const TuneParams* shape) {
+	StreamScratch scratch(scratch_pool);
+	L.order = pose_order(L.dofs, 6, L.n, L.m.grid.outer, s, scratch);
+	const RigidPlan plan = plan_rigid(L, shape ? *shape : tuned("energy", L.n), scratch, s);
+	clear_rigid(L, plan, s);
+	auto launch = [&] { launch_rigid(L, plan, s); };
 	if (!timing) {
 		launch();
 		return;

@@ -18,6 +18,7 @@
 #include <cstring>
 
 #include "gba_internal.h"
+#include "rigid_plan.h"
 
 namespace gba {
 
@@ -264,6 +265,11 @@ struct Context {
 			const ParamsItem& p);
 	/* tp: launch shape (nullptr: the context-wide "energy" shape) */
 	void run_rigid(RigidLaunch& L, cudaStream_t s, const TuneParams* tp = nullptr);
+	/* its parts: the form and shape of L's launch, with L.next and L.split
+	 * from `scratch`; the counter's clearing; the launch */
+	RigidPlan plan_rigid(RigidLaunch& L, const TuneParams& tp, StreamScratch& scratch, cudaStream_t s) const;
+	static void clear_rigid(const RigidLaunch& L, const RigidPlan& plan, cudaStream_t s);
+	static void launch_rigid(const RigidLaunch& L, const RigidPlan& plan, cudaStream_t s);
 	ModesLaunch modes_launch(gba_id rec, gba_id lig, gba_id grid_rec, gba_id grid_lig, gba_id params);
 	void run_modes(ModesLaunch& L, cudaStream_t s);
 

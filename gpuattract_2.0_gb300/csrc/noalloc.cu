@@ -79,7 +79,8 @@ extern "C" int gba_energy_6d_noalloc(gba_ctx* ctx, gba_id rec, gba_id lig, gba_i
 				? pose_order_in(dofs, 6, n, L.m.grid.outer, (char*)scratch + kCounterBytes,
 						kNoAllocScratchBytes - kCounterBytes, s)
 				: nullptr;
-		/* launch shape as gba_energy_6d chooses it */
+		/* whole poses always (the records of split ones have no place in the
+		 * scratch), in the pair's shape */
 		const TuneParams tp = ctx->pair_tuned("energy", PairKey{rec, lig, grid, params});
 		const int threads = tp.threads;
 		const int bps = std::min(tp.blocks_per_sm, rigid_blocks_per_sm(threads, false, L.bound4 != 0, L.ref_order != 0));

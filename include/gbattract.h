@@ -425,8 +425,10 @@ typedef struct {
  * resident blocks per SM) and of the persistent minimizer (threads per block x
  * poses per queue grab with one warp per pose, or teams of 2..7 warps per pose
  * -- poses per CTA below one) on `sample` poses of this pair and keeps the
- * fastest for this pair: gba_energy_6d, gba_minimize_6d and the plain form
- * launch the pair with them, and a gba_batch_minimize_6d batch launches the
+ * fastest for this pair: gba_energy_6d, gba_energy_6d_noalloc,
+ * gba_minimize_6d and the plain form launch the pair with them, whole poses
+ * and poses split into 64-bead rounds alike (small batches of gba_energy_6d
+ * are split; the sample is timed in the form that its size takes), and a gba_batch_minimize_6d batch launches the
  * pairs of each tuned shape as one persistent kernel, the groups running
  * concurrently in one CUDA graph.  A tuned team applies to minimizations of
  * at most the sample's size.  With cache_path, results are read from /
