@@ -73,6 +73,18 @@ __device__ __forceinline__ void load_modes(const float* __restrict__ v, uint32_t
 	}
 }
 
+/* The same in 16-byte loads, for the reference order, whose kernel the wide
+ * ones cost registers (500 poses, 700/300 beads, 5 modes: 363 against 433 us). */
+template <int MM>
+__device__ __forceinline__ void load_modes16(const float* __restrict__ v, uint32_t M, float (&w)[4 * kModeWords<MM>]) {
+	const float4* q = reinterpret_cast<const float4*>(v);
+#pragma unroll
+	for (int k = 0; k < kModeWords<MM>; ++k) {
+		const float4 t = 4 * k < 3 * (int)M ? __ldg(q + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+		w[4 * k] = t.x; w[4 * k + 1] = t.y; w[4 * k + 2] = t.z; w[4 * k + 3] = t.w;
+	}
+}
+
 /* x + sum_m a_m v_m, unfused in mode order (rotate_translate_deform), with
  * the bead's vectors w already loaded. */
 template <int MM>
@@ -91,7 +103,7 @@ template <int MM>
 __device__ __forceinline__ void deform(const float* __restrict__ v, uint32_t M, const float* amp,
 		float& x, float& y, float& z) {
 	float w[4 * kModeWords<MM>];
-	load_modes<MM>(v, M, w);
+	load_modes16<MM>(v, M, w);
 	deform_w<MM>(w, M, amp, x, y, z);
 }
 
@@ -270,18 +282,41 @@ __device__ __forceinline__ void get_frame(const ModeStage<MM>& MS, int at, float
 	for (int k = 0; k < N; ++k) out[k] = v[k];
 }
 
+/* What staging a round takes of the parked frame.  Five modes on native grids
+ * read it once per pass: reading it each round left the compiler few
+ * registers' worth of lookups in flight (6,000 poses, 700/300 beads, 3 modes:
+ * 482 against 392 us).  On octets, and at ten modes, the registers are better
+ * spent on warps. */
+template <int MM, int LAYOUT>
+constexpr bool kHoldFrame = LAYOUT == kNative && MM <= 5;
+template <int MM>
+struct RecFrame {
+	float Rm[9], Ri[9], ip[3], ampR[MM];
+	__device__ __forceinline__ void read(const ModeStage<MM>& MS) {
+		get_frame(MS, 0, Rm);
+		get_frame(MS, 15, Ri);
+		get_frame(MS, 24, ip);
+		get_frame(MS, 30, ampR);
+	}
+};
+template <int MM>
+struct LigFrame {
+	float Rm[9], tr[3], ampL[MM];
+	__device__ __forceinline__ void read(const ModeStage<MM>& MS) {
+		get_frame(MS, 0, Rm);
+		get_frame(MS, 27, tr);
+		get_frame(MS, 30 + MM, ampL);
+	}
+};
+
 /* Stages 64 receptor beads from j0: deformed, moved into the ligand frame,
  * their lookups in the LIGAND grid queued, their mode vectors rotated for the
  * cooperative lookups.  Returns the number of lookups. */
 template <int MM, class Stage>
-__device__ __forceinline__ uint32_t modes_rec_stage(const ModesLaunch& L, const uint32_t j0, const int lane, Stage& W,
-		ModeStage<MM>& MS) {
+__device__ __forceinline__ uint32_t modes_rec_stage(const ModesLaunch& L, const RecFrame<MM>& F, const uint32_t j0,
+		const int lane, Stage& W, ModeStage<MM>& MS) {
 	const uint32_t Mr = L.rec.n_modes;
-	float Rm[9], Ri[9], ip[3], ampR[MM];
-	get_frame(MS, 0, Rm);
-	get_frame(MS, 15, Ri);
-	get_frame(MS, 24, ip);
-	get_frame(MS, 30, ampR);
+	const float (&Rm)[9] = F.Rm, (&Ri)[9] = F.Ri, (&ip)[3] = F.ip, (&ampR)[MM] = F.ampR;
 	uint32_t nlk[2];
 	BeadGrid bg[2];
 #pragma unroll
@@ -325,8 +360,11 @@ __device__ __forceinline__ void modes_rec_pass(const ModesLaunch& L, const int l
 		float gR[MM]) {
 	const uint32_t Mr = L.rec.n_modes;
 	const int comp = coop_component(lane);
+	RecFrame<MM> F;
+	if (kHoldFrame<MM, LAYOUT>) F.read(MS);
 	for (uint32_t j0 = 0; j0 < L.rec.n; j0 += kBeadsPerRound) {
-		const uint32_t n_look = modes_rec_stage<MM>(L, j0, lane, W, MS);
+		if (!kHoldFrame<MM, LAYOUT>) F.read(MS);
+		const uint32_t n_look = modes_rec_stage<MM>(L, F, j0, lane, W, MS);
 		if (LAYOUT == kAnyLayout ? L.grid_lig.coop_lookup != 0 : LAYOUT == kOctets) {
 			for (uint32_t k0 = 0; k0 < n_look; k0 += 8 * BLOCKS) {
 				CoopStep<BLOCKS> st;
@@ -338,8 +376,7 @@ __device__ __forceinline__ void modes_rec_pass(const ModesLaunch& L, const int l
 				}
 			}
 		} else {
-			float Rm[9];
-			get_frame(MS, 0, Rm);
+			float (&Rm)[9] = F.Rm;
 			for (uint32_t q = lane; q < n_look; q += 32) {
 				const uint32_t s = lookup_slot(W, q);
 				const float4 v = grid_lookup(L.grid_lig, W, q);
@@ -358,13 +395,10 @@ __device__ __forceinline__ void modes_rec_pass(const ModesLaunch& L, const int l
  * lookups and neighbour lists queued, mode vectors rotated.  Returns the
  * number of lookups; n_pair, nln, start as queue_pairs has them. */
 template <int MM>
-__device__ __forceinline__ uint32_t modes_lig_stage(const ModesLaunch& L, const uint32_t i0, const int lane,
-		WarpStage& W, ModeStage<MM>& MS, uint32_t nln[2], uint32_t start[2], uint32_t& n_pair) {
+__device__ __forceinline__ uint32_t modes_lig_stage(const ModesLaunch& L, const LigFrame<MM>& F, const uint32_t i0,
+		const int lane, WarpStage& W, ModeStage<MM>& MS, uint32_t nln[2], uint32_t start[2], uint32_t& n_pair) {
 	const uint32_t Ml = L.lig.n_modes;
-	float Rm[9], tr[3], ampL[MM];
-	get_frame(MS, 0, Rm);
-	get_frame(MS, 27, tr);
-	get_frame(MS, 30 + MM, ampL);
+	const float (&Rm)[9] = F.Rm, (&tr)[3] = F.tr, (&ampL)[MM] = F.ampL;
 	uint32_t nlk[2];
 	BeadGrid bg[2];
 #pragma unroll
@@ -450,9 +484,16 @@ __device__ __forceinline__ void modes_lig_pass(const ModesLaunch& L, const int l
 		PoseSums& S, CoopSums& C, float gL[MM], float gR[MM]) {
 	const uint32_t Mr = L.rec.n_modes, Ml = L.lig.n_modes;
 	const int comp = coop_component(lane);
+	LigFrame<MM> F;
+	float ampR[MM];
+	if (kHoldFrame<MM, LAYOUT>) {
+		F.read(MS);
+		get_frame(MS, 30, ampR);
+	}
 	for (uint32_t i0 = 0; i0 < L.lig.n; i0 += kBeadsPerRound) {
 		uint32_t nln[2], start[2], n_pair;
-		const uint32_t n_look = modes_lig_stage<MM>(L, i0, lane, W, MS, nln, start, n_pair);
+		if (!kHoldFrame<MM, LAYOUT>) F.read(MS);
+		const uint32_t n_look = modes_lig_stage<MM>(L, F, i0, lane, W, MS, nln, start, n_pair);
 		if (LAYOUT == kAnyLayout ? L.grid_rec.coop_lookup != 0 : LAYOUT == kOctets) {
 			for (uint32_t k0 = 0; k0 < n_look; k0 += 16) {
 				CoopStep<2> st;
@@ -478,8 +519,7 @@ __device__ __forceinline__ void modes_lig_pass(const ModesLaunch& L, const int l
 		}
 		/* neighbour pairs after the lookups: measured faster here (the rigid
 		 * kernel measured the opposite) */
-		float ampR[MM];
-		get_frame(MS, 30, ampR);
+		if (!kHoldFrame<MM, LAYOUT>) get_frame(MS, 30, ampR);
 		PairWindow win;
 		for (uint32_t w = 0; w < n_pair; w += 64) {
 			uint32_t so[2];
@@ -721,7 +761,9 @@ __device__ __forceinline__ float eval_pose_modes_team(const ModesLaunch& L, cons
 		for (uint32_t r0 = 0; r0 < rounds; r0 += G) {
 			uint32_t n_look = 0;
 			if (r0 + t < rounds) {
-				n_look = modes_rec_stage<MM>(L, (r0 + t) * kBeadsPerRound, lane, me.W, me.MS);
+				RecFrame<MM> F;
+				F.read(me.MS);
+				n_look = modes_rec_stage<MM>(L, F, (r0 + t) * kBeadsPerRound, lane, me.W, me.MS);
 				team_lookups<MM>(L.grid_lig, me, n_look, lane);
 			}
 			if (lane == 0) sh.n_look[t] = n_look;
@@ -763,7 +805,9 @@ __device__ __forceinline__ float eval_pose_modes_team(const ModesLaunch& L, cons
 	for (uint32_t r0 = 0; r0 < rounds; r0 += G) {
 		uint32_t n_look = 0, n_pair = 0, nln[2] = {0, 0}, start[2] = {0, 0};
 		if (r0 + t < rounds) {
-			n_look = modes_lig_stage<MM>(L, (r0 + t) * kBeadsPerRound, lane, me.W, me.MS, nln, start, n_pair);
+			LigFrame<MM> F;
+			F.read(me.MS);
+			n_look = modes_lig_stage<MM>(L, F, (r0 + t) * kBeadsPerRound, lane, me.W, me.MS, nln, start, n_pair);
 			team_lookups<MM>(L.grid_rec, me, n_look, lane);
 		}
 #pragma unroll
@@ -1197,9 +1241,12 @@ __global__ void __launch_bounds__(32 * kModesMaxTeam, 2) modes_team_kernel(const
 }
 
 /* GBA_KOPT_REFERENCE_ORDER scoring: a warp takes whole poses
- * (eval_pose_modes_ref) with its own receptor array in L.ref_rf. */
+ * (eval_pose_modes_ref) with its own receptor array in L.ref_rf.  Five blocks
+ * per SM asked for: 96 registers and no spills, where the compiler by itself
+ * took 80 and spilled (500 poses, 700/300 beads, 3 modes 287 against 363 us,
+ * 6,000 poses 831 against 872; four blocks 290 and 918, one 284 and 1,055). */
 template <int MM>
-__global__ void __launch_bounds__(kModesRefThreads) modes_ref_kernel(const ModesLaunch L) {
+__global__ void __launch_bounds__(kModesRefThreads, 5) modes_ref_kernel(const ModesLaunch L) {
 	__shared__ WarpStage stage[kModesRefThreads / 32];
 	__shared__ RefModesExtra extra[kModesRefThreads / 32];
 	const int lane = threadIdx.x & 31;
@@ -1247,9 +1294,14 @@ __device__ __forceinline__ int modes_gradient_entry(int j, int Mr, int jn, bool&
 
 /* LAYOUT: compiled for octets where both grids have them, which leaves the
  * native lookups' code out (6,000 poses, 700/300 beads, 20 evaluations: 17.6 ->
- * 16.9 ms). */
+ * 16.9 ms).  Elsewhere three blocks per SM are asked for: with no
+ * number named the compiler schedules the native lookups and the reference
+ * order worse in as many registers (3,000 poses, 700/300 beads, 3 modes, 15
+ * evaluations: 9.6 against 6.2 ms on native grids, 20.3 against 16.8 in the
+ * reference order; one block 6.9 and 18.7); on octets three lose (6,000 poses:
+ * 11.3 against 12.8). */
 template <int MM, bool REF, int LAYOUT>
-__global__ void __launch_bounds__(kModesMinThreads) minimize_modes_kernel(const ModesMinLaunch M) {
+__global__ void __launch_bounds__(kModesMinThreads, LAYOUT == kOctets ? 0 : 3) minimize_modes_kernel(const ModesMinLaunch M) {
 	__shared__ FullStage stage[kModesMinThreads / 32];
 	ModeStage<MM>* ms = reinterpret_cast<ModeStage<MM>*>(modes_dyn_smem);
 	/* per warp, after the mode staging areas: its pose's VA13 state, which
