@@ -485,6 +485,23 @@ __device__ __forceinline__ void pairwise_finish(const PairwiseLaunch& L, size_t 
 	if (lane < 6) L.g_dofs[6 * p + lane] = v;
 }
 
+/* Adds a type pair's (k: ligand type major) or a charge's (q: ligand, then
+ * receptor beads) sums to the caller's gradients: with rc = eps r0^8 and
+ * ac = eps r0^6, d/dr0 = eps (8 r0^7 d/drc + 6 r0^5 d/dac) and
+ * d/deps = r0^8 d/drc + r0^6 d/dac.  Atomics for callers that add several
+ * calls' gradients at once. */
+__device__ __forceinline__ void add_type_pair(const PairwiseLaunch& L, uint32_t k, double drc, double dac) {
+	if (drc == 0.0 && dac == 0.0) return;
+	const uint32_t to = L.T * (k % L.T) + k / L.T;
+	const double r0 = L.r0[to], eps = L.eps[to];
+	const double p2 = r0 * r0, p5 = p2 * p2 * r0, p6 = p5 * r0, p7 = p6 * r0;
+	atomicAdd(&L.g_r0[to], eps * (8.0 * p7 * drc + 6.0 * p5 * dac));
+	atomicAdd(&L.g_eps[to], p7 * r0 * drc + p6 * dac);
+}
+__device__ __forceinline__ void add_charge(const PairwiseLaunch& L, uint32_t q, double g) {
+	if (g != 0.0) atomicAdd(q < L.lig.n ? &L.g_qlig[q] : &L.g_qrec[q - L.lig.n], g);
+}
+
 /* Backward: large blocks, so that few copies of the cells take shared memory
  * (256 threads where they leave no room for more); forward: small ones. */
 constexpr int kPairwiseThreads = 512, kForwardThreads = 256;
@@ -548,25 +565,32 @@ __global__ void __launch_bounds__(BACKWARD ? kPairwiseThreads : kForwardThreads,
 	}
 	if (BACKWARD) {
 		__syncthreads();
-		double* out = L.part + (size_t)(1 + blockIdx.x) * cells.count();
-		for (uint32_t k = threadIdx.x; k < cells.count(); k += blockDim.x) {
+		auto sum = [&](uint32_t k) {
 			const unsigned long long c = cell[k];
 			double v = (double)__uint_as_float((uint32_t)c) + (double)__uint_as_float((uint32_t)(c >> 32));
 			if (k < spare) {
 				const unsigned long long d = cell[second + k];
 				v += (double)__uint_as_float((uint32_t)d) + (double)__uint_as_float((uint32_t)(d >> 32));
 			}
-			out[k] = v * kCellUnscale;
+			return v * kCellUnscale;
+		};
+		if (gridDim.x > 1) {
+			double* out = L.part + (size_t)(1 + blockIdx.x) * cells.count();
+			for (uint32_t k = threadIdx.x; k < cells.count(); k += blockDim.x) out[k] = sum(k);
+			return;
 		}
+		/* the launch's only block needs no other to add its sums up (one pose,
+		 * 300/60 beads: 39 against 34 us for three launches) */
+		for (uint32_t k = threadIdx.x; k < cells.T2; k += blockDim.x)
+			add_type_pair(L, k, __ldcg(&L.part[2 * k]) + sum(2 * k), __ldcg(&L.part[2 * k + 1]) + sum(2 * k + 1));
+		for (uint32_t q = threadIdx.x; q < cells.lig + cells.rec; q += blockDim.x)
+			add_charge(L, q, __ldcg(&L.part[cells.qlig() + q]) + sum(cells.qlig() + q));
 	}
 }
 
-/* Adds the blocks' sums up and to the caller's gradients: with rc = eps r0^8
- * and ac = eps r0^6, d/dr0 = eps (8 r0^7 d/drc + 6 r0^5 d/dac) and
- * d/deps = r0^8 d/drc + r0^6 d/dac.  32 cells per block, eight warps a share
- * of the blocks' sums each (one thread per cell waited 34 us for 456 loads in
- * a row); the atomics are for callers that add several calls' gradients at
- * once. */
+/* Adds the blocks' sums up.  32 cells per block, eight warps a share of the
+ * blocks' sums each (one thread per cell waited 34 us for 456 loads in a
+ * row). */
 __device__ __forceinline__ double cell_sum(const PairwiseLaunch& L, const PairCells& cells, uint32_t k, uint32_t blocks,
 		double (*share)[32]) {
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -593,22 +617,13 @@ __global__ void __launch_bounds__(256) pairwise_gather_kernel(const PairwiseLaun
 		const bool in = k < cells.T2;
 		const double drc = cell_sum(L, cells, in ? 2 * k : cells.count(), blocks, share);
 		const double dac = cell_sum(L, cells, in ? 2 * k + 1 : cells.count(), blocks, share);
-		if (w != 0 || !in || (drc == 0.0 && dac == 0.0)) return;
-		const uint32_t to = L.T * (k % L.T) + k / L.T;
-		const double r0 = L.r0[to], eps = L.eps[to];
-		const double p2 = r0 * r0, p5 = p2 * p2 * r0, p6 = p5 * r0, p7 = p6 * r0;
-		atomicAdd(&L.g_r0[to], eps * (8.0 * p7 * drc + 6.0 * p5 * dac));
-		atomicAdd(&L.g_eps[to], p7 * r0 * drc + p6 * dac);
+		if (w == 0 && in) add_type_pair(L, k, drc, dac);
 		return;
 	}
 	const uint32_t q = (blockIdx.x - type_blocks) * 32 + lane;
 	const bool in = q < cells.lig + cells.rec;
 	const double g = cell_sum(L, cells, in ? cells.qlig() + q : cells.count(), blocks, share);
-	if (w != 0 || !in || g == 0.0) return;
-	if (q < cells.lig)
-		atomicAdd(&L.g_qlig[q], g);
-	else
-		atomicAdd(&L.g_qrec[q - cells.lig], g);
+	if (w == 0 && in) add_charge(L, q, g);
 }
 
 /* The shared memory a block may use. */
@@ -767,7 +782,7 @@ extern "C" int gba_pairwise_6d(gba_ctx* ctx, gba_id rec, gba_id lig, gba_id grid
 		if (backward) {
 			pairwise_kernel<true><<<(unsigned)blocks, threads, smem, s>>>(L);
 			check_cuda(cudaGetLastError(), "pairwise launch");
-			pairwise_gather_kernel<<<(unsigned)((T2 + 31) / 32 + (L.lig.n + L.rec.n + 31) / 32), 256, 0, s>>>(L,
+			if (blocks > 1) pairwise_gather_kernel<<<(unsigned)((T2 + 31) / 32 + (L.lig.n + L.rec.n + 31) / 32), 256, 0, s>>>(L,
 					(uint32_t)blocks);
 		} else {
 			pairwise_kernel<false><<<(unsigned)blocks, threads, smem, s>>>(L);

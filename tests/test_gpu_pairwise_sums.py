@@ -103,3 +103,24 @@ def test_terms_of_both_signs(pkg):
             # drc and dac come back from d/dr0 and d/deps: a few roundings of 8 drc + 6 dac
             bound += 2.0 ** -46 * np.abs(w.astype(np.float64)[:, None] * terms[which, 2:]).sum()
             assert abs(got[k] - math.fsum(v)) <= bound
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17])
+@pytest.mark.parametrize("T", [32, 60, 100])
+def test_one_block_equals_several(pkg, n, T):
+    """At most 16 poses of one round are one block (8 with 100 types, whose
+    cells leave room for 256 threads), which adds its sums to the caller's
+    gradients by itself; four times the poses are several, gathered by a
+    second kernel.  Each sum has some hundred terms: 2^-40 of the largest."""
+    import torch
+    sysm, d, *par = _system(pkg, 40, T)
+    d = d[:n].contiguous()
+    w = torch.linspace(0.5, 2.0, n, device="cuda")
+    one = _backward(sysm, d, *par, w)
+    four = _backward(sysm, d.repeat(4, 1), *par, w.repeat(4))
+    assert np.array_equal(four[0].reshape(4, n), np.tile(one[0], (4, 1)))
+    assert np.array_equal(four[1].reshape(4, n, 6), np.tile(one[1], (4, 1, 1)))
+    for k in range(2, 6):
+        assert np.abs(one[k]).max() > 0
+        assert np.abs(four[k] / 4 - one[k]).max() <= 2.0 ** -40 * np.abs(one[k]).max()
+    sysm.ctx.close()
