@@ -171,7 +171,11 @@ __device__ __forceinline__ void cell_add2(TwoFloat2* cell, float w, float xa, fl
 constexpr int kSetupThreads = 512;
 constexpr int kNearBins = 8192, kNearShift = 18;
 constexpr size_t kNearFirstMinPoses = 2048;
-constexpr size_t kNearOneBlock = 65536;    /* beyond: radix sort (near_first_order) */
+/* Beyond these the radix sort (near_first_order).  Forward, the last size of
+ * one and the first of the other: 300/60 beads 227 against 242 us, 500/200 387
+ * against 403, 2000/700 1,073 against 1,086; the one block's time grows with
+ * the poses, the sort's 30 us hardly. */
+constexpr size_t kNearOneBlock = 65536;
 
 __device__ __forceinline__ uint32_t near_key(const gba_dof6d* __restrict__ dofs, size_t p) {
 	const float* d = reinterpret_cast<const float*>(dofs + p);
@@ -659,6 +663,77 @@ int pairwise_blocks_per_sm(const void* kernel, bool backward, int threads, size_
 	return known[key] = std::max(nb, 1);
 }
 
+/* A launch's poses at most: what it takes of scratch per pose (a record of 80
+ * bytes, 16 and the sort's own for the order) stays within 128 MB however many
+ * poses a call brings. */
+constexpr size_t kPairwiseChunk = (size_t)1 << 20;
+
+/* The launches for the poses of L, at most kPairwiseChunk. */
+void launch_pairwise(Context& ctx, PairwiseLaunch L, bool backward, cudaStream_t s) {
+	const size_t n = L.n;
+	const PairCells cells{L.T * L.T, L.lig.n, L.rec.n};
+	const size_t cell_bytes = backward ? pairwise_cell_bytes(L.T, L.lig.n, L.rec.n) : 0;
+	const size_t rounds = (L.lig.n + kBeadsPerRound - 1) / kBeadsPerRound;
+	const int threads = !backward ? kForwardThreads
+			: cell_bytes + kPairwiseThreads / 32 * sizeof(PairStage) <= kPairwiseSmem ? kPairwiseThreads : 256;
+	const size_t warps = threads / 32;
+	/* a second copy of the type pairs' cells where two blocks still fit an
+	 * SM: half as many lanes meet in a cell.  2000/700 beads, 32 types, forward
+	 * and backward, one copy against two: 10,000 poses 901 -> 876 us, 30,000
+	 * 2,312 -> 2,218; 500/200, 30,000 poses: 887 -> 825. */
+	const size_t two_copies = (cell_bytes + 15) / 16 * 16 + (size_t)2 * L.T * L.T * sizeof(unsigned long long);
+	L.copies = backward && threads == kPairwiseThreads &&
+			2 * (two_copies + warps * sizeof(PairStage) + 1024) <= kPairwiseSmem ? 2 : 1;
+	const size_t smem = (L.copies > 1 ? two_copies : (cell_bytes + 15) / 16 * 16) + warps * sizeof(PairStage);
+	const void* kernel = backward ? (const void*)pairwise_kernel<true> : (const void*)pairwise_kernel<false>;
+	const size_t resident = (size_t)ctx.num_sms * pairwise_blocks_per_sm(kernel, backward, threads, smem);
+	L.by_round = rounds > 1 && n <= (backward ? kBackwardPosesPerWarp : kForwardPosesPerWarp) * resident * warps &&
+			n * rounds * 16 * sizeof(float) <= kPairwiseSplitBytes;
+	const size_t units = L.by_round ? n * rounds : n;
+	const size_t blocks = std::max<size_t>(1, std::min<size_t>((units + warps - 1) / warps, resident));
+	/* one block of scratch, every part 16-byte aligned */
+	StreamScratch scratch(ctx.scratch_pool);
+	const bool sorted = n >= kNearFirstMinPoses && n <= kNearOneBlock;
+	const size_t T2 = cells.T2;
+	size_t at = 0;
+	auto place = [&](size_t bytes) {
+		const size_t o = at;
+		at += (bytes + 15) & ~(size_t)15;
+		return o;
+	};
+	const size_t o_next = place(sizeof(unsigned long long)), o_tab = place(2 * T2 * sizeof(float4)),
+			o_rq = place(L.rec.n * sizeof(float4)), o_pose = place(n * kPoseRecord * sizeof(float)),
+			o_done = place(L.by_round ? n * sizeof(uint32_t) : 0),
+			o_tot = place(L.by_round ? n * rounds * 16 * sizeof(float) : 0),
+			o_order = place(sorted ? n * sizeof(uint32_t) : 0),
+			o_part = place(backward ? (blocks + 1) * cells.count() * sizeof(double) : 0);
+	char* base = (char*)scratch.get(at, s);
+	L.next = (unsigned long long*)(base + o_next);
+	L.tab = (float4*)(base + o_tab);
+	L.rq = (float4*)(base + o_rq);
+	L.split.pose = (float*)(base + o_pose);
+	L.split.done = (uint32_t*)(base + o_done);
+	L.split.totals = (float*)(base + o_tot);
+	L.split.rounds = (uint32_t)rounds;
+	L.part = (double*)(base + o_part);
+	L.order = sorted ? (uint32_t*)(base + o_order) : n > kNearOneBlock ? near_first_order(L.dofs, n, scratch, s) : nullptr;
+	const uint32_t pose_blocks = (uint32_t)((4 * n + kSetupThreads - 1) / kSetupThreads);
+	const uint32_t table_blocks = (uint32_t)std::min<size_t>(
+			(std::max<size_t>(T2, backward ? cells.count() : L.rec.n) + kSetupThreads - 1) / kSetupThreads, 256);
+	pairwise_setup_kernel<<<1 + pose_blocks + std::max(1u, table_blocks), kSetupThreads, 0, s>>>(L, pose_blocks, sorted,
+			backward ? cells.count() : 0);
+	check_cuda(cudaGetLastError(), "pairwise: setup");
+	if (backward) {
+		pairwise_kernel<true><<<(unsigned)blocks, threads, smem, s>>>(L);
+		check_cuda(cudaGetLastError(), "pairwise launch");
+		if (blocks > 1) pairwise_gather_kernel<<<(unsigned)((T2 + 31) / 32 + (L.lig.n + L.rec.n + 31) / 32), 256, 0, s>>>(L,
+				(uint32_t)blocks);
+	} else {
+		pairwise_kernel<false><<<(unsigned)blocks, threads, smem, s>>>(L);
+	}
+	check_cuda(cudaGetLastError(), "pairwise launch");
+}
+
 }  // namespace
 
 }  // namespace gba
@@ -725,69 +800,19 @@ extern "C" int gba_pairwise_6d(gba_ctx* ctx, gba_id rec, gba_id lig, gba_id grid
 		cudaStream_t s = (cudaStream_t)stream;
 		if (const char* why = pairwise_refused(backward, L.T, L.lig.n, L.rec.n))
 			throw ApiError(GBA_ERR_INVALID_ARGUMENT, why);
-		const PairCells cells{L.T * L.T, L.lig.n, L.rec.n};
-		const size_t cell_bytes = backward ? pairwise_cell_bytes(L.T, L.lig.n, L.rec.n) : 0;
-		const size_t rounds = (L.lig.n + kBeadsPerRound - 1) / kBeadsPerRound;
-		const int threads = !backward ? kForwardThreads
-				: cell_bytes + kPairwiseThreads / 32 * sizeof(PairStage) <= kPairwiseSmem ? kPairwiseThreads : 256;
-		const size_t warps = threads / 32;
-		/* a second copy of the type pairs' cells where two blocks still fit an
-		 * SM: half as many lanes meet in a cell.  2000/700 beads, 32 types, forward
-		 * and backward, one copy against two: 10,000 poses 901 -> 876 us, 30,000
-		 * 2,312 -> 2,218; 500/200, 30,000 poses: 887 -> 825. */
-		const size_t two_copies = (cell_bytes + 15) / 16 * 16 + (size_t)2 * L.T * L.T * sizeof(unsigned long long);
-		L.copies = backward && threads == kPairwiseThreads &&
-				2 * (two_copies + warps * sizeof(PairStage) + 1024) <= kPairwiseSmem ? 2 : 1;
-		const size_t smem = (L.copies > 1 ? two_copies : (cell_bytes + 15) / 16 * 16) + warps * sizeof(PairStage);
-		const void* kernel = backward ? (const void*)pairwise_kernel<true> : (const void*)pairwise_kernel<false>;
-		const size_t resident = (size_t)ctx->num_sms * pairwise_blocks_per_sm(kernel, backward, threads, smem);
-		L.by_round = rounds > 1 && n <= (backward ? kBackwardPosesPerWarp : kForwardPosesPerWarp) * resident * warps &&
-				n * rounds * 16 * sizeof(float) <= kPairwiseSplitBytes;
-		const size_t units = L.by_round ? n * rounds : n;
-		const size_t blocks = std::max<size_t>(1, std::min<size_t>((units + warps - 1) / warps, resident));
-		/* one block of scratch, every part 16-byte aligned */
-		StreamScratch scratch(ctx->scratch_pool);
-		const bool sorted = n >= kNearFirstMinPoses && n <= kNearOneBlock;
-		const size_t T2 = cells.T2;
-		size_t at = 0;
-		auto place = [&](size_t bytes) {
-			const size_t o = at;
-			at += (bytes + 15) & ~(size_t)15;
-			return o;
-		};
-		const size_t o_next = place(sizeof(unsigned long long)), o_tab = place(2 * T2 * sizeof(float4)),
-				o_rq = place(L.rec.n * sizeof(float4)), o_pose = place(n * kPoseRecord * sizeof(float)),
-				o_done = place(L.by_round ? n * sizeof(uint32_t) : 0),
-				o_tot = place(L.by_round ? n * rounds * 16 * sizeof(float) : 0),
-				o_order = place(sorted ? n * sizeof(uint32_t) : 0),
-				o_part = place(backward ? (blocks + 1) * cells.count() * sizeof(double) : 0);
-		char* base = (char*)scratch.get(at, s);
-		L.next = (unsigned long long*)(base + o_next);
-		L.tab = (float4*)(base + o_tab);
-		L.rq = (float4*)(base + o_rq);
-		L.split.pose = (float*)(base + o_pose);
-		L.split.done = (uint32_t*)(base + o_done);
-		L.split.totals = (float*)(base + o_tot);
-		L.split.rounds = (uint32_t)rounds;
-		L.part = (double*)(base + o_part);
-		/* the sort takes an int item count: larger batches keep submission order */
-		L.order = sorted ? (uint32_t*)(base + o_order)
-				: n > kNearOneBlock && n <= 0x7fffffffu ? near_first_order(dofs, n, scratch, s) : nullptr;
-		const uint32_t pose_blocks = (uint32_t)((4 * n + kSetupThreads - 1) / kSetupThreads);
-		const uint32_t table_blocks = (uint32_t)std::min<size_t>(
-				(std::max<size_t>(T2, backward ? cells.count() : L.rec.n) + kSetupThreads - 1) / kSetupThreads, 256);
-		pairwise_setup_kernel<<<1 + pose_blocks + std::max(1u, table_blocks), kSetupThreads, 0, s>>>(L, pose_blocks, sorted,
-				backward ? cells.count() : 0);
-		check_cuda(cudaGetLastError(), "pairwise: setup");
-		if (backward) {
-			pairwise_kernel<true><<<(unsigned)blocks, threads, smem, s>>>(L);
-			check_cuda(cudaGetLastError(), "pairwise launch");
-			if (blocks > 1) pairwise_gather_kernel<<<(unsigned)((T2 + 31) / 32 + (L.lig.n + L.rec.n + 31) / 32), 256, 0, s>>>(L,
-					(uint32_t)blocks);
-		} else {
-			pairwise_kernel<false><<<(unsigned)blocks, threads, smem, s>>>(L);
+		/* per-pose results do not depend on the launch, and the sums are added */
+		for (size_t at = 0; at < n; at += kPairwiseChunk) {
+			PairwiseLaunch C = L;
+			C.n = std::min(kPairwiseChunk, n - at);
+			C.dofs = dofs + at;
+			if (backward) {
+				C.gE = gE + at;
+				C.g_dofs = g_dofs + 6 * at;
+			} else {
+				C.E = E_out + at;
+			}
+			launch_pairwise(*ctx, C, backward, s);
 		}
-		check_cuda(cudaGetLastError(), "pairwise launch");
 	} catch (const ApiError& e) {
 		ctx->set_error(e.what());
 		return e.code;
