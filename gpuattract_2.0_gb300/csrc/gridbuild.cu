@@ -53,6 +53,7 @@ struct BuildArgs {
 	const float4* rows;
 	uint32_t n_lj;
 	float one;               /* 1 */
+	uint32_t blank[4];       /* channels of ligand type 0 (a bit each): all zero */
 };
 
 /* ---- potentials -------------------------------------------------------------
@@ -150,14 +151,17 @@ __global__ void pair_rows_kernel(DevParams par, const uint32_t* __restrict__ alp
  * also sums the charge channel takes fewer. */
 constexpr int kPairs = kChunk / 2, kChargePairs = 3;
 
-/* Bead j of the receptor as one lane holds it for its chunk: nothing for a
- * dummy bead (type 0) or past the end. */
+/* Bead j of the receptor as one lane holds it for its chunk.  A dummy bead
+ * (type 0) or one past the end adds zeros to every sum, and lies so far away
+ * that its powers of 1/d are finite: within a plateau of 1e-7 A of a voxel
+ * 1/d^6 is infinite, and zero times that no number. */
+constexpr float kNowhere = 1e18f;
 struct Bead {
 	float4 r;
 	uint32_t type;
 };
 __device__ __forceinline__ Bead load_bead(const BuildArgs& a, uint32_t j) {
-	Bead b{make_float4(0.f, 0.f, 0.f, 0.f), 0u};
+	Bead b{make_float4(kNowhere, kNowhere, kNowhere, 0.f), 0u};
 	if (j < a.n) {
 		b.type = __ldg(&a.tm[j]) & 0xffffu;
 		if (b.type != 0) b.r = __ldg(&a.xyzq[j]);
@@ -392,6 +396,11 @@ __global__ void __launch_bounds__(32 * (kBlockChan / CH + 2), 2) grid_potential_
 	for (int i = 0; i < CH; ++i)
 		if (c0 + i < a.n_alphabet) {
 			float4* o = out + (size_t)(1 + c0 + i) * N;
+			if (!PLAIN && (a.blank[(c0 + i) >> 5] >> ((c0 + i) & 31) & 1u)) {
+				if (in0) o[v0] = make_float4(0.f, 0.f, 0.f, 0.f);
+				if (in1) o[v1] = make_float4(0.f, 0.f, 0.f, 0.f);
+				continue;
+			}
 			if (in0) o[v0] = make_float4((float)acc[i][0][0], (float)acc[i][1][0], (float)acc[i][2][0], (float)acc[i][3][0]);
 			if (in1) o[v1] = make_float4((float)acc[i][0][1], (float)acc[i][1][1], (float)acc[i][2][1], (float)acc[i][3][1]);
 		}
@@ -684,6 +693,8 @@ extern "C" int gba_build_grid(gba_ctx* ctx, gba_id rec, gba_id params,
 		a.tm = R->dev.tm;
 		a.n = R->dev.n;
 		a.one = 1.0f;
+		for (uint32_t c = 0; c < opt->n_alphabet; ++c)
+			if (opt->alphabet[c] == 0) a.blank[c >> 5] |= 1u << (c & 31);
 		a.par = P->dev;
 		a.n_alphabet = opt->n_alphabet;
 		a.plateau = opt->plateau;
