@@ -319,8 +319,10 @@ __global__ void __launch_bounds__(32 * (kBlockChan / CH + 2), 2) grid_potential_
 	const uint32_t c0 = blockIdx.y * kBlockChan + warp * CH;   /* first type channel */
 	const float4* rows = PLAIN ? a.rows + c0 / 2 : a.rows + 2 * (size_t)c0;
 	/* The assembler fuses a packed product into a packed sum that follows it,
-	 * although both round; a factor of one that it cannot see keeps them apart. */
-	const f2 six = pack2(6.f, 6.f), one = pack2(a.one, a.one);
+	 * although both round; a factor of one that it cannot see keeps them apart,
+	 * in every such sum below (a product's second use may keep it whole too,
+	 * but nothing says so). */
+	const f2 six = pack2(6.f, 6.f), two = pack2(2.f, 2.f), one = pack2(a.one, a.one);
 	/* in local memory, read and written every 256 beads: the registers are the
 	 * partial sums' */
 	volatile double acc[CH][4][2];
@@ -337,7 +339,7 @@ __global__ void __launch_bounds__(32 * (kBlockChan / CH + 2), 2) grid_potential_
 			for (int b = 0; b < kChunk; ++b) {
 				const VoxelGeo& g = C.geo[b];
 				const f2 rr2 = g.rr2[lane], ux = g.ux[lane], uy = g.uy[lane], uz = g.uz[lane];
-				const f2 rr23 = mul2(mul2(rr2, rr2), rr2), dbl = add2(rr23, rr23);
+				const f2 rr23 = mul2(mul2(rr2, rr2), rr2), dbl = mul2(rr23, two);
 				const float4* row = rows + (size_t)(C.row[b] * (a.n_lj / 2));
 				float4 q[CH / 2];
 #pragma unroll
@@ -346,12 +348,12 @@ __global__ void __launch_bounds__(32 * (kBlockChan / CH + 2), 2) grid_potential_
 				for (int i = 0; i < CH; ++i) {
 					const float rc = i & 1 ? q[i / 2].z : q[i / 2].x, ac = i & 1 ? q[i / 2].w : q[i / 2].y;
 					const f2 rep = mul2(pack2(rc, rc), rr2);
-					const f2 vlj = mul2(add2(rep, pack2(ac, ac)), rr23);
+					const f2 vlj = mul2(fma2(rep, one, pack2(ac, ac)), rr23);
 					const f2 fb = fma2(six, vlj, mul2(rep, dbl));
 					part[i][0] = fma2(mul2(fb, ux), one, part[i][0]);
 					part[i][1] = fma2(mul2(fb, uy), one, part[i][1]);
 					part[i][2] = fma2(mul2(fb, uz), one, part[i][2]);
-					part[i][3] = add2(part[i][3], vlj);
+					part[i][3] = fma2(vlj, one, part[i][3]);
 				}
 			}
 		} else {
@@ -368,7 +370,7 @@ __global__ void __launch_bounds__(32 * (kBlockChan / CH + 2), 2) grid_potential_
 				for (int i = 0; i < CH; ++i) {
 					const float4 p = __ldg(row + 2 * i), m = __ldg(row + 2 * i + 1);   /* m: ipon, ipon, rmin2, emin */
 					const f2 rep = mul2(pack2(p.x, p.y), rrd);
-					const f2 vlj = mul2(add2(rep, pack2(p.z, p.w)), rr23);
+					const f2 vlj = mul2(fma2(rep, one, pack2(p.z, p.w)), rr23);
 					const f2 fb = fma2(six, vlj, mul2(sd, mul2(rep, rr23)));
 					const f2 iv = pack2(m.x, m.y), off = pack2(fsub(m.x, 1.0f), fsub(m.x, 1.0f));
 					float e_in[2], e_out[2], f_in[2], f_out[2];
@@ -381,7 +383,7 @@ __global__ void __launch_bounds__(32 * (kBlockChan / CH + 2), 2) grid_potential_
 					part[i][0] = fma2(mul2(f, ux), one, part[i][0]);
 					part[i][1] = fma2(mul2(f, uy), one, part[i][1]);
 					part[i][2] = fma2(mul2(f, uz), one, part[i][2]);
-					part[i][3] = add2(part[i][3], e);
+					part[i][3] = fma2(e, one, part[i][3]);
 				}
 			}
 		}
