@@ -794,7 +794,7 @@ RigidPlan Context::plan_rigid(RigidLaunch& L, const TuneParams& tp, StreamScratc
 	const size_t rounds = (L.m.lig.n + 63) / 64;
 	const bool bound4 = L.bound4 && !L.census;
 	const bool split = !L.census && !L.ref_order &&
-			rigid_splits(L.n, rounds, num_sms, rigid_blocks_per_sm(256, false, bound4, false, true));
+			rigid_splits(L.n, L.m.lig.n, num_sms, rigid_blocks_per_sm(256, false, bound4, false, true));
 	const int resident = rigid_blocks_per_sm(tp.threads, L.census != nullptr, bound4, L.ref_order && !L.census, split);
 	if (split) {
 		/* one block: the records, the totals, the counts, the counter */

@@ -21,29 +21,30 @@ def plan(tmp_path_factory):
     f = C.CDLL(str(out)).plan
     f.argtypes = [C.c_size_t] * 2 + [C.c_int] * 4 + [C.POINTER(C.c_int)]
 
-    def run(n, rounds, threads, bps, resident):
+    def run(n, beads, threads, bps, resident):
         o = (C.c_int * 3)()
-        f(n, rounds, SMS, threads, bps, resident, o)
+        f(n, beads, SMS, threads, bps, resident, o)
         return tuple(o)
     return run
 
 
 @pytest.mark.parametrize("threads,bps", [(32, 1), (64, 3), (128, 2), (128, 7), (256, 1), (256, 4)])
-@pytest.mark.parametrize("n,rounds,split", [(1, 1, 0), (100, 11, 1), (19_456, 2, 1), (19_457, 2, 0), (5_000, 1, 0),
-                                            (100_000, 11, 0)])
-def test_shape_asked_for_is_launched(plan, threads, bps, n, rounds, split):
-    units = n * rounds if split else n
+@pytest.mark.parametrize("n,beads,split", [(1, 1, 0), (1, 64, 0), (100, 700, 1), (19_456, 700, 1), (19_457, 700, 0),
+                                           (5_000, 64, 0), (100_000, 700, 0), (1, 72, 0), (76, 73, 1), (77, 73, 0),
+                                           (9_728, 200, 1), (9_729, 200, 0), (19_456, 328, 1), (19_456, 327, 0)])
+def test_shape_asked_for_is_launched(plan, threads, bps, n, beads, split):
+    units = n * -(-beads // 64) if split else n
     warps = threads // 32
     want = max(1, min(-(-units // warps), SMS * bps))
-    assert plan(n, rounds, threads, bps, 8) == (split, threads, want)
+    assert plan(n, beads, threads, bps, 8) == (split, threads, want)
     # more blocks than are resident are not launched
-    assert plan(n, rounds, threads, 64, bps) == (split, threads, want)
+    assert plan(n, beads, threads, 64, bps) == (split, threads, want)
 
 
 def test_totals_stay_bounded(plan):
     """64 MiB of round totals at most: 16 floats per pose and round."""
-    assert plan(1000, 1048, 256, 64, 4)[0] == 1
-    assert plan(1000, 1049, 256, 64, 4)[0] == 0
+    assert plan(1000, 64 * 1048, 256, 64, 4)[0] == 1
+    assert plan(1000, 64 * 1048 + 1, 256, 64, 4)[0] == 0
 
 
 @pytest.mark.gpu
