@@ -634,14 +634,25 @@ __global__ void __launch_bounds__(256) pairwise_gather_kernel(const PairwiseLaun
 constexpr size_t kPairwiseSmem = 227 * 1024;
 static_assert(kPairwiseCellBytes + 8 * sizeof(PairStage) <= kPairwiseSmem, "a block of 256 threads always fits");
 
-/* Launches of at most this many poses per resident warp take rounds (their
- * totals within kPairwiseSplitBytes), larger ones whole poses.  The forward
- * pass orders its poses nearest first, so its tail is short, and rounds cost
- * it more sooner.  Measured, whole poses against rounds, 2000/700 beads:
- * forward 1,000 poses (0.2 a warp) 164 -> 69 us, 10,000 (1.6) 216 -> 285;
- * backward 10,000 (2.1) 722 -> 657, 30,000 (6.2) 1,716 -> 1,828. */
-constexpr size_t kForwardPosesPerWarp = 1, kBackwardPosesPerWarp = 4;
+/* Launches of few poses per resident warp take rounds (their totals within
+ * kPairwiseSplitBytes), others whole poses: at most 2.5 a warp backward;
+ * forward, where poses are ordered nearest first, so that the tail is short
+ * and rounds cost more sooner, (beads - 72) / 256 and at most one.  Measured,
+ * whole poses against rounds in us:
+ *              poses   2,000     4,000     6,000    10,000      19,000
+ *   forward   300/100  35 41     38 45     43 57     54 86      90 153
+ *             500/200  54 52     58 58     65 83    76 132     127 241
+ *            2000/700 166 90   180 128   193 184   216 296     334 550
+ *   backward  300/100 103 97   119 109   139 126   158 174     248 285
+ *             500/200 158 114  181 129   208 166   224 241     366 408
+ *            2000/700 477 195  516 274   598 379   606 586    981 1060
+ * (6,080 and 4,864 resident warps). */
 constexpr size_t kPairwiseSplitBytes = (size_t)64 << 20;
+inline bool pairwise_splits(bool backward, size_t n, size_t beads, size_t warps) {
+	const size_t rounds = (beads + kBeadsPerRound - 1) / kBeadsPerRound;
+	if (rounds < 2 || n * rounds * 16 * sizeof(float) > kPairwiseSplitBytes) return false;
+	return backward ? 2 * n <= 5 * warps : beads > 72 && 256 * n <= std::min<size_t>(256, beads - 72) * warps;
+}
 
 /* Resident blocks per SM: the opt-in to the shared memory and the query once
  * per device, kernel, block size and shared memory. */
@@ -687,8 +698,7 @@ void launch_pairwise(Context& ctx, PairwiseLaunch L, bool backward, cudaStream_t
 	const size_t smem = (L.copies > 1 ? two_copies : (cell_bytes + 15) / 16 * 16) + warps * sizeof(PairStage);
 	const void* kernel = backward ? (const void*)pairwise_kernel<true> : (const void*)pairwise_kernel<false>;
 	const size_t resident = (size_t)ctx.num_sms * pairwise_blocks_per_sm(kernel, backward, threads, smem);
-	L.by_round = rounds > 1 && n <= (backward ? kBackwardPosesPerWarp : kForwardPosesPerWarp) * resident * warps &&
-			n * rounds * 16 * sizeof(float) <= kPairwiseSplitBytes;
+	L.by_round = pairwise_splits(backward, n, L.lig.n, resident * warps);
 	const size_t units = L.by_round ? n * rounds : n;
 	const size_t blocks = std::max<size_t>(1, std::min<size_t>((units + warps - 1) / warps, resident));
 	/* one block of scratch, every part 16-byte aligned */
