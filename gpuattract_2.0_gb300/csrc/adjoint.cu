@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(BACKWARD ? kPairwiseThreads : kForwardThreads,
 				const unsigned long long d = cell[second + k];
 				v += (double)__uint_as_float((uint32_t)d) + (double)__uint_as_float((uint32_t)(d >> 32));
 			}
-			return v * kCellUnscale;
+			return v;
 		};
 		if (gridDim.x > 1) {
 			double* out = L.part + (size_t)(1 + blockIdx.x) * cells.count();
@@ -586,29 +586,36 @@ __global__ void __launch_bounds__(BACKWARD ? kPairwiseThreads : kForwardThreads,
 		/* the launch's only block needs no other to add its sums up (one pose,
 		 * 300/60 beads: 39 against 34 us for three launches) */
 		for (uint32_t k = threadIdx.x; k < cells.T2; k += blockDim.x)
-			add_type_pair(L, k, __ldcg(&L.part[2 * k]) + sum(2 * k), __ldcg(&L.part[2 * k + 1]) + sum(2 * k + 1));
+			add_type_pair(L, k, __ldcg(&L.part[2 * k]) + sum(2 * k) * kCellUnscale,
+					__ldcg(&L.part[2 * k + 1]) + sum(2 * k + 1) * kCellUnscale);
 		for (uint32_t q = threadIdx.x; q < cells.lig + cells.rec; q += blockDim.x)
-			add_charge(L, q, __ldcg(&L.part[cells.qlig() + q]) + sum(cells.qlig() + q));
+			add_charge(L, q, __ldcg(&L.part[cells.qlig() + q]) + sum(cells.qlig() + q) * kCellUnscale);
 	}
 }
 
-/* Adds the blocks' sums up.  32 cells per block, eight warps a share of the
- * blocks' sums each (one thread per cell waited 34 us for 456 loads in a
- * row). */
+/* Adds the blocks' sums up, scaled as they are (taking the scale off in the
+ * blocks cost each of them 2 us of its FP64 pipe), and what no TwoFloat held.
+ * 32 cells per block, eight warps a share of the blocks' sums each (one thread
+ * per cell waited 34 us for 456 loads in a row). */
 __device__ __forceinline__ double cell_sum(const PairwiseLaunch& L, const PairCells& cells, uint32_t k, uint32_t blocks,
 		double (*share)[32]) {
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 	double v = 0.0;
-	if (k < cells.count())
+	const bool in = k < cells.count();
+	const double beyond = in && w == 0 ? L.part[k] : 0.0;
+	if (in)
 #pragma unroll 8
-		for (uint32_t b = w; b <= blocks; b += 8) v += L.part[(size_t)b * cells.count() + k];
+		for (uint32_t b = w + 1; b <= blocks; b += 8) v += L.part[(size_t)b * cells.count() + k];
 	share[w][lane] = v;
 	__syncthreads();
-	v = 0.0;
+	if (w == 0) {
+		v = 0.0;
 #pragma unroll
-	for (int q = 0; q < 8; ++q) v += share[q][lane];
+		for (int q = 0; q < 8; ++q) v += share[q][lane];
+		v = v * kCellUnscale + beyond;
+	}
 	__syncthreads();
-	return v;
+	return v;      /* warp 0's */
 }
 
 __global__ void __launch_bounds__(256) pairwise_gather_kernel(const PairwiseLaunch L, const uint32_t blocks) {
