@@ -109,9 +109,9 @@ def test_terms_of_both_signs(pkg):
 @pytest.mark.parametrize("T", [32, 60, 100])
 def test_one_block_equals_several(pkg, n, T):
     """At most 16 poses of one round are one block (8 with 100 types, whose
-    cells leave room for 256 threads), which adds its sums to the caller's
-    gradients by itself; four times the poses are several, gathered by a
-    second kernel.  Each sum has some hundred terms: 2^-40 of the largest."""
+    cells leave room for 256 threads), most of whose cells stay empty; four
+    times the poses are several.  Each sum has some hundred terms: 2^-40 of the
+    largest."""
     import torch
     sysm, d, *par = _system(pkg, 40, T)
     d = d[:n].contiguous()
