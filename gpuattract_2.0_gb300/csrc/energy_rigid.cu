@@ -21,9 +21,11 @@
 namespace gba {
 
 /* BOUND4: registers capped for four resident 256-thread blocks per SM
- * (GBA_KOPT_FOUR_BLOCKS). */
+ * (GBA_KOPT_FOUR_BLOCKS), else for three: a few registers more than 80 would
+ * leave two (30,000 poses, 1500/600 beads, every option off: 1,962 against
+ * 1,795 us; without FOUR_BLOCKS alone 1,547 against 1,214). */
 template <bool CENSUS, bool BOUND4>
-__global__ void __launch_bounds__(256, BOUND4 ? 4 : 1) rigid_energy_kernel(const RigidLaunch L) {
+__global__ void __launch_bounds__(256, BOUND4 ? 4 : 3) rigid_energy_kernel(const RigidLaunch L) {
 	__shared__ WarpStage stage[8];   /* one per warp of a <=256-thread block */
 	const int lane = threadIdx.x & 31;
 	for (size_t k = next_pose(L.next, lane); k < L.n; k = next_pose(L.next, lane)) {
@@ -64,8 +66,7 @@ __global__ void __launch_bounds__(128) rigid_setup_kernel(const RigidLaunch L) {
  * a pose's last round adds the totals of all of them in round order, so the
  * result is eval_pose_rigid's bit for bit.  Bound by the latency of one
  * round, where a warp walking whole poses is bound by the sum of them. */
-template <bool BOUND4>
-__global__ void __launch_bounds__(256, BOUND4 ? 4 : 1) rigid_rounds_kernel(const RigidLaunch L) {
+__global__ void __launch_bounds__(256, 4) rigid_rounds_kernel(const RigidLaunch L) {
 	__shared__ WarpStage stage[8];
 	const int lane = threadIdx.x & 31;
 	WarpStage& W = stage[threadIdx.x >> 5];
@@ -166,30 +167,25 @@ cudaError_t launch_rigid_energy(const RigidLaunch& L, int blocks, int threads, c
 
 cudaError_t launch_rigid_rounds(const RigidLaunch& L, int blocks, int threads, cudaStream_t s) {
 	rigid_setup_kernel<<<(unsigned)((4 * L.n + 127) / 128), 128, 0, s>>>(L);
-	if (L.bound4)
-		rigid_rounds_kernel<true><<<blocks, threads, 0, s>>>(L);
-	else
-		rigid_rounds_kernel<false><<<blocks, threads, 0, s>>>(L);
+	rigid_rounds_kernel<<<blocks, threads, 0, s>>>(L);
 	return cudaGetLastError();
 }
 
 /* resident blocks per SM, queried once per device, instantiation and block
  * size (the query costs host time on every launch otherwise) */
 int rigid_blocks_per_sm(int threads, bool census, bool bound4, bool ref_order, bool rounds) {
-	static std::atomic<int> cache[64][6][33];
+	static std::atomic<int> cache[64][5][33];
 	int dev = 0;
 	cudaGetDevice(&dev);
-	const int v = rounds ? (bound4 ? 4 : 5) : census ? 0 : ref_order ? 1 : bound4 ? 2 : 3, t = threads / 32;
+	const int v = rounds ? 4 : census ? 0 : ref_order ? 1 : bound4 ? 2 : 3, t = threads / 32;
 	const bool cacheable = dev >= 0 && dev < 64 && threads % 32 == 0 && t >= 1 && t <= 32;
 	if (cacheable) {
 		const int c = cache[dev][v][t].load(std::memory_order_relaxed);
 		if (c > 0) return c;
 	}
 	int nb = 0;
-	if (rounds && bound4)
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rigid_rounds_kernel<true>, threads, 0);
-	else if (rounds)
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rigid_rounds_kernel<false>, threads, 0);
+	if (rounds)
+		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rigid_rounds_kernel, threads, 0);
 	else if (census)
 		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rigid_energy_kernel<true, false>, threads, 0);
 	else if (ref_order)

@@ -172,8 +172,11 @@ int gba_set_pose_order(gba_ctx* ctx, int enable);
  *   GBA_KOPT_COOP_LOOKUP     on grids with the octet layout (gba_grid_octets),
  *                            4 lanes share one grid lookup, two corners each,
  *                            loaded without L1 allocation;
- *   GBA_KOPT_FOUR_BLOCKS     the scoring kernel is compiled for four resident
- *                            256-thread blocks per SM (64 registers a thread);
+ *   GBA_KOPT_FOUR_BLOCKS     the scoring kernel of whole poses is compiled for
+ *                            four resident 256-thread blocks per SM (64
+ *                            registers a thread); batches split into 64-bead
+ *                            rounds always run so (1,000 poses, 1500/600
+ *                            beads: 71 us, with all registers 91);
  *   GBA_KOPT_TYPED_LIST      the rigid kernels read a copy of the neighbour
  *                            list whose entries carry the receptor bead's
  *                            type in their top 8 bits (built on the device at
@@ -426,14 +429,14 @@ typedef struct {
  * poses per queue grab with one warp per pose, or teams of 2..7 warps per pose
  * -- poses per CTA below one) on `sample` poses of this pair and keeps the
  * fastest for this pair: gba_energy_6d, gba_energy_6d_noalloc,
- * gba_minimize_6d and the plain form launch the pair with them, whole poses
- * and poses split into 64-bead rounds alike (small batches of gba_energy_6d
- * are split; the sample is timed in the form that its size takes), and a gba_batch_minimize_6d batch launches the
- * pairs of each tuned shape as one persistent kernel, the groups running
- * concurrently in one CUDA graph.  A tuned team applies to minimizations of
- * at most the sample's size.  With cache_path, results are read from /
- * appended to that text file (keyed by device, SM count and pair size).  No
- * reference counterpart: the reference fixes 128-thread blocks
+ * gba_minimize_6d and the plain form launch the pair with them -- batches of
+ * gba_energy_6d that are small enough to be split into 64-bead rounds, and
+ * samples of that size, in that form -- and a gba_batch_minimize_6d batch
+ * launches the pairs of each tuned shape as one persistent kernel, the groups
+ * running concurrently in one CUDA graph.  A tuned team applies to
+ * minimizations of at most the sample's size.  With cache_path, results are
+ * read from / appended to that text file (keyed by device, SM count and pair
+ * size).  No reference counterpart: the reference fixes 128-thread blocks
  * (src/service/GPUEnergyService6D.tpp:440-441) and sizes its reduction block
  * from the device (src/service/GPUEnergyService6D.tpp:184-198). */
 int gba_autotune(gba_ctx* ctx, gba_id rec, gba_id lig, gba_id grid, gba_id params,
