@@ -433,7 +433,7 @@ def bench_modes(ctx, pkg, n_poses: int, steps: int, minimize: bool = True, with_
     gr = ctx.build_grid(rec, par, pkg.GridOptions())
     gl = ctx.build_grid(lig, par, pkg.GridOptions())
     for g in (gr, gl):
-        ctx.grid_octets(g, True)      # cooperative 8-lane lookups in both passes
+        ctx.grid_octets(g, True)      # cooperative lookups in both passes
     ids = (rec, lig, gr, gl, par)
     d = torch.from_numpy(wl.dofs).cuda()
     out = ctx.energy_6d_modes(*ids, d)

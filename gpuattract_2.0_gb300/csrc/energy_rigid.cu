@@ -103,10 +103,9 @@ __global__ void __launch_bounds__(256, 4) rigid_rounds_kernel(const RigidLaunch 
 
 /* GBA_KOPT_REFERENCE_ORDER: each pose summed in the reference CPU path's
  * order (eval_pose_rigid_ref).  Compiled for four resident 256-thread blocks
- * per SM (64 registers): it spills 152 bytes there, but the latency of its
- * double-precision chains wants the warps -- config 1 measured 15.4 ms per
- * 100,000 poses at four blocks, 16.7 ms at three (80 registers) and 20.7 ms
- * at two (108, no spills). */
+ * per SM (64 registers, 16 bytes spilled): the latency of its
+ * double-precision chains wants the warps (100,000 poses of 2000/700 beads,
+ * when this was chosen: 15.4 ms at four blocks, 16.7 at three, 20.7 at two). */
 __global__ void __launch_bounds__(256, 4) rigid_energy_ref_kernel(const RigidLaunch L) {
 	__shared__ WarpStage stage[8];
 	const int lane = threadIdx.x & 31;

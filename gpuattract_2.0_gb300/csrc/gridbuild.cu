@@ -58,29 +58,22 @@ struct BuildArgs {
 
 /* ---- potentials -------------------------------------------------------------
  *
- * Per voxel, channel and bead 12 FP32 operations that must each round on
- * their own (the CPU builder's bits), so the FP32 pipe bounds the kernel:
- * 1,500 beads, 1.15 M voxels and 32 channels are 6.6e11 operations, 17.5 ms at
- * the 37.8e12 a second that the pipe does.  One thread per voxel and four
- * channels repeated the geometry -- a division, near beads a square root and
- * another division -- nine times per voxel and bead and took 77.7 ms.  Here a
- * block holds a brick of 4 x 4 x 4 voxels and up to 32 channels: two warps
- * compute the brick's geometry for 16 beads at a time into shared memory
- * (one also sums the charge channel), warps of four or eight channels each read it
- * back, two voxels per lane in packed FP32 instructions, which halve the
- * issue slots.  Double-buffered, one barrier per 16 beads (8: 6 % slower).
- * Measured for the 1,500 beads: 36.8 ms with one geometry warp, which the
- * others waited for; 27.5 ms with two (three: 29.0, four: 28.8).
- *   What the channel warps read then bound it (the L1 data pipe 81 % busy,
- * FP32 36 % of its issue): per bead five 8-byte words a lane and a 16-byte row
- * per channel.  Now four words (1/d^6 is two products away), and rows of 16 bytes
- * for two channels; the double sums, touched every 256 beads, lie in local memory,
- * where they had pushed other registers out.  With the lists and descriptors
- * 28.2 -> 26.6 ms with four channels a warp and 25.1 with eight, which share a
- * word among more channels but leave fewer warps: 600 beads and 8, 16, 20, 28, 32
- * and 33 channels 2.58, 3.64, 5.24, 6.05, 6.35 and 11.98 ms with four, 2.90,
- * 4.65, 5.89, 6.22, 6.25 and 11.75 with eight (3.15, 3.86, 5.45, 6.37, 6.84 and
- * 13.00 before).  Three blocks of eight-channel warps per SM: 27.4. */
+ * Per voxel, channel and bead 12 FP32 operations, each rounded on its own (the
+ * CPU builder's bits): 6.6e11 for 1,500 beads, 1.15 M voxels and 32 channels,
+ * 17.5 ms at the 37.8e12 a second of the FP32 pipe.  A block holds a brick of
+ * 4 x 4 x 4 voxels and up to 32 channels: two warps compute the geometry of 16
+ * beads at a time into shared memory (one also sums the charge channel; with
+ * one such warp the others waited, 36.8 ms against 27.5, with three 29.0),
+ * warps of four or eight channels each read it back, two voxels per lane in
+ * packed FP32 instructions, which halve the issue slots.  Double-buffered, one
+ * barrier per 16 beads (8: 6 % slower).
+ *   What the channel warps read bounds it next (L1 data pipe 81 % busy): four
+ * 8-byte words per bead and lane (1/d^6 is two products away) and a 16-byte row
+ * per two channels.  The double sums, touched every 256 beads, lie in local
+ * memory, where they leave the partial sums their registers.  Eight channels a
+ * warp share a word among more of them but leave fewer warps: with the lists
+ * 25.1 against 26.6 ms; 600 beads and 8, 20, 28, 32 and 33 channels 2.90, 5.89,
+ * 6.22, 6.25 and 11.75 ms against 2.58, 5.24, 6.05, 6.35 and 11.98 with four. */
 
 constexpr int kBlockChan = 32;                /* most type channels per block */
 constexpr int kCube = 4;                      /* voxels per axis of a block */

@@ -26,14 +26,9 @@
 /* Device code of the machine stays small: its loops rolled, its divisions in
  * one function (va_div), mc11a there once.  It runs between two evaluations,
  * the warps of an SM are spread over both, and what the instruction cache
- * does not hold every one of them waits for: with the warp form's loops
- * unrolled by the compiler and its divisions inline the rigid kernel was
- * 159 KB long (now 106 KB, the scoring kernel 39) and its warps spent 15 of 27
- * cycles per instruction waiting for code (then 97 KB and 9 of 21; 8,000 poses
- * of a 120-bead ligand, 40 evaluations: 13.4 -> 10.2 ms).  Fewer FP64
- * instructions at the price of more code in the step's way lost: divisions and
- * comparisons in integer arithmetic 14.5 ms.  mc11a_pair_w's 8 KB take the
- * place of mc11a_w's, which then seldom runs. */
+ * does not hold every one of them waits for (8,000 poses of a 120-bead ligand,
+ * 40 evaluations: 159 KB of code 13.4 ms, 15 of 27 cycles per instruction
+ * waiting for it; 97 KB 10.2 ms, 9 of 21). */
 #ifdef __CUDA_ARCH__
 #define GBA_VA_LOOP _Pragma("unroll 1")
 #else
