@@ -124,3 +124,18 @@ def test_one_block_equals_several(pkg, n, T):
         assert np.abs(one[k]).max() > 0
         assert np.abs(four[k] / 4 - one[k]).max() <= 2.0 ** -40 * np.abs(one[k]).max()
     sysm.ctx.close()
+
+
+@pytest.mark.parametrize("n_lig", [65, 200])
+def test_sums_of_rounds_and_whole_poses(pkg, n_lig):
+    """Forty times the poses, enough for launches of whole poses: the same
+    terms, in other blocks and in another order, to 48 bits a block: 1e-9 of
+    the largest."""
+    import torch
+    sysm, d, *par = _system(pkg, n_lig, 32)
+    w = torch.linspace(0.5, 2.0, len(d), device="cuda")
+    small = _backward(sysm, d, *par, w)
+    big = _backward(sysm, d.repeat(40, 1), *par, w.repeat(40))
+    for k in range(2, 6):
+        assert np.abs(big[k] / 40 - small[k]).max() <= 1e-9 * np.abs(small[k]).max()
+    sysm.ctx.close()
