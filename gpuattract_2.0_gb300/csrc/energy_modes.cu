@@ -73,8 +73,9 @@ __device__ __forceinline__ void load_modes(const float* __restrict__ v, uint32_t
 	}
 }
 
-/* The same in 16-byte loads, for the reference order, whose kernel the wide
- * ones cost registers (500 poses, 700/300 beads, 5 modes: 363 against 433 us). */
+/* The same in 16-byte loads, for the reference order, whose kernels the wide
+ * ones cost registers (500 poses, 700/300 beads, 5 modes: 363 against 433 us)
+ * but for ten modes and many poses (kRefWide). */
 template <int MM>
 __device__ __forceinline__ void load_modes16(const float* __restrict__ v, uint32_t M, float (&w)[4 * kModeWords<MM>]) {
 	const float4* q = reinterpret_cast<const float4*>(v);
@@ -99,11 +100,12 @@ __device__ __forceinline__ void deform_w(const float (&w)[4 * kModeWords<MM>], u
 		}
 }
 
-template <int MM>
+template <int MM, bool WIDE>
 __device__ __forceinline__ void deform(const float* __restrict__ v, uint32_t M, const float* amp,
 		float& x, float& y, float& z) {
 	float w[4 * kModeWords<MM>];
-	load_modes16<MM>(v, M, w);
+	if (WIDE) load_modes<MM>(v, M, w);
+	else load_modes16<MM>(v, M, w);
 	deform_w<MM>(w, M, amp, x, y, z);
 }
 
@@ -932,7 +934,7 @@ __device__ __forceinline__ double pow4_rn(double x) {
 /* One pose in the reference's order; rf: this warp's receptor array.  Lane
  * k (k < 26) brings the k-th float of the DOF_6D_Modes record; returns on
  * lane k (k < 27) the k-th float of the Result_6D_Modes record. */
-template <int MM>
+template <int MM, bool WIDE>
 __device__ __forceinline__ float eval_pose_modes_ref(const ModesLaunch& L, const float dv, const int lane,
 		WarpStage& W, RefModesExtra& X, float4* __restrict__ rf) {
 	const uint32_t Mr = L.rec.n_modes, Ml = L.lig.n_modes;
@@ -967,7 +969,7 @@ __device__ __forceinline__ float eval_pose_modes_ref(const ModesLaunch& L, const
 				const float4 r = __ldg(&L.rec.xyzq[j]);
 				const uint32_t mapped = __ldg(&L.rec.tm[j]) >> 16;
 				float x = r.x, y = r.y, z = r.z;
-				deform<MM>(L.rec_modes + (size_t)j * L.rec_ms, Mr, ampR, x, y, z);
+				deform<MM, WIDE>(L.rec_modes + (size_t)j * L.rec_ms, Mr, ampR, x, y, z);
 				float px, py, pz;
 				rot_apply(Rn.m, x, y, z, px, py, pz);
 				px = fadd(px, ipx); py = fadd(py, ipy); pz = fadd(pz, ipz);
@@ -1002,7 +1004,7 @@ __device__ __forceinline__ float eval_pose_modes_ref(const ModesLaunch& L, const
 			const uint32_t tm = __ldg(&L.lig.tm[i]);
 			const uint32_t type = tm & 0xffffu, mapped = tm >> 16;
 			float x = b.x, y = b.y, z = b.z;
-			deform<MM>(L.lig_modes + (size_t)i * L.lig_ms, Ml, ampL, x, y, z);
+			deform<MM, WIDE>(L.lig_modes + (size_t)i * L.lig_ms, Ml, ampL, x, y, z);
 			float px, py, pz;
 			rot_apply(R0.m, x, y, z, px, py, pz);
 			px = fadd(px, tx); py = fadd(py, ty); pz = fadd(pz, tz);
@@ -1034,7 +1036,7 @@ __device__ __forceinline__ float eval_pose_modes_ref(const ModesLaunch& L, const
 					const uint32_t trec = typed ? ent >> 24 : __ldg(&L.rec.tm[j]) & 0xffffu;
 					const float4 r = __ldg(&L.rec.xyzq[j]);
 					float rx = r.x, ry = r.y, rz = r.z;
-					deform<MM>(L.rec_modes + (size_t)j * L.rec_ms, Mr, ampR, rx, ry, rz);
+					deform<MM, WIDE>(L.rec_modes + (size_t)j * L.rec_ms, Mr, ampR, rx, ry, rz);
 					ref_pair_terms(L.grid_rec.nl, L.par, W, half ? sb : sa, make_float4(rx, ry, rz, r.w), trec,
 							lane);
 					X.j[lane] = j;
@@ -1241,12 +1243,19 @@ __global__ void __launch_bounds__(32 * kModesMaxTeam, 2) modes_team_kernel(const
 }
 
 /* GBA_KOPT_REFERENCE_ORDER scoring: a warp takes whole poses
- * (eval_pose_modes_ref) with its own receptor array in L.ref_rf.  Five blocks
- * per SM asked for: 96 registers and no spills, where the compiler by itself
- * took 80 and spilled (500 poses, 700/300 beads, 3 modes 287 against 363 us,
- * 6,000 poses 831 against 872; four blocks 290 and 918, one 284 and 1,055). */
-template <int MM>
-__global__ void __launch_bounds__(kModesRefThreads, 5) modes_ref_kernel(const ModesLaunch L) {
+ * (eval_pose_modes_ref) with its own receptor array in L.ref_rf.  FEW, for
+ * launches whose poses are all resident: latency bounds them, and the kernel
+ * asks for the registers of five blocks per SM (ten modes: four); beyond, the
+ * compiler's own 80 or 72 hold more warps.  Measured, few against many in us,
+ * 700/300 beads, native grids: 5 modes 500 poses 296 372, 3,000 427 490, 20,000
+ * poses on octets 2,798 2,683; 10 modes 500 poses 320 434, 50,000 on octets
+ * 8,500 (with five blocks) 7,186. */
+template <int MM, bool FEW>
+constexpr int kRefBlocks = FEW ? (MM <= 5 ? 5 : 4) : 0;
+template <int MM, bool FEW>
+constexpr bool kRefWide = MM > 5 && !FEW;
+template <int MM, bool FEW>
+__global__ void __launch_bounds__(kModesRefThreads, kRefBlocks<MM, FEW>) modes_ref_kernel(const ModesLaunch L) {
 	__shared__ WarpStage stage[kModesRefThreads / 32];
 	__shared__ RefModesExtra extra[kModesRefThreads / 32];
 	const int lane = threadIdx.x & 31;
@@ -1255,7 +1264,7 @@ __global__ void __launch_bounds__(kModesRefThreads, 5) modes_ref_kernel(const Mo
 	for (size_t p = next_pose(L.next, lane); p < L.n; p = next_pose(L.next, lane)) {
 		const float* d = reinterpret_cast<const float*>(L.dofs + p);
 		const float dv = lane < 26 ? __ldg(d + lane) : 0.f;
-		const float v = eval_pose_modes_ref<MM>(L, dv, lane, stage[wib], extra[wib], rf);
+		const float v = eval_pose_modes_ref<MM, kRefWide<MM, FEW>>(L, dv, lane, stage[wib], extra[wib], rf);
 		if (lane < 27) reinterpret_cast<float*>(L.out + p)[lane] = v;
 	}
 }
@@ -1298,10 +1307,11 @@ __device__ __forceinline__ int modes_gradient_entry(int j, int Mr, int jn, bool&
  * number named the compiler schedules the native lookups and the reference
  * order worse in as many registers (3,000 poses, 700/300 beads, 3 modes, 15
  * evaluations: 9.6 against 6.2 ms on native grids, 20.3 against 16.8 in the
- * reference order; one block 6.9 and 18.7); on octets three lose (6,000 poses:
- * 11.3 against 12.8). */
+ * * reference order; one block 6.9 and 18.7); on octets three lose (6,000 poses:
+ * 11.3 against 12.8), and so they do in the reference order at ten modes. */
 template <int MM, bool REF, int LAYOUT>
-__global__ void __launch_bounds__(kModesMinThreads, LAYOUT == kOctets ? 0 : 3) minimize_modes_kernel(const ModesMinLaunch M) {
+__global__ void __launch_bounds__(kModesMinThreads, LAYOUT == kOctets || (REF && MM > 5) ? 0 : 3)
+		minimize_modes_kernel(const ModesMinLaunch M) {
 	__shared__ FullStage stage[kModesMinThreads / 32];
 	ModeStage<MM>* ms = reinterpret_cast<ModeStage<MM>*>(modes_dyn_smem);
 	/* per warp, after the mode staging areas: its pose's VA13 state, which
@@ -1354,7 +1364,7 @@ __global__ void __launch_bounds__(kModesMinThreads, LAYOUT == kOctets ? 0 : 3) m
 			const float xf = __shfl_sync(GBA_FULL_MASK, pf, max(from, 0));
 			dv = from >= 0 ? xf : 0.f;
 			if (REF)
-				v = eval_pose_modes_ref<MM>(L, dv, lane, stage[wib], *reinterpret_cast<RefModesExtra*>(&ms[wib]),
+				v = eval_pose_modes_ref<MM, (MM > 5)>(L, dv, lane, stage[wib], *reinterpret_cast<RefModesExtra*>(&ms[wib]),
 						L.ref_rf + (((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * L.rec.n);
 			else
 				v = eval_pose_modes<MM, LAYOUT>(L, dv, lane, stage[wib], ms[wib]);
@@ -1551,16 +1561,25 @@ cudaError_t launch_modes_mm(const ModesLaunch& L, int num_sms, cudaStream_t s) {
 	return cudaGetLastError();
 }
 
+/* The reference-order scoring kernel for L's poses, and its blocks. */
+struct RefLaunch {
+	void (*kernel)(ModesLaunch);
+	size_t blocks;
+};
 template <int MM>
-size_t ref_blocks_mm(const ModesLaunch& L, int num_sms) {
-	const size_t want = (L.n + kModesRefThreads / 32 - 1) / (kModesRefThreads / 32);
-	return std::max<size_t>(1, std::min<size_t>(want,
-			(size_t)num_sms * resident_blocks(modes_ref_kernel<MM>, kModesRefThreads, 0)));
+RefLaunch ref_launch_mm(const ModesLaunch& L, int num_sms) {
+	constexpr size_t warps = kModesRefThreads / 32;
+	const size_t want = std::max<size_t>(1, (L.n + warps - 1) / warps);
+	const size_t few = (size_t)num_sms * resident_blocks(modes_ref_kernel<MM, true>, kModesRefThreads, 0);
+	if (want <= few) return {modes_ref_kernel<MM, true>, want};
+	return {modes_ref_kernel<MM, false>, std::min<size_t>(want,
+			(size_t)num_sms * resident_blocks(modes_ref_kernel<MM, false>, kModesRefThreads, 0))};
 }
 
 template <int MM>
 cudaError_t launch_ref_mm(const ModesLaunch& L, int num_sms, cudaStream_t s) {
-	modes_ref_kernel<MM><<<(unsigned)ref_blocks_mm<MM>(L, num_sms), kModesRefThreads, 0, s>>>(L);
+	const RefLaunch r = ref_launch_mm<MM>(L, num_sms);
+	r.kernel<<<(unsigned)r.blocks, kModesRefThreads, 0, s>>>(L);
 	return cudaGetLastError();
 }
 
@@ -1612,8 +1631,8 @@ cudaError_t launch_modes_energy(const ModesLaunch& L, int num_sms, cudaStream_t 
 }
 
 size_t modes_ref_warps(const ModesLaunch& L, int num_sms) {
-	const size_t blocks = mode_capacity(L) == 5 ? ref_blocks_mm<5>(L, num_sms)
-	                                            : ref_blocks_mm<GBA_MODES_MAX>(L, num_sms);
+	const size_t blocks = mode_capacity(L) == 5 ? ref_launch_mm<5>(L, num_sms).blocks
+	                                            : ref_launch_mm<GBA_MODES_MAX>(L, num_sms).blocks;
 	return blocks * (kModesRefThreads / 32);
 }
 
