@@ -224,6 +224,7 @@ __device__ void near_first_block(const PairwiseLaunch& L, uint32_t* bin) {
 __global__ void __launch_bounds__(kSetupThreads) pairwise_setup_kernel(const PairwiseLaunch L, const uint32_t pose_blocks,
 		const int sort, const uint32_t cells) {
 	__shared__ uint32_t bin[kNearBins];
+	cudaTriggerProgrammaticLaunchCompletion();      /* the pair kernel's blocks may come and wait */
 	if (blockIdx.x == 0) {
 		if (threadIdx.x == 0) *L.next = 0;
 		if (sort) near_first_block(L, bin);
@@ -530,6 +531,7 @@ __global__ void __launch_bounds__(BACKWARD ? kPairwiseThreads : kForwardThreads,
 		for (uint32_t k = threadIdx.x; k < second + spare; k += blockDim.x) cell[k] = 0;
 		__syncthreads();
 	}
+	cudaGridDependencySynchronize();      /* the setup kernel's records and tables */
 	const int lane = threadIdx.x & 31;
 	PairStage& W = stage[threadIdx.x >> 5];
 	const uint32_t rounds = L.split.rounds;
@@ -569,6 +571,7 @@ __global__ void __launch_bounds__(BACKWARD ? kPairwiseThreads : kForwardThreads,
 		__syncwarp();
 	}
 	if (BACKWARD) {
+		cudaTriggerProgrammaticLaunchCompletion();
 		__syncthreads();
 		double* out = L.part + (size_t)(1 + blockIdx.x) * cells.count();
 		for (uint32_t k = threadIdx.x; k < cells.count(); k += blockDim.x) {
@@ -613,6 +616,7 @@ __device__ __forceinline__ double cell_sum(const PairwiseLaunch& L, const PairCe
 
 __global__ void __launch_bounds__(256) pairwise_gather_kernel(const PairwiseLaunch L, const uint32_t blocks) {
 	__shared__ double share[8][32];
+	cudaGridDependencySynchronize();      /* the blocks' sums */
 	const PairCells cells{L.T * L.T, L.lig.n, L.rec.n};
 	const uint32_t type_blocks = (cells.T2 + 31) / 32;
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -679,6 +683,24 @@ int pairwise_blocks_per_sm(const void* kernel, bool backward, int threads, size_
  * poses a call brings. */
 constexpr size_t kPairwiseChunk = (size_t)1 << 20;
 
+/* A launch that, if `early`, may begin while the kernel before it runs; the
+ * kernel itself waits for that one's results (cudaGridDependencySynchronize). */
+template <class... P, class... A>
+void launch_after(bool early, void (*kernel)(P...), size_t blocks, int threads, size_t smem, cudaStream_t s,
+		const A&... args) {
+	cudaLaunchAttribute attr{};
+	attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr.val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+	cudaLaunchConfig_t cfg{};
+	cfg.gridDim = dim3((unsigned)blocks);
+	cfg.blockDim = dim3(threads);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = s;
+	cfg.attrs = &attr;
+	cfg.numAttrs = 1;
+	check_cuda(cudaLaunchKernelEx(&cfg, kernel, P(args)...), "pairwise launch");
+}
+
 /* The launches for the poses of L, at most kPairwiseChunk. */
 void launch_pairwise(Context& ctx, PairwiseLaunch L, bool backward, cudaStream_t s) {
 	const size_t n = L.n;
@@ -733,13 +755,17 @@ void launch_pairwise(Context& ctx, PairwiseLaunch L, bool backward, cudaStream_t
 	pairwise_setup_kernel<<<1 + pose_blocks + std::max(1u, table_blocks), kSetupThreads, 0, s>>>(L, pose_blocks, sorted,
 			backward ? cells.count() : 0);
 	check_cuda(cudaGetLastError(), "pairwise: setup");
+	/* few blocks: the launches overlap (one pose, 300/60 beads, backward 34 ->
+	 * 29 us; 64 poses, 56/17: 37.5 -> 32.5).  A launch that fills the chip would
+	 * have its blocks placed around the setup's (30,000 poses, 2000/700 beads,
+	 * forward 509 -> 524). */
+	const bool early = 2 * blocks <= resident;
 	if (backward) {
-		pairwise_kernel<true><<<(unsigned)blocks, threads, smem, s>>>(L);
-		check_cuda(cudaGetLastError(), "pairwise launch");
-		pairwise_gather_kernel<<<(unsigned)((T2 + 31) / 32 + (L.lig.n + L.rec.n + 31) / 32), 256, 0, s>>>(L,
+		launch_after(early, pairwise_kernel<true>, blocks, threads, smem, s, L);
+		launch_after(early, pairwise_gather_kernel, (T2 + 31) / 32 + (L.lig.n + L.rec.n + 31) / 32, 256, 0, s, L,
 				(uint32_t)blocks);
 	} else {
-		pairwise_kernel<false><<<(unsigned)blocks, threads, smem, s>>>(L);
+		launch_after(early, pairwise_kernel<false>, blocks, threads, smem, s, L);
 	}
 	check_cuda(cudaGetLastError(), "pairwise launch");
 }
